@@ -1,13 +1,13 @@
 // dustb_fp64.cu -- the FP64 form of the dust drag step: one kernel per reference kernel,
-// one thread per particle or per cell, FP64 global atomics for the deposits.  This is the
-// straightforward GPU form of the reference's Kokkos kernels (the "plain FP64" baseline of
-// the mixed-precision form in dustb_mixed.cu).  Compiled with --fmad=false so that the
-// per-particle arithmetic rounds exactly as the CPU oracle's does.
+// one thread per particle or per cell, the deposits combined per cell inside a warp
+// (dustb_deposit.cuh).  Compiled with --fmad=false so that the per-particle arithmetic rounds
+// exactly as the CPU oracle's does.
 #include <cfloat>
 #include <cstdio>
 #include <cstring>
 
 #include "dustb_common.cuh"
+#include "dustb_deposit.cuh"
 #include "dustb_sort.cuh"
 
 using namespace dustb;
@@ -472,35 +472,91 @@ __global__ void k_route(PCtx P, MCtx M, Ind d, int x3bc, double *x3rem, unsigned
   else if (hi3) { P.r(DUSTB_IPZ, p) -= Lz; P.r(DUSTB_IPZ1, p) -= Lz; }
 }
 
-// ---- DepositDrag imex scatter, src/dust/dust_pm.cpp:225-274 ------------------------------
-__global__ void k_scatter(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh,
-                          unsigned *err) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
-  int m = P.i(DUSTB_PGID, p) - M.gids;
-  if (!block_ok(d, m)) { report(err, DUSTB_ERR_PGID); return; }
-  int ip, jp, kp; double wx[3], wy[3], wz[3];
-  weights3(M, d, m, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p) + sh * P.r(DUSTB_IPX, p),
-           P.r(DUSTB_IPZ, p), ip, jp, kp, wx, wy, wz);
-  if (!halo_ok(d, ip, jp, kp)) { report(err, DUSTB_ERR_HALO); return; }
-  double vol = cell_vol(M, d, m);
-  double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
-  double muc = P.r(DUSTB_IPM, p) * cj / vol;
-  double vx = P.r(DUSTB_IPVX, p), vy = P.r(DUSTB_IPVY, p), vz = P.r(DUSTB_IPVZ, p);
-  int clo = d.three_d ? 0 : 1, chi = d.three_d ? 2 : 1;
-  for (int c = clo; c <= chi; ++c)
-    for (int b = 0; b < 3; ++b) {
-      double wcb = wz[c] * wy[b] * muc;
-      if (wcb == 0.0) continue;
-      for (int a = 0; a < 3; ++a) {
-        double w = wcb * wx[a];
-        int kk = kp + c - 1, jj = jp + b - 1, ii = ip + a - 1;
-        atomicAdd(&qdep[d.at(m, 5, 0, kk, jj, ii)], w);
-        atomicAdd(&qdep[d.at(m, 5, 1, kk, jj, ii)], w * vx);
-        atomicAdd(&qdep[d.at(m, 5, 2, kk, jj, ii)], w * vy);
-        atomicAdd(&qdep[d.at(m, 5, 3, kk, jj, ii)], w * vz);
+// ---- deposits: a warp's particles combined per cell (dustb_deposit.cuh) -------------------
+// a depositing particle: its block, anchor cell, weights and staged values
+struct Stencil {
+  int m, ip, jp, kp;
+  double wx[3], wy[3], wz[3], q[4];
+};
+
+// every particle of the launch through particle(p, stencil), which returns whether it deposits,
+// and its deposit into variable v0 on of an nvar-variable field
+template <int NV, bool FAC, bool ONE, typename F>
+__device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &d, double *field,
+                                                  int nvar, int v0, F &&particle) {
+  __shared__ WarpStage s_stage[kDepWarps];
+  WarpStage &st = s_stage[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  CellDeposit<NV, FAC, ONE> dep;
+  dep.init(field, d);
+  const long long first = ((long long)blockIdx.x * kDepWarps + (threadIdx.x >> 5)) * nb * 32;
+  for (int b = 0; b < nb; ++b) {
+    const long long p0 = first + 32LL * b;
+    if (p0 >= npart) break;
+    unsigned key = kNoCell;
+    long long kb = 0;
+    bool live = false;
+    if (p0 + lane < npart) {
+      Stencil t;
+      live = particle((int)(p0 + lane), t);
+      if (live) {
+        key = (unsigned)d.at(t.m, 1, 0, t.kp, t.jp, t.ip);   // (below 2^32: one GPU's memory)
+        kb = d.at(t.m, nvar, v0, t.kp, t.jp, t.ip);
+        st.put(lane, t.wx, t.wy, t.wz, t.q[0], t.q[1], t.q[2], t.q[3]);
       }
     }
+    __syncwarp();
+    dep.batch(st, key, kb, live);
+    __syncwarp();
+  }
+  dep.flush();
+}
+
+// the gather of a 3-variable field with the particle's weights, in the reference's order
+__device__ __forceinline__ void gather3(const Ind &d, const Stencil &t, const double *f,
+                                        double &g0, double &g1, double &g2) {
+  g0 = g1 = g2 = 0.0;
+  const int clo = d.three_d ? 0 : 1, chi = d.three_d ? 2 : 1;
+  const long long vs = d.cells();
+  for (int c = clo; c <= chi; ++c)
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const double wcb = t.wz[c] * t.wy[b];
+      if (wcb == 0.0) continue;
+      const double *r = f + d.at(t.m, 3, 0, t.kp + c - 1, t.jp + b - 1, t.ip - 1);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const double w = wcb * t.wx[a];
+        g0 += w * r[a];
+        g1 += w * r[a + vs];
+        g2 += w * r[a + 2 * vs];
+      }
+    }
+}
+
+// the block, anchor cell and weights of a position; false (and the error bit) outside the pack
+// or the block's halo
+__device__ __forceinline__ bool place(const PCtx &P, const MCtx &M, const Ind &d, int p, double x,
+                                      double y, double z, Stencil &t, unsigned *err) {
+  t.m = P.i(DUSTB_PGID, p) - M.gids;
+  if (!block_ok(d, t.m)) { report(err, DUSTB_ERR_PGID); return false; }
+  weights3(M, d, t.m, x, y, z, t.ip, t.jp, t.kp, t.wx, t.wy, t.wz);
+  if (!halo_ok(d, t.ip, t.jp, t.kp)) { report(err, DUSTB_ERR_HALO); return false; }
+  return true;
+}
+
+// ---- DepositDrag imex scatter, src/dust/dust_pm.cpp:225-274 ------------------------------
+__global__ void __launch_bounds__(32 * kDepWarps)
+k_scatter(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh, unsigned *err, int nb) {
+  deposit_particles<4, true, true>(P.npart, nb, d, qdep, 5, 0, [&](int p, Stencil &t) {
+    const double x = P.r(DUSTB_IPX, p);
+    if (!place(P, M, d, p, x, P.r(DUSTB_IPY, p) + sh * x, P.r(DUSTB_IPZ, p), t, err)) return false;
+    const double vol = cell_vol(M, d, t.m);
+    const double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
+    t.q[0] = P.r(DUSTB_IPM, p) * cj / vol;
+    t.q[1] = P.r(DUSTB_IPVX, p); t.q[2] = P.r(DUSTB_IPVY, p); t.q[3] = P.r(DUSTB_IPVZ, p);
+    return true;
+  });
 }
 
 // ---- ghost exchanges (pull form, one thread per destination cell) -----------------------
@@ -720,45 +776,18 @@ __global__ void k_solve_ustar(Ind d, const double *u0, int nv, const double *qde
 }
 
 // ---- PointOperatorParticles, src/dust/dust_solver.cpp:151-201 ---------------------------
-__global__ void k_operator(PCtx P, MCtx M, Ind d, const double *field, double *result,
-                           double a_dt, double sh, unsigned *err) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
-  int m = P.i(DUSTB_PGID, p) - M.gids;
-  if (!block_ok(d, m)) { report(err, DUSTB_ERR_PGID); return; }
-  int ip, jp, kp; double wx[3], wy[3], wz[3];
-  weights3(M, d, m, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p) + sh * P.r(DUSTB_IPX, p),
-           P.r(DUSTB_IPZ, p), ip, jp, kp, wx, wy, wz);
-  if (!halo_ok(d, ip, jp, kp)) { report(err, DUSTB_ERR_HALO); return; }
-  double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-  int clo = d.three_d ? 0 : 1, chi = d.three_d ? 2 : 1;
-  for (int c = clo; c <= chi; ++c)
-    for (int b = 0; b < 3; ++b) {
-      double wcb = wz[c] * wy[b];
-      if (wcb == 0.0) continue;
-      for (int a = 0; a < 3; ++a) {
-        double w = wcb * wx[a];
-        int kk = kp + c - 1, jj = jp + b - 1, ii = ip + a - 1;
-        g0 += w * field[d.at(m, 3, 0, kk, jj, ii)];
-        g1 += w * field[d.at(m, 3, 1, kk, jj, ii)];
-        g2 += w * field[d.at(m, 3, 2, kk, jj, ii)];
-      }
-    }
-  double vol = cell_vol(M, d, m);
-  double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
-  double fac = P.r(DUSTB_IPM, p) * cj / vol;
-  for (int c = clo; c <= chi; ++c)
-    for (int b = 0; b < 3; ++b) {
-      double wcb = wz[c] * wy[b] * fac;
-      if (wcb == 0.0) continue;
-      for (int a = 0; a < 3; ++a) {
-        double w = wcb * wx[a];
-        int kk = kp + c - 1, jj = jp + b - 1, ii = ip + a - 1;
-        atomicAdd(&result[d.at(m, 3, 0, kk, jj, ii)], w * g0);
-        atomicAdd(&result[d.at(m, 3, 1, kk, jj, ii)], w * g1);
-        atomicAdd(&result[d.at(m, 3, 2, kk, jj, ii)], w * g2);
-      }
-    }
+__global__ void __launch_bounds__(32 * kDepWarps)
+k_operator(PCtx P, MCtx M, Ind d, const double *field, double *result, double a_dt, double sh,
+           unsigned *err, int nb) {
+  deposit_particles<3, true, false>(P.npart, nb, d, result, 3, 0, [&](int p, Stencil &t) {
+    const double x = P.r(DUSTB_IPX, p);
+    if (!place(P, M, d, p, x, P.r(DUSTB_IPY, p) + sh * x, P.r(DUSTB_IPZ, p), t, err)) return false;
+    gather3(d, t, field, t.q[1], t.q[2], t.q[3]);
+    const double vol = cell_vol(M, d, t.m);
+    const double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
+    t.q[0] = P.r(DUSTB_IPM, p) * cj / vol;
+    return true;
+  });
 }
 
 // dust_applya_dc, src/dust/dust_solver.cpp:243-252
@@ -777,51 +806,24 @@ __global__ void k_dc_correct(Ind d, const double *u0, int nv, const double *qdep
 }
 
 // ---- GatherKickPMBR, src/dust/dust_pm.cpp:500-564 ----------------------------------------
-__global__ void k_gather_kick(PCtx P, MCtx M, Ind d, const double *us, double *dmom, double a_dt,
-                              double sh, int br, unsigned *err) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
-  int m = P.i(DUSTB_PGID, p) - M.gids;
-  if (!block_ok(d, m)) { report(err, DUSTB_ERR_PGID); return; }
-  int ip, jp, kp; double wx[3], wy[3], wz[3];
-  weights3(M, d, m, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p) + sh * P.r(DUSTB_IPX, p),
-           P.r(DUSTB_IPZ, p), ip, jp, kp, wx, wy, wz);
-  if (!halo_ok(d, ip, jp, kp)) { report(err, DUSTB_ERR_HALO); return; }
-  double ux = 0.0, uy = 0.0, uz = 0.0;
-  int clo = d.three_d ? 0 : 1, chi = d.three_d ? 2 : 1;
-  for (int c = clo; c <= chi; ++c)
-    for (int b = 0; b < 3; ++b) {
-      double wcb = wz[c] * wy[b];
-      if (wcb == 0.0) continue;
-      for (int a = 0; a < 3; ++a) {
-        double w = wcb * wx[a];
-        int kk = kp + c - 1, jj = jp + b - 1, ii = ip + a - 1;
-        ux += w * us[d.at(m, 3, 0, kk, jj, ii)];
-        uy += w * us[d.at(m, 3, 1, kk, jj, ii)];
-        uz += w * us[d.at(m, 3, 2, kk, jj, ii)];
-      }
-    }
-  double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
-  double dvx = cj * (ux - P.r(DUSTB_IPVX, p));
-  double dvy = cj * (uy - P.r(DUSTB_IPVY, p));
-  double dvz = cj * (uz - P.r(DUSTB_IPVZ, p));
-  P.r(DUSTB_IPVX, p) += dvx; P.r(DUSTB_IPVY, p) += dvy; P.r(DUSTB_IPVZ, p) += dvz;
-  P.r(DUSTB_IPRX, p) = dvx / a_dt; P.r(DUSTB_IPRY, p) = dvy / a_dt; P.r(DUSTB_IPRZ, p) = dvz / a_dt;
-  if (!br) return;
-  double vol = cell_vol(M, d, m);
-  double fac = -P.r(DUSTB_IPM, p) / vol;
-  for (int c = clo; c <= chi; ++c)
-    for (int b = 0; b < 3; ++b) {
-      double wcb = wz[c] * wy[b] * fac;
-      if (wcb == 0.0) continue;
-      for (int a = 0; a < 3; ++a) {
-        double w = wcb * wx[a];
-        int kk = kp + c - 1, jj = jp + b - 1, ii = ip + a - 1;
-        atomicAdd(&dmom[d.at(m, 3, 0, kk, jj, ii)], w * dvx);
-        atomicAdd(&dmom[d.at(m, 3, 1, kk, jj, ii)], w * dvy);
-        atomicAdd(&dmom[d.at(m, 3, 2, kk, jj, ii)], w * dvz);
-      }
-    }
+__global__ void __launch_bounds__(32 * kDepWarps)
+k_gather_kick(PCtx P, MCtx M, Ind d, const double *us, double *dmom, double a_dt, double sh, int br,
+              unsigned *err, int nb) {
+  deposit_particles<3, true, false>(P.npart, nb, d, dmom, 3, 0, [&](int p, Stencil &t) {
+    const double x = P.r(DUSTB_IPX, p);
+    if (!place(P, M, d, p, x, P.r(DUSTB_IPY, p) + sh * x, P.r(DUSTB_IPZ, p), t, err)) return false;
+    double ux, uy, uz;
+    gather3(d, t, us, ux, uy, uz);
+    const double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
+    const double vx = P.r(DUSTB_IPVX, p), vy = P.r(DUSTB_IPVY, p), vz = P.r(DUSTB_IPVZ, p);
+    const double dvx = cj * (ux - vx), dvy = cj * (uy - vy), dvz = cj * (uz - vz);
+    P.r(DUSTB_IPVX, p) = vx + dvx; P.r(DUSTB_IPVY, p) = vy + dvy; P.r(DUSTB_IPVZ, p) = vz + dvz;
+    P.r(DUSTB_IPRX, p) = dvx / a_dt; P.r(DUSTB_IPRY, p) = dvy / a_dt; P.r(DUSTB_IPRZ, p) = dvz / a_dt;
+    if (!br) return false;
+    t.q[0] = -P.r(DUSTB_IPM, p) / cell_vol(M, d, t.m);
+    t.q[1] = dvx; t.q[2] = dvy; t.q[3] = dvz;
+    return true;
+  });
 }
 
 // ---- ApplyPMBR, src/dust/dust_pm.cpp:649-708 ---------------------------------------------
@@ -837,15 +839,41 @@ __device__ __forceinline__ bool center_cell(const PCtx &P, const MCtx &M, const 
   return halo_ok(d, ip, jp, kp);
 }
 
+// the sum of v over the lanes of a warp, in every lane
+__device__ __forceinline__ double warp_total(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// (the particles of a warp that share a centre cell add once: rows in cell order put a cell's
+// particles next to each other, where one atomic per particle would queue up on its address)
 __global__ void k_center_mass(PCtx P, MCtx M, Ind d, double *res, double a_dt, unsigned *err) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
-  if (P.r(DUSTB_IPM, p) <= 0.0) return;
-  int m, ip, jp, kp;
-  if (!center_cell(P, M, d, p, m, ip, jp, kp)) { report(err, DUSTB_ERR_HALO); return; }
-  double vol = cell_vol(M, d, m);
-  atomicAdd(&res[d.at(m, 4, 3, kp, jp, ip)],
-            P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt)) / vol);
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  long long at = -1;
+  double mc = 0.0;
+  if (p < P.npart && !(P.r(DUSTB_IPM, p) <= 0.0)) {
+    int m, ip, jp, kp;
+    if (!center_cell(P, M, d, p, m, ip, jp, kp)) {
+      report(err, DUSTB_ERR_HALO);
+    } else {
+      at = d.at(m, 4, 3, kp, jp, ip);
+      mc = P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt)) / cell_vol(M, d, m);
+    }
+  }
+  unsigned rem = __ballot_sync(0xffffffffu, at >= 0);
+  while (rem) {
+    const int lead = __ffs(rem) - 1;
+    const long long k = __shfl_sync(0xffffffffu, at, lead);
+    const unsigned grp = __ballot_sync(0xffffffffu, at == k) & rem;
+    rem &= ~grp;
+    if (grp == (1u << lead)) {
+      if ((int)(threadIdx.x & 31) == lead) atomicAdd(&res[at], mc);
+    } else {
+      const double t = warp_total(at == k ? mc : 0.0);
+      if ((int)(threadIdx.x & 31) == lead) atomicAdd(&res[at], t);
+    }
+  }
 }
 
 __global__ void k_consistent_gas(Ind d, double *u0, int nv, const double *us, const double *qdep,
@@ -945,48 +973,38 @@ __global__ void k_tstop(PCtx P, double *out, unsigned *err) {
 
 // ---- pc2 ---------------------------------------------------------------------------------
 // DepositDrag pc2 predictor, src/dust/dust_pm.cpp:141-193
-__global__ void k_pc2_predictor(PCtx P, MCtx M, Ind d, const double *uold, int nv, double *qdep,
-                                double dt, int rate_dep, unsigned *err) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
-  int m = P.i(DUSTB_PGID, p) - M.gids;
-  if (!block_ok(d, m)) { report(err, DUSTB_ERR_PGID); return; }
-  int ip, jp, kp; double wx[3], wy[3], wz[3];
-  weights3(M, d, m, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p), P.r(DUSTB_IPZ, p), ip, jp, kp, wx, wy, wz);
-  if (!halo_ok(d, ip, jp, kp)) { report(err, DUSTB_ERR_HALO); return; }
-  double ugx = 0.0, ugy = 0.0, ugz = 0.0;
-  int clo = d.three_d ? 0 : 1, chi = d.three_d ? 2 : 1;
-  for (int c = clo; c <= chi; ++c)
-    for (int b = 0; b < 3; ++b) {
-      double wcb = wz[c] * wy[b];
-      if (wcb == 0.0) continue;
-      for (int a = 0; a < 3; ++a) {
-        double w = wcb * wx[a];
-        int kk = kp + c - 1, jj = jp + b - 1, ii = ip + a - 1;
-        double invrho = 1.0 / uold[d.at(m, nv, 0, kk, jj, ii)];
-        ugx += w * uold[d.at(m, nv, 1, kk, jj, ii)] * invrho;
-        ugy += w * uold[d.at(m, nv, 2, kk, jj, ii)] * invrho;
-        ugz += w * uold[d.at(m, nv, 3, kk, jj, ii)] * invrho;
+__global__ void __launch_bounds__(32 * kDepWarps)
+k_pc2_predictor(PCtx P, MCtx M, Ind d, const double *uold, int nv, double *qdep, double dt,
+                int rate_dep, unsigned *err, int nb) {
+  deposit_particles<4, false, false>(P.npart, nb, d, qdep, 5, 1, [&](int p, Stencil &t) {
+    if (!place(P, M, d, p, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p), P.r(DUSTB_IPZ, p), t, err))
+      return false;
+    double ugx = 0.0, ugy = 0.0, ugz = 0.0;
+    const int clo = d.three_d ? 0 : 1, chi = d.three_d ? 2 : 1;
+    const long long vs = d.cells();
+    for (int c = clo; c <= chi; ++c)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        const double wcb = t.wz[c] * t.wy[b];
+        if (wcb == 0.0) continue;
+        const double *r = uold + d.at(t.m, nv, 0, t.kp + c - 1, t.jp + b - 1, t.ip - 1);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const double w = wcb * t.wx[a];
+          const double invrho = 1.0 / r[a];
+          ugx += w * r[a + vs] * invrho;
+          ugy += w * r[a + 2 * vs] * invrho;
+          ugz += w * r[a + 3 * vs] * invrho;
+        }
       }
-    }
-  double vol = cell_vol(M, d, m);
-  double rate = P.r(DUSTB_IPM, p) / (P.r(DUSTB_IPTS, p) * vol);
-  double gx = -dt * rate * (ugx - P.r(DUSTB_IPVX, p));
-  double gy = -dt * rate * (ugy - P.r(DUSTB_IPVY, p));
-  double gz = -dt * rate * (ugz - P.r(DUSTB_IPVZ, p));
-  for (int c = clo; c <= chi; ++c)
-    for (int b = 0; b < 3; ++b) {
-      double wcb = wz[c] * wy[b];
-      if (wcb == 0.0) continue;
-      for (int a = 0; a < 3; ++a) {
-        double w = wcb * wx[a];
-        int kk = kp + c - 1, jj = jp + b - 1, ii = ip + a - 1;
-        atomicAdd(&qdep[d.at(m, 5, 1, kk, jj, ii)], w * gx);
-        atomicAdd(&qdep[d.at(m, 5, 2, kk, jj, ii)], w * gy);
-        atomicAdd(&qdep[d.at(m, 5, 3, kk, jj, ii)], w * gz);
-        if (rate_dep) atomicAdd(&qdep[d.at(m, 5, 4, kk, jj, ii)], w * rate);
-      }
-    }
+    const double vol = cell_vol(M, d, t.m);
+    const double rate = P.r(DUSTB_IPM, p) / (P.r(DUSTB_IPTS, p) * vol);
+    t.q[0] = -dt * rate * (ugx - P.r(DUSTB_IPVX, p));
+    t.q[1] = -dt * rate * (ugy - P.r(DUSTB_IPVY, p));
+    t.q[2] = -dt * rate * (ugz - P.r(DUSTB_IPVZ, p));
+    t.q[3] = rate_dep ? rate : 0.0;
+    return true;
+  });
 }
 
 // UpdateStiffness's maximum of qdep4/rho (dust_pm.cpp:295-301), before the damping
@@ -1029,85 +1047,58 @@ __global__ void k_pc2_midpoint(Ind d, const double *u0, const double *u1, int nv
 }
 
 // dust_pc2_advance, src/dust/dust_push.cpp:132-245
-__global__ void k_pc2_advance(PCtx P, MCtx M, Ind d, const double *us, double *dmom, double dt,
-                              int br, int sbox, int strat, double q, double om, double aphi,
-                              unsigned *err) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
-  int m = P.i(DUSTB_PGID, p) - M.gids;
-  if (!block_ok(d, m)) { report(err, DUSTB_ERR_PGID); return; }
-  const bool three_d = d.three_d;
-  double x0 = P.r(DUSTB_IPX1, p), y0 = P.r(DUSTB_IPY1, p), z0 = P.r(DUSTB_IPZ1, p);
-  double vx0 = P.r(DUSTB_IPVX1, p), vy0 = P.r(DUSTB_IPVY1, p), vz0 = P.r(DUSTB_IPVZ1, p);
-  double xh = x0 + 0.5 * dt * vx0;
-  double yh = y0 + 0.5 * dt * (vy0 - ((sbox && three_d) ? q * om * x0 : 0.0));
-  double zh = three_d ? z0 + 0.5 * dt * vz0 : z0;
-  double yg = yh + ((sbox && three_d) ? q * om * xh * 0.5 * dt : 0.0);
-  int ip, jp, kp; double wx[3], wy[3], wz[3];
-  weights3(M, d, m, xh, yg, zh, ip, jp, kp, wx, wy, wz);
-  if (!halo_ok(d, ip, jp, kp)) { report(err, DUSTB_ERR_HALO); return; }
-  double ugx = 0.0, ugy = 0.0, ugz = 0.0;
-  int clo = three_d ? 0 : 1, chi = three_d ? 2 : 1;
-  for (int c = clo; c <= chi; ++c)
-    for (int b = 0; b < 3; ++b) {
-      double wcb = wz[c] * wy[b];
-      if (wcb == 0.0) continue;
-      for (int a = 0; a < 3; ++a) {
-        double w = wcb * wx[a];
-        int kk = kp + c - 1, jj = jp + b - 1, ii = ip + a - 1;
-        ugx += w * us[d.at(m, 3, 0, kk, jj, ii)];
-        ugy += w * us[d.at(m, 3, 1, kk, jj, ii)];
-        ugz += w * us[d.at(m, 3, 2, kk, jj, ii)];
-      }
+__global__ void __launch_bounds__(32 * kDepWarps)
+k_pc2_advance(PCtx P, MCtx M, Ind d, const double *us, double *dmom, double dt, int br, int sbox,
+              int strat, double q, double om, double aphi, unsigned *err, int nb) {
+  deposit_particles<3, true, false>(P.npart, nb, d, dmom, 3, 0, [&](int p, Stencil &t) {
+    const bool three_d = d.three_d;
+    double x0 = P.r(DUSTB_IPX1, p), y0 = P.r(DUSTB_IPY1, p), z0 = P.r(DUSTB_IPZ1, p);
+    double vx0 = P.r(DUSTB_IPVX1, p), vy0 = P.r(DUSTB_IPVY1, p), vz0 = P.r(DUSTB_IPVZ1, p);
+    double xh = x0 + 0.5 * dt * vx0;
+    double yh = y0 + 0.5 * dt * (vy0 - ((sbox && three_d) ? q * om * x0 : 0.0));
+    double zh = three_d ? z0 + 0.5 * dt * vz0 : z0;
+    double yg = yh + ((sbox && three_d) ? q * om * xh * 0.5 * dt : 0.0);
+    if (!place(P, M, d, p, xh, yg, zh, t, err)) return false;
+    double ugx, ugy, ugz;
+    gather3(d, t, us, ugx, ugy, ugz);
+    double h = 0.5 * dt;
+    double lambda = h / P.r(DUSTB_IPTS, p);
+    double aa = 1.0 + lambda;
+    double rx = vx0 + lambda * ugx, ry = vy0 + lambda * ugy, rz = vz0 + lambda * ugz;
+    double vxh, vyh, vzh;
+    if (sbox && three_d) {
+      double cxy = 2.0 * h * om, cyx = h * (2.0 - q) * om;
+      double det = aa * aa + cxy * cyx;
+      vxh = (aa * rx + cxy * ry) / det;
+      vyh = (aa * ry - cyx * rx) / det;
+      if (strat) rz -= h * (om * om) * zh;
+      vzh = rz / aa;
+    } else if (sbox) {
+      double cxz = 2.0 * h * om, czx = h * (2.0 - q) * om;
+      double det = aa * aa + cxz * czx;
+      if (aphi != 0.0) rz += h * aphi;
+      vxh = (aa * rx + cxz * rz) / det;
+      vzh = (aa * rz - czx * rx) / det;
+      vyh = ry / aa;
+    } else {
+      vxh = rx / aa; vyh = ry / aa; vzh = rz / aa;
     }
-  double h = 0.5 * dt;
-  double lambda = h / P.r(DUSTB_IPTS, p);
-  double aa = 1.0 + lambda;
-  double rx = vx0 + lambda * ugx, ry = vy0 + lambda * ugy, rz = vz0 + lambda * ugz;
-  double vxh, vyh, vzh;
-  if (sbox && three_d) {
-    double cxy = 2.0 * h * om, cyx = h * (2.0 - q) * om;
-    double det = aa * aa + cxy * cyx;
-    vxh = (aa * rx + cxy * ry) / det;
-    vyh = (aa * ry - cyx * rx) / det;
-    if (strat) rz -= h * (om * om) * zh;
-    vzh = rz / aa;
-  } else if (sbox) {
-    double cxz = 2.0 * h * om, czx = h * (2.0 - q) * om;
-    double det = aa * aa + cxz * czx;
-    if (aphi != 0.0) rz += h * aphi;
-    vxh = (aa * rx + cxz * rz) / det;
-    vzh = (aa * rz - czx * rx) / det;
-    vyh = ry / aa;
-  } else {
-    vxh = rx / aa; vyh = ry / aa; vzh = rz / aa;
-  }
-  P.r(DUSTB_IPVX, p) = 2.0 * vxh - vx0;
-  P.r(DUSTB_IPVY, p) = 2.0 * vyh - vy0;
-  P.r(DUSTB_IPVZ, p) = 2.0 * vzh - vz0;
-  P.r(DUSTB_IPX, p) = x0 + dt * vxh;
-  P.r(DUSTB_IPY, p) = y0 + dt * (vyh - ((sbox && three_d) ? q * om * xh : 0.0));
-  if (three_d) P.r(DUSTB_IPZ, p) = z0 + dt * vzh;
-  P.r(DUSTB_IPX1, p) = xh; P.r(DUSTB_IPY1, p) = yh; P.r(DUSTB_IPZ1, p) = zh;
-  double dvx = dt * (ugx - vxh) / P.r(DUSTB_IPTS, p);
-  double dvy = dt * (ugy - vyh) / P.r(DUSTB_IPTS, p);
-  double dvz = dt * (ugz - vzh) / P.r(DUSTB_IPTS, p);
-  P.r(DUSTB_IPRX, p) = dvx; P.r(DUSTB_IPRY, p) = dvy; P.r(DUSTB_IPRZ, p) = dvz;
-  if (!br) return;
-  double vol = cell_vol(M, d, m);
-  double fac = -P.r(DUSTB_IPM, p) / vol;
-  for (int c = clo; c <= chi; ++c)
-    for (int b = 0; b < 3; ++b) {
-      double wcb = wz[c] * wy[b] * fac;
-      if (wcb == 0.0) continue;
-      for (int a = 0; a < 3; ++a) {
-        double w = wcb * wx[a];
-        int kk = kp + c - 1, jj = jp + b - 1, ii = ip + a - 1;
-        atomicAdd(&dmom[d.at(m, 3, 0, kk, jj, ii)], w * dvx);
-        atomicAdd(&dmom[d.at(m, 3, 1, kk, jj, ii)], w * dvy);
-        atomicAdd(&dmom[d.at(m, 3, 2, kk, jj, ii)], w * dvz);
-      }
-    }
+    P.r(DUSTB_IPVX, p) = 2.0 * vxh - vx0;
+    P.r(DUSTB_IPVY, p) = 2.0 * vyh - vy0;
+    P.r(DUSTB_IPVZ, p) = 2.0 * vzh - vz0;
+    P.r(DUSTB_IPX, p) = x0 + dt * vxh;
+    P.r(DUSTB_IPY, p) = y0 + dt * (vyh - ((sbox && three_d) ? q * om * xh : 0.0));
+    if (three_d) P.r(DUSTB_IPZ, p) = z0 + dt * vzh;
+    P.r(DUSTB_IPX1, p) = xh; P.r(DUSTB_IPY1, p) = yh; P.r(DUSTB_IPZ1, p) = zh;
+    double dvx = dt * (ugx - vxh) / P.r(DUSTB_IPTS, p);
+    double dvy = dt * (ugy - vyh) / P.r(DUSTB_IPTS, p);
+    double dvz = dt * (ugz - vzh) / P.r(DUSTB_IPTS, p);
+    P.r(DUSTB_IPRX, p) = dvx; P.r(DUSTB_IPRY, p) = dvy; P.r(DUSTB_IPRZ, p) = dvz;
+    if (!br) return false;
+    t.q[0] = -P.r(DUSTB_IPM, p) / cell_vol(M, d, t.m);
+    t.q[1] = dvx; t.q[2] = dvy; t.q[3] = dvz;
+    return true;
+  });
 }
 
 // dust_pc2_commit, dust_pm.cpp:596-601
@@ -1159,24 +1150,17 @@ __global__ void k_phst_sums(const double *part, int nchunk, const double *chi, i
 
 // the mass component of DepositPointScienceFields (src/dust/dust_gravity_points.cpp:277-304):
 // m/V with the deposit weights into the block's cells, ghost cells included
-__global__ void k_mass_deposit(PCtx P, MCtx M, Ind d, double *f, unsigned *err) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
-  const double mass = P.r(DUSTB_IPM, p);
-  if (mass == 0.0) return;
-  const int m = P.i(DUSTB_PGID, p) - M.gids;
-  if (!block_ok(d, m)) { report(err, DUSTB_ERR_PGID); return; }
-  int ip, jp, kp; double wx[3], wy[3], wz[3];
-  weights3(M, d, m, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p), P.r(DUSTB_IPZ, p), ip, jp, kp, wx, wy, wz);
-  if (!halo_ok(d, ip, jp, kp)) { report(err, DUSTB_ERR_HALO); return; }
-  const double density = mass / cell_vol(M, d, m);
-  for (int c = 0; c < 3; ++c)
-    for (int b = 0; b < 3; ++b)
-      for (int a = 0; a < 3; ++a) {
-        const double w = density * wz[c] * wy[b] * wx[a];
-        if (w == 0.0) continue;
-        atomicAdd(&f[d.at(m, 1, 0, kp + c - 1, jp + b - 1, ip + a - 1)], w);
-      }
+__global__ void __launch_bounds__(32 * kDepWarps)
+k_mass_deposit(PCtx P, MCtx M, Ind d, double *f, unsigned *err, int nb) {
+  deposit_particles<1, true, true>(P.npart, nb, d, f, 1, 0, [&](int p, Stencil &t) {
+    const double mass = P.r(DUSTB_IPM, p);
+    if (mass == 0.0) return false;
+    if (!place(P, M, d, p, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p), P.r(DUSTB_IPZ, p), t, err))
+      return false;
+    t.q[0] = mass / cell_vol(M, d, t.m);
+    t.q[1] = t.q[2] = t.q[3] = 0.0;
+    return true;
+  });
 }
 
 // the densest active cell (dust_science.cpp:428-441): per block of threads the largest value
@@ -1250,35 +1234,30 @@ __device__ __forceinline__ bool point_stencil(const PCtx &P, const MCtx &M, cons
 // DepositPointGravityDensity (:215-245; gravity = 1: density only, mass >= 0) and
 // DepositPointScienceFields (:257-304; ncomp 1 or 4: m/V and m v/V, one species or all):
 // the density with the deposit weights into the owner block's cells, ghost cells included
-__global__ void k_point_deposit(PCtx P, MCtx M, Ind d, double *f, int ncomp, int species,
-                                int gravity, unsigned *err) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
-  const double mass = P.r(DUSTB_IPM, p);
-  if (gravity) {
-    if (!(mass >= 0.0) || !isfinite(mass)) { report(err, DUSTB_ERR_POINT); return; }
-    if (mass == 0.0) return;
-  } else {
-    if (mass == 0.0) return;
-    if (species >= 0 && P.i(DUSTB_PSP, p) != species) return;
-    if (!isfinite(mass)) { report(err, DUSTB_ERR_POINT); return; }
-  }
-  int m, ip, jp, kp; double wx[3], wy[3], wz[3];
-  if (!point_stencil(P, M, d, p, m, ip, jp, kp, wx, wy, wz)) { report(err, DUSTB_ERR_POINT); return; }
-  const double density = mass / (M.s(m, DX1) * M.s(m, DX2) * M.s(m, DX3));
-  const double v1 = P.r(DUSTB_IPVX, p), v2 = P.r(DUSTB_IPVY, p), v3 = P.r(DUSTB_IPVZ, p);
-  for (int c = 0; c < 3; ++c)
-    for (int b = 0; b < 3; ++b)
-      for (int a = 0; a < 3; ++a) {
-        const double w = density * wz[c] * wy[b] * wx[a];
-        if (w == 0.0) continue;
-        const int kk = kp + c - 1, jj = jp + b - 1, ii = ip + a - 1;
-        atomicAdd(&f[d.at(m, ncomp, 0, kk, jj, ii)], w);
-        if (ncomp == 1) continue;
-        atomicAdd(&f[d.at(m, ncomp, 1, kk, jj, ii)], w * v1);
-        atomicAdd(&f[d.at(m, ncomp, 2, kk, jj, ii)], w * v2);
-        atomicAdd(&f[d.at(m, ncomp, 3, kk, jj, ii)], w * v3);
-      }
+template <int NCOMP>
+__global__ void __launch_bounds__(32 * kDepWarps)
+k_point_deposit(PCtx P, MCtx M, Ind d, double *f, int species, int gravity, unsigned *err, int nb) {
+  deposit_particles<NCOMP, true, true>(P.npart, nb, d, f, NCOMP, 0, [&](int p, Stencil &t) {
+    const double mass = P.r(DUSTB_IPM, p);
+    if (gravity) {
+      if (!(mass >= 0.0) || !isfinite(mass)) { report(err, DUSTB_ERR_POINT); return false; }
+      if (mass == 0.0) return false;
+    } else {
+      if (mass == 0.0) return false;
+      if (species >= 0 && P.i(DUSTB_PSP, p) != species) return false;
+      if (!isfinite(mass)) { report(err, DUSTB_ERR_POINT); return false; }
+    }
+    if (!point_stencil(P, M, d, p, t.m, t.ip, t.jp, t.kp, t.wx, t.wy, t.wz)) {
+      report(err, DUSTB_ERR_POINT);
+      return false;
+    }
+    t.q[0] = mass / (M.s(t.m, DX1) * M.s(t.m, DX2) * M.s(t.m, DX3));
+    t.q[1] = t.q[2] = t.q[3] = 0.0;
+    if (NCOMP > 1) {
+      t.q[1] = P.r(DUSTB_IPVX, p); t.q[2] = P.r(DUSTB_IPVY, p); t.q[3] = P.r(DUSTB_IPVZ, p);
+    }
+    return true;
+  });
 }
 
 // the remapped field's active cells, the ghost cells zero (:246-248, :297-304)
@@ -2610,6 +2589,9 @@ bool ctx_valid(const dustb_ctx *c) { return ctx_cells_ok(c); }
 #define CHECK_CTX(c) do { if (!ctx_ok(c)) { return DUSTB_EINVAL; } } while (0)
 #define CHECK_CELLS(c) do { if (!ctx_cells_ok(c)) { return DUSTB_EINVAL; } } while (0)
 #define PGRID(c) blocks_for((c)->part.npart), kThreads, 0, S(stream)
+// the depositing kernels: nb batches of 32 particles per warp
+#define DGRID(c, nb) dep_blocks((c)->part.npart, nb), 32 * kDepWarps, 0, S(stream)
+#define NB(c) dep_batches((c)->part.npart)
 
 extern "C" {
 
@@ -2668,7 +2650,7 @@ int dustb_deposit_qp(const dustb_ctx *c, double a_dt, double sh, void *stream) {
   Ind d = make_ind(c->mesh);
   cudaMemsetAsync(c->f.qdep, 0, (size_t)n_all(d) * 5 * sizeof(double), S(stream));
   if (c->part.npart > 0)
-    k_scatter<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, c->err);
+    k_scatter<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, c->err, NB(c));
   return launch_status("deposit_qp");
 }
 
@@ -2737,7 +2719,7 @@ int dustb_dc1_sweep(const dustb_ctx *c, double a_dt, double sh, void *stream) {
   if (rc) return rc;
   cudaMemsetAsync(c->f.work, 0, (size_t)n_all(d) * 3 * sizeof(double), S(stream));
   if (c->part.npart > 0)
-    k_operator<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.ustar, c->f.work, a_dt, sh, c->err);
+    k_operator<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.ustar, c->f.work, a_dt, sh, c->err, NB(c));
   rc = dustb_ghost_add(c, c->f.work, 3, stream);
   if (rc) return rc;
   k_dc_correct<<<blocks_for(n_active(d)), kThreads, 0, S(stream)>>>(d, c->f.u0, c->f.nvar_gas, c->f.qdep,
@@ -2751,7 +2733,7 @@ int dustb_gather_kick_pmbr(const dustb_ctx *c, double a_dt, double sh, void *str
   const int br = c->phys.back_reaction;
   if (br) cudaMemsetAsync(c->f.dmom, 0, (size_t)n_all(d) * 3 * sizeof(double), S(stream));
   if (c->part.npart > 0)
-    k_gather_kick<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.ustar, c->f.dmom, a_dt, sh, br, c->err);
+    k_gather_kick<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.ustar, c->f.dmom, a_dt, sh, br, c->err, NB(c));
   return launch_status("gather_kick_pmbr");
 }
 
@@ -2799,8 +2781,8 @@ int dustb_pc2_predictor(const dustb_ctx *c, double dt, int rate_dep, void *strea
   Ind d = make_ind(c->mesh);
   cudaMemsetAsync(c->f.qdep, 0, (size_t)n_all(d) * 5 * sizeof(double), S(stream));
   if (c->part.npart > 0)
-    k_pc2_predictor<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.u1, c->f.nvar_gas, c->f.qdep, dt,
-                                  rate_dep, c->err);
+    k_pc2_predictor<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.u1, c->f.nvar_gas, c->f.qdep, dt,
+                                  rate_dep, c->err, NB(c));
   return launch_status("pc2_predictor");
 }
 
@@ -2830,9 +2812,9 @@ int dustb_pc2_advance(const dustb_ctx *c, double dt, void *stream) {
   const int br = c->phys.back_reaction;
   if (br) cudaMemsetAsync(c->f.dmom, 0, (size_t)n_all(d) * 3 * sizeof(double), S(stream));
   if (c->part.npart > 0)
-    k_pc2_advance<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.ustar, c->f.dmom, dt, br,
+    k_pc2_advance<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.ustar, c->f.dmom, dt, br,
                                 c->phys.shearing_box, c->phys.stratified, c->phys.qshear,
-                                c->phys.omega0, c->phys.const_accel_phi, c->err);
+                                c->phys.omega0, c->phys.const_accel_phi, c->err, NB(c));
   return launch_status("pc2_advance");
 }
 
@@ -2872,7 +2854,7 @@ int dustb_phst(const dustb_ctx *c, const double *chi_max, double *row, void *scr
   if (np > 0) k_phst_chunks<<<blocks_for(nchunk), kThreads, 0, S(stream)>>>(pview(c), DUSTB_IPZ, part, nchunk);
   k_phst_sums<<<1, 1, 0, S(stream)>>>(part, nchunk, chi_max, c->phys.back_reaction, row);
   cudaMemsetAsync(field, 0, (size_t)d.cells() * d.nmb * 8, S(stream));
-  if (np > 0) k_mass_deposit<<<PGRID(c)>>>(pview(c), mview(c), d, field, c->err);
+  if (np > 0) k_mass_deposit<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, field, c->err, NB(c));
   int rc = dustb_ghost_add(c, field, 1, stream);
   if (rc) return rc;
   const int nb = 1024;
@@ -3117,7 +3099,12 @@ static int point_deposit(const dustb_ctx *c, double *out, double *halo, int ncom
   const dustb_ctx g = fold_ctx(c);
   cudaMemsetAsync(halo, 0, (size_t)(n_all(d) * ncomp) * sizeof(double), S(stream));
   if (c->part.npart > 0)
-    k_point_deposit<<<PGRID(c)>>>(pview(c), mview(c), d, halo, ncomp, species, gravity, c->err);
+  {
+    if (ncomp == 1)
+      k_point_deposit<1><<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, halo, species, gravity, c->err, NB(c));
+    else
+      k_point_deposit<4><<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, halo, species, gravity, c->err, NB(c));
+  }
   int rc = dustb_ghost_add(&g, halo, ncomp, stream);
   if (rc) return rc;
   k_owned_copy<<<blocks_for(n_all(d) * ncomp), kThreads, 0, S(stream)>>>(d, halo, out, ncomp);
@@ -3212,7 +3199,7 @@ int dustb_dc1_sweep_plan(const dustb_ctx *c, const dustb_dep_plan *plan, double 
   if (rc) return rc;
   cudaMemsetAsync(c->f.work, 0, (size_t)n_all(d) * 3 * sizeof(double), S(stream));
   if (c->part.npart > 0)
-    k_operator<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.ustar, c->f.work, a_dt, 0.0, c->err);
+    k_operator<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.ustar, c->f.work, a_dt, 0.0, c->err, NB(c));
   rc = dustb_ghost_add_plan(c, plan, c->f.work, 3, stream);
   if (rc) return rc;
   k_dc_correct<<<blocks_for(n_active(d)), kThreads, 0, S(stream)>>>(
