@@ -1,18 +1,24 @@
 // dustb_deposit.cuh -- FP64 stencil deposits combined per cell inside a warp.
 //
 // A particle's deposit is 27 cells (9 in 2-D) times up to four values.  One FP64 atomic per
-// particle, cell and value is bound by the L2's atomic rate (the three 3-D deposits of a stage
-// of 4.2 M particles at 16 per cell took 2.6-2.9 ms each, 0.17 T atomics/s).  Here a warp takes
-// 32 consecutive particles at a time: every lane forms its own particle's weights and values
-// and stages them in the warp's shared memory, then the lanes become the 27 cells of one
-// stencil and walk the particles that share an anchor cell, summing in registers.  The groups
-// of a batch go in ascending cell order; when the next group is the next cell along x, two
-// thirds of the window carry over by a shuffle and only the column left behind is added to the
-// field (9 lanes x values atomics per cell instead of 27 per particle).  Rows in cell order
-// need about 2 atomics per particle instead of 108; rows in no order make groups of one
-// particle, whose atomics are no more than before and land on three consecutive cells per
-// row.  The products are those of the one-thread-per-particle form; only the order of the
-// sums differs.
+// particle, cell and value is bound by the L2's atomic rate (0.17 T atomics/s: 2.6-2.9 ms for
+// each 3-D deposit of 4.2 M particles at 16 per cell).  Here a warp takes 32 consecutive
+// particles at a time: every lane forms one particle's weights and values and stages them in
+// the warp's shared memory in ascending order of the anchor cells; then the lanes become the
+// 27 cells of one stencil and walk the particles of one anchor cell after the other, summing
+// in registers.  When the next anchor is the next cell along x, two thirds of the window carry
+// over by a shuffle and only the column left behind is added to the field (9 lanes x values
+// atomics per cell instead of 27 per particle).  Rows in cell order need about 2 atomics per
+// particle instead of 108; rows in no order make groups of one particle, whose atomics are no
+// more than before and land on three consecutive cells per row.  The products are those of the
+// one-thread-per-particle form; only the order of the sums differs.
+//
+// 4.2 M particles at 16 per cell in cell order (64^3 cells, 5 CTAs per SM): Q/P 2.88 -> 0.30 ms,
+// operator 2.59 -> 0.40, gather-kick 2.63 -> 0.47.  What bounds it now is instruction issue and
+// its latencies (IPC 2.0, 38 warp instructions per particle in Q/P: about 9 to form and stage
+// a particle, 10 to sum it, the rest the changes of cell), no longer atomics (L2 at 25 %).
+// Measured and not kept: nine lanes per stream with three x columns and all values in registers
+// (0.40 ms Q/P: the streams' flushes diverge).
 #pragma once
 
 #include "dustb_common.cuh"
@@ -22,29 +28,37 @@ namespace dustb {
 constexpr int kDepWarps = 4;                     // warps per CTA of the depositing kernels
 constexpr unsigned kNoCell = 0xffffffffu;
 
-// one warp's staged batch: the weights (x, y, z: rows 0-2, 3-5, 6-8; 33 columns, so that the
-// three rows the lanes of one load read lie in different banks) and four values per particle
+// one warp's staged batch: up to four values per particle, the x weights (rows 0-2) and the
+// products of y and z weights with the particle's factor (rows 3-11: 3 + 3 c + b).  33 columns:
+// the rows the lanes of one load read lie in different banks
 struct alignas(16) WarpStage {
-  double q[32][4];              // (first: its 16-byte loads; the struct's size is padded to 16)
-  double w[9][33];
-  __device__ __forceinline__ void put(int lane, const double wx[3], const double wy[3],
-                                      const double wz[3], double q0, double q1, double q2,
-                                      double q3) {
+  double q[32][4];              // (first: its 16-byte loads; the size is a multiple of 16)
+  double w[12][33];
+  long long kb[32];             // the anchor cell's field index
+  unsigned key[32];             // the anchor cell (ascending)
+  __device__ __forceinline__ void put(int at, const double wx[3], const double wy[3],
+                                      const double wz[3], double fac, const double v[4],
+                                      unsigned k, long long at_k) {
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      w[a][lane] = wx[a];
-      w[3 + a][lane] = wy[a];
-      w[6 + a][lane] = wz[a];
+    for (int a = 0; a < 3; ++a) w[a][at] = wx[a];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double f = wz[c] * fac;
+#pragma unroll
+      for (int b = 0; b < 3; ++b) w[3 + 3 * c + b][at] = f * wy[b];
     }
-    *(double2 *)&q[lane][0] = make_double2(q0, q1);
-    *(double2 *)&q[lane][2] = make_double2(q2, q3);
+    *(double2 *)&q[at][0] = make_double2(v[0], v[1]);
+    *(double2 *)&q[at][2] = make_double2(v[2], v[3]);
+    key[at] = k;
+    kb[at] = at_k;
   }
 };
+static_assert(sizeof(WarpStage) % 16 == 0, "the stages of a CTA follow one another");
 
-// consecutive batches of 32 particles a warp takes: enough that the cells at a batch's ends
-// are shared, few enough that small sets still give every SM 32 warps
+// consecutive batches of 32 particles a warp takes: enough that the cells at a warp's ends are
+// shared, few enough for several waves of CTAs
 inline int dep_batches(long long n) {
-  const long long per = n / (32LL * 148 * 32);
+  const long long per = n / (32LL * 148 * 64);
   return per < 1 ? 1 : (per > 8 ? 8 : (int)per);
 }
 inline unsigned dep_blocks(long long n, int nb) {
@@ -52,101 +66,120 @@ inline unsigned dep_blocks(long long n, int nb) {
   return (unsigned)((n + per - 1) / per);
 }
 
-// NV values per cell.  FAC: q[0] is a factor of the weights; ONE: the first value is the weight
-// itself, the others the weight times q[FAC], q[FAC + 1], ...
-template <int NV, bool FAC, bool ONE>
+// the place of this lane's particle among the warp's live ones in ascending key order (equal
+// keys by lane; a lane without a particle holds kNoCell); all lanes of the warp take part
+__device__ __forceinline__ int warp_rank(unsigned key, bool live) {
+  const int lane = threadIdx.x & 31;
+  const unsigned up = __shfl_up_sync(0xffffffffu, key, 1);
+  if (__all_sync(0xffffffffu, lane == 0 || up <= key)) return lane;
+  const unsigned below = (1u << lane) - 1u;
+  int rank = 0, base = 0;
+  unsigned rem = __ballot_sync(0xffffffffu, live);
+  while (rem) {
+    const bool mine = (rem >> lane) & 1u;
+    const unsigned k = __reduce_min_sync(0xffffffffu, mine ? key : kNoCell);
+    const unsigned grp = __ballot_sync(0xffffffffu, mine && key == k);
+    if (mine && key == k) rank = base + __popc(grp & below);
+    base += __popc(grp);
+    rem &= ~grp;
+  }
+  return rank;
+}
+
+// NV values per cell; ONE: the first is the weight itself, the others the weight times q[0],
+// q[1], ...
+// at(k): the field address (variable 0) of this lane's window cell about the anchor with field
+// index k, null if no block owns it; variables vs apart
+template <int NV, bool ONE>
 struct CellDeposit {
+  static constexpr int NQ = NV - (ONE ? 1 : 0);
   double acc[NV];
-  double *f;                    // variable 0 of the deposit
-  long long vs;                 // its stride per variable
   long long base;               // the field index of the current anchor cell
   unsigned cur;                 // the current anchor cell (kNoCell: none)
-  int ra, rb, rc, off;          // this lane's weights' rows and its cell's offset
+  int a, b, c;                  // this lane's cell of the window, -1..1 each
   bool on;
 
-  __device__ __forceinline__ void init(double *field, const Ind &d) {
-    const int lane = threadIdx.x & 31;
-    const int l = lane < 27 ? lane : 0;
-    const int a = l / 9, r = l - a * 9, c = r / 3, b = r - c * 3;
-    f = field;
-    vs = d.cells();
-    ra = a; rb = 3 + b; rc = 6 + c;
-    off = ((c - 1) * d.n2 + (b - 1)) * d.n1 + (a - 1);
-    on = lane < 27 && (d.three_d || c == 1);
+  // lane = 9 (a + 1) + 3 (c + 1) + b + 1: a column is nine consecutive lanes
+  __device__ __forceinline__ void init(bool three_d) {
+    const int lane = threadIdx.x & 31, l = lane < 27 ? lane : 0;
+    const int r = l % 9;
+    a = l / 9 - 1; c = r / 3 - 1; b = r % 3 - 1;
+    on = lane < 27 && (three_d || c == 0);
     cur = kNoCell;
     base = 0;
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[v] = 0.0;
   }
-  __device__ __forceinline__ void add_acc(bool who) {
+  template <typename At>
+  __device__ __forceinline__ void put(bool who, long long vs, At &&at) {
     if (!who) return;
-    double *t = f + base + off;
+    double *t = at(base);
+    if (!t) return;
 #pragma unroll
     for (int v = 0; v < NV; ++v)
       if (acc[v] != 0.0) atomicAdd(t + v * vs, acc[v]);
   }
-  __device__ __forceinline__ void flush() {
-    if (cur != kNoCell) add_acc(on);
+  template <typename At>
+  __device__ __forceinline__ void flush(long long vs, At &&at) {
+    if (cur != kNoCell) put(on, vs, at);
     cur = kNoCell;
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[v] = 0.0;
   }
-  // the window moved to anchor cell k (field index kb)
-  __device__ __forceinline__ void move_to(unsigned k, long long kb) {
+  template <typename At>
+  __device__ __forceinline__ void move_to(unsigned k, long long kb, long long vs, At &&at) {
+    if (k == cur) return;
     if (cur != kNoCell && k == cur + 1) {
       // the next cell of the row (a row's last padded cell is no anchor, so cur + 1 is never
       // the next row's): column 0 is finished, columns 1 and 2 become 0 and 1
       const int lane = threadIdx.x & 31;
-      add_acc(on && lane < 9);
+      put(on && lane < 9, vs, at);
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
         const double y = __shfl_down_sync(0xffffffffu, acc[v], 9);
         acc[v] = lane < 18 ? y : 0.0;
       }
     } else {
-      flush();
+      flush(vs, at);
     }
     cur = k;
     base = kb;
   }
-  __device__ __forceinline__ void one(const WarpStage &s, int p, bool take) {
-    double wcb = s.w[rc][p] * s.w[rb][p];
-    const double2 q01 = *(const double2 *)&s.q[p][0];
-    const double2 q23 = *(const double2 *)&s.q[p][2];
-    if (FAC) wcb *= q01.x;
-    if (!take || wcb == 0.0) return;
-    const double w = wcb * s.w[ra][p];
-    const double val[4] = {q01.x, q01.y, q23.x, q23.y};
-    if (ONE) acc[0] += w;
+  // the n staged particles of the batch.  check: some staged value is not finite, so that zero
+  // weights (skipped, as the reference skips them) have to be told apart
+  template <typename At>
+  __device__ __forceinline__ void walk(const WarpStage &s, int n, bool check, long long vs,
+                                       At &&at) {
+    const int lane = threadIdx.x & 31;
+    const unsigned key = lane < n ? s.key[lane] : kNoCell;
+    const double *wx = s.w[a + 1], *wyz = s.w[3 + 3 * (c + 1) + b + 1];
+    int lo = 0;
+    while (lo < n) {
+      const unsigned k = __shfl_sync(0xffffffffu, key, lo);
+      const int hi = lo + __popc(__ballot_sync(0xffffffffu, key == k));
+      move_to(k, s.kb[lo], vs, at);
+      if (!check) {
+#pragma unroll 4
+        for (int p = lo; p < hi; ++p) {
+          const double w = wyz[p] * wx[p];
+          if (ONE) acc[0] += w;
 #pragma unroll
-    for (int v = ONE ? 1 : 0; v < NV; ++v)
-      acc[v] = __fma_rn(w, val[v - (ONE ? 1 : 0) + (FAC ? 1 : 0)], acc[v]);
-  }
-  // the staged batch: key this lane's anchor cell (the padded cell's index over all blocks),
-  // kb its index in the field (variable 0); live: the lane holds a particle that deposits
-  __device__ __forceinline__ void batch(const WarpStage &s, unsigned key, long long kb,
-                                        bool live) {
-    unsigned rem = __ballot_sync(0xffffffffu, live);
-    while (rem) {
-      const bool mine = (rem >> (threadIdx.x & 31)) & 1u;
-      const unsigned k = __reduce_min_sync(0xffffffffu, mine ? key : kNoCell);
-      unsigned grp = __ballot_sync(0xffffffffu, mine && key == k);
-      rem &= ~grp;
-      if (k != cur) move_to(k, __shfl_sync(0xffffffffu, kb, __ffs(grp) - 1));
-      while (grp) {
-        // two particles at a time: their shared loads fly together
-        const int p = __ffs(grp) - 1;
-        grp &= grp - 1;
-        const int p2 = grp ? __ffs(grp) - 1 : p;
-        const bool two = grp != 0;
-        grp &= grp - 1;                            // (0 & x stays 0)
-        one(s, p, true);
-        one(s, p2, two);
+          for (int v = 0; v < NQ; ++v)
+            acc[v + (ONE ? 1 : 0)] = __fma_rn(w, s.q[p][v], acc[v + (ONE ? 1 : 0)]);
+        }
+      } else {
+        for (int p = lo; p < hi; ++p) {
+          if (wyz[p] == 0.0) continue;
+          const double w = wyz[p] * wx[p];
+          if (ONE) acc[0] += w;
+#pragma unroll
+          for (int v = 0; v < NQ; ++v)
+            acc[v + (ONE ? 1 : 0)] = __fma_rn(w, s.q[p][v], acc[v + (ONE ? 1 : 0)]);
+        }
       }
+      lo = hi;
     }
   }
 };
-
-static_assert(sizeof(WarpStage) % 16 == 0, "the stages of a CTA follow one another");
 
 }  // namespace dustb

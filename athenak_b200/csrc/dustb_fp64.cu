@@ -473,52 +473,76 @@ __global__ void k_route(PCtx P, MCtx M, Ind d, int x3bc, double *x3rem, unsigned
 }
 
 // ---- deposits: a warp's particles combined per cell (dustb_deposit.cuh) -------------------
-// a depositing particle: its block, anchor cell, weights and staged values
+// a depositing particle: its block, anchor cell, weights, the factor of the weights and the
+// values
 struct Stencil {
   int m, ip, jp, kp;
-  double wx[3], wy[3], wz[3], q[4];
+  double wx[3], wy[3], wz[3], fac, q[4];
 };
 
-// every particle of the launch through particle(p, stencil), which returns whether it deposits,
-// and its deposit into variable v0 on of an nvar-variable field
-template <int NV, bool FAC, bool ONE, typename F>
+// the part of a particle's weights that only its block sets, kept from one particle of a lane
+// to the next
+struct BlockScale {
+  int m = -1;
+  double x0[3], s[3], vol;
+  __device__ __forceinline__ void set(const MCtx &M, const Ind &d, int mm) {
+    if (mm == m) return;
+    m = mm;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      x0[a] = M.s(m, X1MIN + a);
+      s[a] = (double)(a == 0 ? d.nx1 : a == 1 ? d.nx2 : d.nx3) / (M.s(m, X1MAX + a) - x0[a]);
+    }
+    vol = cell_vol(M, d, m);
+  }
+};
+
+// every particle of the launch through particle(p, stencil, scale), which returns whether it
+// deposits, and its deposit into variable v0 on of an nvar-variable field
+template <int NV, bool ONE, typename F>
 __device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &d, double *field,
                                                   int nvar, int v0, F &&particle) {
   __shared__ WarpStage s_stage[kDepWarps];
   WarpStage &st = s_stage[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  CellDeposit<NV, FAC, ONE> dep;
-  dep.init(field, d);
+  CellDeposit<NV, ONE> dep;
+  dep.init(d.three_d);
+  const long long vs = d.cells();
+  double *mine = field + ((long long)(dep.c * d.n2 + dep.b) * d.n1 + dep.a);
+  auto at = [&](long long k) { return mine + k; };
+  BlockScale bs;
   const long long first = ((long long)blockIdx.x * kDepWarps + (threadIdx.x >> 5)) * nb * 32;
   for (int b = 0; b < nb; ++b) {
     const long long p0 = first + 32LL * b;
     if (p0 >= npart) break;
-    unsigned key = kNoCell;
-    long long kb = 0;
-    bool live = false;
-    if (p0 + lane < npart) {
-      Stencil t;
-      live = particle((int)(p0 + lane), t);
-      if (live) {
-        key = (unsigned)d.at(t.m, 1, 0, t.kp, t.jp, t.ip);   // (below 2^32: one GPU's memory)
-        kb = d.at(t.m, nvar, v0, t.kp, t.jp, t.ip);
-        st.put(lane, t.wx, t.wy, t.wz, t.q[0], t.q[1], t.q[2], t.q[3]);
-      }
+    Stencil t;
+    const bool live = p0 + lane < npart && particle((int)(p0 + lane), t, bs);
+    // (the padded cell's index over all blocks: below 2^32 in one GPU's memory)
+    const unsigned key = live ? (unsigned)d.at(t.m, 1, 0, t.kp, t.jp, t.ip) : kNoCell;
+    const int at_ = warp_rank(key, live);
+    double sum = 0.0;                            // (not finite: some value is not, or their sum)
+    if (live) {
+      st.put(at_, t.wx, t.wy, t.wz, t.fac, t.q, key, d.at(t.m, nvar, v0, t.kp, t.jp, t.ip));
+#pragma unroll
+      for (int v = 0; v < NV - (ONE ? 1 : 0); ++v) sum += t.q[v];
     }
+    const int n = __popc(__ballot_sync(0xffffffffu, live));
+    const bool check = __any_sync(0xffffffffu, !isfinite(sum));
     __syncwarp();
-    dep.batch(st, key, kb, live);
+    dep.walk(st, n, check, vs, at);
     __syncwarp();
   }
-  dep.flush();
+  dep.flush(vs, at);
 }
 
 // the gather of a 3-variable field with the particle's weights, in the reference's order
 __device__ __forceinline__ void gather3(const Ind &d, const Stencil &t, const double *f,
                                         double &g0, double &g1, double &g2) {
   g0 = g1 = g2 = 0.0;
-  const int clo = d.three_d ? 0 : 1, chi = d.three_d ? 2 : 1;
   const long long vs = d.cells();
-  for (int c = clo; c <= chi; ++c)
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    if (!d.three_d && c != 1) continue;
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       const double wcb = t.wz[c] * t.wy[b];
@@ -532,29 +556,56 @@ __device__ __forceinline__ void gather3(const Ind &d, const Stencil &t, const do
         g2 += w * r[a + 2 * vs];
       }
     }
+  }
+}
+
+// PMWeights (pm_weights, dustb_common.cuh) with the block's origin and cells per length
+__device__ __forceinline__ void scaled_weights(double x, double x0, double sc, int is, int scheme,
+                                               int &ip, double w[3]) {
+  const double cell = (x - x0) * sc;
+  const int ig = (int)(cell + 1.0) - 1;
+  const double del = cell - ((double)ig + 0.5);
+  ip = ig + is;
+  if (scheme == 0) {
+    w[0] = 0.0; w[1] = 1.0; w[2] = 0.0;
+  } else if (scheme == 1) {
+    w[0] = fmax(0.0, -del); w[1] = 1.0 - fabs(del); w[2] = fmax(0.0, del);
+  } else {
+    w[0] = 0.5 * ((0.5 - del) * (0.5 - del));
+    w[1] = 0.75 - del * del;
+    w[2] = 0.5 * ((0.5 + del) * (0.5 + del));
+  }
 }
 
 // the block, anchor cell and weights of a position; false (and the error bit) outside the pack
 // or the block's halo
 __device__ __forceinline__ bool place(const PCtx &P, const MCtx &M, const Ind &d, int p, double x,
-                                      double y, double z, Stencil &t, unsigned *err) {
+                                      double y, double z, Stencil &t, BlockScale &bs,
+                                      unsigned *err) {
   t.m = P.i(DUSTB_PGID, p) - M.gids;
   if (!block_ok(d, t.m)) { report(err, DUSTB_ERR_PGID); return false; }
-  weights3(M, d, t.m, x, y, z, t.ip, t.jp, t.kp, t.wx, t.wy, t.wz);
+  bs.set(M, d, t.m);
+  scaled_weights(x, bs.x0[0], bs.s[0], d.is, M.scheme, t.ip, t.wx);
+  scaled_weights(y, bs.x0[1], bs.s[1], d.js, M.scheme, t.jp, t.wy);
+  if (d.three_d) {
+    scaled_weights(z, bs.x0[2], bs.s[2], d.ks, M.scheme, t.kp, t.wz);
+  } else {
+    t.kp = d.ks; t.wz[0] = 0.0; t.wz[1] = 1.0; t.wz[2] = 0.0;
+  }
   if (!halo_ok(d, t.ip, t.jp, t.kp)) { report(err, DUSTB_ERR_HALO); return false; }
   return true;
 }
 
 // ---- DepositDrag imex scatter, src/dust/dust_pm.cpp:225-274 ------------------------------
-__global__ void __launch_bounds__(32 * kDepWarps)
+__global__ void __launch_bounds__(32 * kDepWarps, 5)
 k_scatter(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh, unsigned *err, int nb) {
-  deposit_particles<4, true, true>(P.npart, nb, d, qdep, 5, 0, [&](int p, Stencil &t) {
+  deposit_particles<4, true>(P.npart, nb, d, qdep, 5, 0, [&](int p, Stencil &t, BlockScale &bs) {
     const double x = P.r(DUSTB_IPX, p);
-    if (!place(P, M, d, p, x, P.r(DUSTB_IPY, p) + sh * x, P.r(DUSTB_IPZ, p), t, err)) return false;
-    const double vol = cell_vol(M, d, t.m);
+    if (!place(P, M, d, p, x, P.r(DUSTB_IPY, p) + sh * x, P.r(DUSTB_IPZ, p), t, bs, err)) return false;
     const double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
-    t.q[0] = P.r(DUSTB_IPM, p) * cj / vol;
-    t.q[1] = P.r(DUSTB_IPVX, p); t.q[2] = P.r(DUSTB_IPVY, p); t.q[3] = P.r(DUSTB_IPVZ, p);
+    t.fac = P.r(DUSTB_IPM, p) * cj / bs.vol;
+    t.q[0] = P.r(DUSTB_IPVX, p); t.q[1] = P.r(DUSTB_IPVY, p); t.q[2] = P.r(DUSTB_IPVZ, p);
+    t.q[3] = 0.0;
     return true;
   });
 }
@@ -776,16 +827,16 @@ __global__ void k_solve_ustar(Ind d, const double *u0, int nv, const double *qde
 }
 
 // ---- PointOperatorParticles, src/dust/dust_solver.cpp:151-201 ---------------------------
-__global__ void __launch_bounds__(32 * kDepWarps)
+__global__ void __launch_bounds__(32 * kDepWarps, 5)
 k_operator(PCtx P, MCtx M, Ind d, const double *field, double *result, double a_dt, double sh,
            unsigned *err, int nb) {
-  deposit_particles<3, true, false>(P.npart, nb, d, result, 3, 0, [&](int p, Stencil &t) {
+  deposit_particles<3, false>(P.npart, nb, d, result, 3, 0, [&](int p, Stencil &t, BlockScale &bs) {
     const double x = P.r(DUSTB_IPX, p);
-    if (!place(P, M, d, p, x, P.r(DUSTB_IPY, p) + sh * x, P.r(DUSTB_IPZ, p), t, err)) return false;
-    gather3(d, t, field, t.q[1], t.q[2], t.q[3]);
-    const double vol = cell_vol(M, d, t.m);
+    if (!place(P, M, d, p, x, P.r(DUSTB_IPY, p) + sh * x, P.r(DUSTB_IPZ, p), t, bs, err)) return false;
     const double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
-    t.q[0] = P.r(DUSTB_IPM, p) * cj / vol;
+    t.fac = P.r(DUSTB_IPM, p) * cj / bs.vol;
+    gather3(d, t, field, t.q[0], t.q[1], t.q[2]);
+    t.q[3] = 0.0;
     return true;
   });
 }
@@ -806,12 +857,12 @@ __global__ void k_dc_correct(Ind d, const double *u0, int nv, const double *qdep
 }
 
 // ---- GatherKickPMBR, src/dust/dust_pm.cpp:500-564 ----------------------------------------
-__global__ void __launch_bounds__(32 * kDepWarps)
+__global__ void __launch_bounds__(32 * kDepWarps, 5)
 k_gather_kick(PCtx P, MCtx M, Ind d, const double *us, double *dmom, double a_dt, double sh, int br,
               unsigned *err, int nb) {
-  deposit_particles<3, true, false>(P.npart, nb, d, dmom, 3, 0, [&](int p, Stencil &t) {
+  deposit_particles<3, false>(P.npart, nb, d, dmom, 3, 0, [&](int p, Stencil &t, BlockScale &bs) {
     const double x = P.r(DUSTB_IPX, p);
-    if (!place(P, M, d, p, x, P.r(DUSTB_IPY, p) + sh * x, P.r(DUSTB_IPZ, p), t, err)) return false;
+    if (!place(P, M, d, p, x, P.r(DUSTB_IPY, p) + sh * x, P.r(DUSTB_IPZ, p), t, bs, err)) return false;
     double ux, uy, uz;
     gather3(d, t, us, ux, uy, uz);
     const double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
@@ -820,8 +871,8 @@ k_gather_kick(PCtx P, MCtx M, Ind d, const double *us, double *dmom, double a_dt
     P.r(DUSTB_IPVX, p) = vx + dvx; P.r(DUSTB_IPVY, p) = vy + dvy; P.r(DUSTB_IPVZ, p) = vz + dvz;
     P.r(DUSTB_IPRX, p) = dvx / a_dt; P.r(DUSTB_IPRY, p) = dvy / a_dt; P.r(DUSTB_IPRZ, p) = dvz / a_dt;
     if (!br) return false;
-    t.q[0] = -P.r(DUSTB_IPM, p) / cell_vol(M, d, t.m);
-    t.q[1] = dvx; t.q[2] = dvy; t.q[3] = dvz;
+    t.fac = -P.r(DUSTB_IPM, p) / bs.vol;
+    t.q[0] = dvx; t.q[1] = dvy; t.q[2] = dvz; t.q[3] = 0.0;
     return true;
   });
 }
@@ -839,41 +890,15 @@ __device__ __forceinline__ bool center_cell(const PCtx &P, const MCtx &M, const 
   return halo_ok(d, ip, jp, kp);
 }
 
-// the sum of v over the lanes of a warp, in every lane
-__device__ __forceinline__ double warp_total(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// (the particles of a warp that share a centre cell add once: rows in cell order put a cell's
-// particles next to each other, where one atomic per particle would queue up on its address)
 __global__ void k_center_mass(PCtx P, MCtx M, Ind d, double *res, double a_dt, unsigned *err) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  long long at = -1;
-  double mc = 0.0;
-  if (p < P.npart && !(P.r(DUSTB_IPM, p) <= 0.0)) {
-    int m, ip, jp, kp;
-    if (!center_cell(P, M, d, p, m, ip, jp, kp)) {
-      report(err, DUSTB_ERR_HALO);
-    } else {
-      at = d.at(m, 4, 3, kp, jp, ip);
-      mc = P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt)) / cell_vol(M, d, m);
-    }
-  }
-  unsigned rem = __ballot_sync(0xffffffffu, at >= 0);
-  while (rem) {
-    const int lead = __ffs(rem) - 1;
-    const long long k = __shfl_sync(0xffffffffu, at, lead);
-    const unsigned grp = __ballot_sync(0xffffffffu, at == k) & rem;
-    rem &= ~grp;
-    if (grp == (1u << lead)) {
-      if ((int)(threadIdx.x & 31) == lead) atomicAdd(&res[at], mc);
-    } else {
-      const double t = warp_total(at == k ? mc : 0.0);
-      if ((int)(threadIdx.x & 31) == lead) atomicAdd(&res[at], t);
-    }
-  }
+  int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= P.npart) return;
+  if (P.r(DUSTB_IPM, p) <= 0.0) return;
+  int m, ip, jp, kp;
+  if (!center_cell(P, M, d, p, m, ip, jp, kp)) { report(err, DUSTB_ERR_HALO); return; }
+  double vol = cell_vol(M, d, m);
+  atomicAdd(&res[d.at(m, 4, 3, kp, jp, ip)],
+            P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt)) / vol);
 }
 
 __global__ void k_consistent_gas(Ind d, double *u0, int nv, const double *us, const double *qdep,
@@ -973,16 +998,17 @@ __global__ void k_tstop(PCtx P, double *out, unsigned *err) {
 
 // ---- pc2 ---------------------------------------------------------------------------------
 // DepositDrag pc2 predictor, src/dust/dust_pm.cpp:141-193
-__global__ void __launch_bounds__(32 * kDepWarps)
+__global__ void __launch_bounds__(32 * kDepWarps, 5)
 k_pc2_predictor(PCtx P, MCtx M, Ind d, const double *uold, int nv, double *qdep, double dt,
                 int rate_dep, unsigned *err, int nb) {
-  deposit_particles<4, false, false>(P.npart, nb, d, qdep, 5, 1, [&](int p, Stencil &t) {
-    if (!place(P, M, d, p, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p), P.r(DUSTB_IPZ, p), t, err))
+  deposit_particles<4, false>(P.npart, nb, d, qdep, 5, 1, [&](int p, Stencil &t, BlockScale &bs) {
+    if (!place(P, M, d, p, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p), P.r(DUSTB_IPZ, p), t, bs, err))
       return false;
     double ugx = 0.0, ugy = 0.0, ugz = 0.0;
-    const int clo = d.three_d ? 0 : 1, chi = d.three_d ? 2 : 1;
     const long long vs = d.cells();
-    for (int c = clo; c <= chi; ++c)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      if (!d.three_d && c != 1) continue;
 #pragma unroll
       for (int b = 0; b < 3; ++b) {
         const double wcb = t.wz[c] * t.wy[b];
@@ -997,8 +1023,9 @@ k_pc2_predictor(PCtx P, MCtx M, Ind d, const double *uold, int nv, double *qdep,
           ugz += w * r[a + 3 * vs] * invrho;
         }
       }
-    const double vol = cell_vol(M, d, t.m);
-    const double rate = P.r(DUSTB_IPM, p) / (P.r(DUSTB_IPTS, p) * vol);
+    }
+    const double rate = P.r(DUSTB_IPM, p) / (P.r(DUSTB_IPTS, p) * bs.vol);
+    t.fac = 1.0;
     t.q[0] = -dt * rate * (ugx - P.r(DUSTB_IPVX, p));
     t.q[1] = -dt * rate * (ugy - P.r(DUSTB_IPVY, p));
     t.q[2] = -dt * rate * (ugz - P.r(DUSTB_IPVZ, p));
@@ -1047,10 +1074,10 @@ __global__ void k_pc2_midpoint(Ind d, const double *u0, const double *u1, int nv
 }
 
 // dust_pc2_advance, src/dust/dust_push.cpp:132-245
-__global__ void __launch_bounds__(32 * kDepWarps)
+__global__ void __launch_bounds__(32 * kDepWarps, 5)
 k_pc2_advance(PCtx P, MCtx M, Ind d, const double *us, double *dmom, double dt, int br, int sbox,
               int strat, double q, double om, double aphi, unsigned *err, int nb) {
-  deposit_particles<3, true, false>(P.npart, nb, d, dmom, 3, 0, [&](int p, Stencil &t) {
+  deposit_particles<3, false>(P.npart, nb, d, dmom, 3, 0, [&](int p, Stencil &t, BlockScale &bs) {
     const bool three_d = d.three_d;
     double x0 = P.r(DUSTB_IPX1, p), y0 = P.r(DUSTB_IPY1, p), z0 = P.r(DUSTB_IPZ1, p);
     double vx0 = P.r(DUSTB_IPVX1, p), vy0 = P.r(DUSTB_IPVY1, p), vz0 = P.r(DUSTB_IPVZ1, p);
@@ -1058,7 +1085,7 @@ k_pc2_advance(PCtx P, MCtx M, Ind d, const double *us, double *dmom, double dt, 
     double yh = y0 + 0.5 * dt * (vy0 - ((sbox && three_d) ? q * om * x0 : 0.0));
     double zh = three_d ? z0 + 0.5 * dt * vz0 : z0;
     double yg = yh + ((sbox && three_d) ? q * om * xh * 0.5 * dt : 0.0);
-    if (!place(P, M, d, p, xh, yg, zh, t, err)) return false;
+    if (!place(P, M, d, p, xh, yg, zh, t, bs, err)) return false;
     double ugx, ugy, ugz;
     gather3(d, t, us, ugx, ugy, ugz);
     double h = 0.5 * dt;
@@ -1095,8 +1122,8 @@ k_pc2_advance(PCtx P, MCtx M, Ind d, const double *us, double *dmom, double dt, 
     double dvz = dt * (ugz - vzh) / P.r(DUSTB_IPTS, p);
     P.r(DUSTB_IPRX, p) = dvx; P.r(DUSTB_IPRY, p) = dvy; P.r(DUSTB_IPRZ, p) = dvz;
     if (!br) return false;
-    t.q[0] = -P.r(DUSTB_IPM, p) / cell_vol(M, d, t.m);
-    t.q[1] = dvx; t.q[2] = dvy; t.q[3] = dvz;
+    t.fac = -P.r(DUSTB_IPM, p) / bs.vol;
+    t.q[0] = dvx; t.q[1] = dvy; t.q[2] = dvz; t.q[3] = 0.0;
     return true;
   });
 }
@@ -1150,15 +1177,15 @@ __global__ void k_phst_sums(const double *part, int nchunk, const double *chi, i
 
 // the mass component of DepositPointScienceFields (src/dust/dust_gravity_points.cpp:277-304):
 // m/V with the deposit weights into the block's cells, ghost cells included
-__global__ void __launch_bounds__(32 * kDepWarps)
+__global__ void __launch_bounds__(32 * kDepWarps, 5)
 k_mass_deposit(PCtx P, MCtx M, Ind d, double *f, unsigned *err, int nb) {
-  deposit_particles<1, true, true>(P.npart, nb, d, f, 1, 0, [&](int p, Stencil &t) {
+  deposit_particles<1, true>(P.npart, nb, d, f, 1, 0, [&](int p, Stencil &t, BlockScale &bs) {
     const double mass = P.r(DUSTB_IPM, p);
     if (mass == 0.0) return false;
-    if (!place(P, M, d, p, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p), P.r(DUSTB_IPZ, p), t, err))
+    if (!place(P, M, d, p, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p), P.r(DUSTB_IPZ, p), t, bs, err))
       return false;
-    t.q[0] = mass / cell_vol(M, d, t.m);
-    t.q[1] = t.q[2] = t.q[3] = 0.0;
+    t.fac = mass / bs.vol;
+    t.q[0] = t.q[1] = t.q[2] = t.q[3] = 0.0;
     return true;
   });
 }
@@ -1235,9 +1262,9 @@ __device__ __forceinline__ bool point_stencil(const PCtx &P, const MCtx &M, cons
 // DepositPointScienceFields (:257-304; ncomp 1 or 4: m/V and m v/V, one species or all):
 // the density with the deposit weights into the owner block's cells, ghost cells included
 template <int NCOMP>
-__global__ void __launch_bounds__(32 * kDepWarps)
+__global__ void __launch_bounds__(32 * kDepWarps, 5)
 k_point_deposit(PCtx P, MCtx M, Ind d, double *f, int species, int gravity, unsigned *err, int nb) {
-  deposit_particles<NCOMP, true, true>(P.npart, nb, d, f, NCOMP, 0, [&](int p, Stencil &t) {
+  deposit_particles<NCOMP, true>(P.npart, nb, d, f, NCOMP, 0, [&](int p, Stencil &t, BlockScale &bs) {
     const double mass = P.r(DUSTB_IPM, p);
     if (gravity) {
       if (!(mass >= 0.0) || !isfinite(mass)) { report(err, DUSTB_ERR_POINT); return false; }
@@ -1251,10 +1278,10 @@ k_point_deposit(PCtx P, MCtx M, Ind d, double *f, int species, int gravity, unsi
       report(err, DUSTB_ERR_POINT);
       return false;
     }
-    t.q[0] = mass / (M.s(t.m, DX1) * M.s(t.m, DX2) * M.s(t.m, DX3));
-    t.q[1] = t.q[2] = t.q[3] = 0.0;
+    t.fac = mass / (M.s(t.m, DX1) * M.s(t.m, DX2) * M.s(t.m, DX3));
+    t.q[0] = t.q[1] = t.q[2] = t.q[3] = 0.0;
     if (NCOMP > 1) {
-      t.q[1] = P.r(DUSTB_IPVX, p); t.q[2] = P.r(DUSTB_IPVY, p); t.q[3] = P.r(DUSTB_IPVZ, p);
+      t.q[0] = P.r(DUSTB_IPVX, p); t.q[1] = P.r(DUSTB_IPVY, p); t.q[2] = P.r(DUSTB_IPVZ, p);
     }
     return true;
   });
