@@ -2242,6 +2242,310 @@ __device__ void cloud_gather(const MCtx &M, const Ind &d, int m, const double x[
 // warps per SM), _l over the leaf tables of refined meshes (held to 128 registers, 2 CTAs of 256
 // threads per SM: about 15 % faster than its unbounded 230 registers, which allow one CTA).
 
+// ---- the uniform traversal as three slots per direction ---------------------------------
+// On a uniform mesh without physical x3 faces a plain cloud of any level reaches at most the
+// cell that holds it and the one on either side along each direction (half-width dx / 2^level
+// <= dx): cloud_axis's cells are three fixed slots, so the cloud is a 27-cell stencil about its
+// cell and takes the warp-combined deposit of the point particles.  Everything that depends on
+// one direction only -- the hat's weight and moment, the cell centre's distance, the cell width
+// and its reciprocal -- is formed once per slot instead of once per leaf, from the block across
+// the face along that direction (blocks that share a position along a direction have the same
+// faces along it), with the expressions of cloud_axis and cloud_gather: the gathered velocity
+// is the same bit for bit, the deposits to the order of their sums.
+
+// n / d, correctly rounded, from y = 1 / d correctly rounded: two steps of Markstein's
+// quotient iteration (P. Markstein, IBM J. Res. Dev. 34 (1990) 111): the first brings the
+// quotient within an ulp, the second rounds it correctly.  The operands are cell widths and
+// weights times distances, far from overflow and underflow
+__device__ __forceinline__ double div_by(double n, double d, double y) {
+  double q = n * y;
+  q = __fma_rn(__fma_rn(-q, d, n), y, q);
+  return __fma_rn(__fma_rn(-q, d, n), y, q);
+}
+
+struct AxisSlot {
+  double w, g;                  // weight and first moment of the slot's cell
+  double e, dx, y;              // the cloud's distance from the cell's centre, width, 1 / width
+  int o;                        // the block across which face holds it (-1, 0, 1)
+};
+
+// slot of block-local cell i (one block's width beyond m at most) along direction a
+template <bool kM>
+__device__ __forceinline__ AxisSlot axis_slot(const MCtx &M, const Ind &d, int m, int a, int i,
+                                              double x, double dx, double idx, double ell,
+                                              double inv, double L) {
+  const int nx = (a == 0) ? d.nx1 : ((a == 1) ? d.nx2 : d.nx3);
+  AxisSlot s;
+  s.o = (i < 0) ? -1 : ((i >= nx) ? 1 : 0);
+  s.w = s.g = s.e = 0.0;
+  s.dx = dx; s.y = idx;
+  int b = m;
+  if (s.o != 0) {
+    i -= s.o * nx;
+    const int gid = M.nghbr[(long long)m * 27 + dir_slot(a == 0 ? s.o : 0, a == 1 ? s.o : 0,
+                                                         a == 2 ? s.o : 0)];
+    b = gid - M.gids;
+    if (gid < 0 || b < 0 || b >= d.nmb) return s;
+  }
+  const double org = M.s(b, X1MIN + a);
+  double bx0 = org;
+  if (s.o != 0) {
+    const double mo = M.s(m, X1MIN + a);
+    if (s.o < 0 && org >= mo) bx0 -= L;
+    if (s.o > 0 && org <= mo) bx0 += L;
+  }
+  const double za = (bx0 + i * dx - x) * inv, zb = (bx0 + (i + 1) * dx - x) * inv;
+  s.w = hat_cdf(zb) - hat_cdf(za);
+  if (kM) {
+    s.g = ell * (hat_moment(zb) - hat_moment(za));
+    if (s.o != 0) {
+      s.dx = M.s(b, DX1 + a);
+      s.y = 1.0 / s.dx;
+    }
+    const double ex = x - (org + (i + 0.5) * s.dx);
+    s.e = ex - L * round(ex / L);
+  }
+  return s;
+}
+
+// a cloud of block m, its cell and its place
+struct CloudPos {
+  int m, lev, ic[3];
+  double x[3], L[3];
+  bool inside;                  // the 27 cells lie in the block
+};
+
+__device__ __forceinline__ void cloud_cell(const MCtx &M, const Ind &d, CloudPos &c) {
+  const int nx[3] = {d.nx1, d.nx2, d.nx3};
+  c.inside = true;
+  c.ic[2] = 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    if (a == 2 && !d.three_d) break;
+    // (a gather position may lie up to one cell beyond the block; the clamp takes the rounding)
+    c.ic[a] = (int)floor((c.x[a] - M.s(c.m, X1MIN + a)) * (1.0 / M.s(c.m, DX1 + a)));
+    c.ic[a] = min(max(c.ic[a], -1), nx[a]);
+    c.inside = c.inside && c.ic[a] >= 1 && c.ic[a] + 1 < nx[a];
+  }
+}
+
+template <bool kM>
+__device__ __forceinline__ void cloud_slots(const MCtx &M, const Ind &d, const CloudPos &c, int a,
+                                            AxisSlot s[3]) {
+  const double dx = M.s(c.m, DX1 + a), idx = 1.0 / dx;
+  const double ell = ldexp(dx, -c.lev), inv = ldexp(idx, c.lev);
+#pragma unroll
+  for (int t = 0; t < 3; ++t)
+    s[t] = axis_slot<kM>(M, d, c.m, a, c.ic[a] + t - 1, c.x[a], dx, idx, ell, inv, c.L[a]);
+}
+
+// cloud_gather over the slots (kM), or the sum of weights times a field of nvar variables
+// (the overlap split's dust share); returns the three directions' weights in wx, wy, wz
+template <bool kM>
+__device__ __forceinline__ void slot_gather(const MCtx &M, const Ind &d, const CloudPos &c,
+                                            const double *f, int nvar, double ug[3],
+                                            double wx[3], double wy[3], double wz[3],
+                                            unsigned *err) {
+  AxisSlot X[3], Y[3];
+  cloud_slots<kM>(M, d, c, 0, X);
+  cloud_slots<kM>(M, d, c, 1, Y);
+  const double dz = M.s(c.m, DX3), idz = 1.0 / dz;
+  const double ellz = ldexp(dz, -c.lev), invz = ldexp(idz, c.lev);
+  ug[0] = ug[1] = ug[2] = 0.0;
+  wz[0] = wz[2] = 0.0; wz[1] = 1.0;
+#pragma unroll 1
+  for (int q = 0; q < 3; ++q) {
+    AxisSlot Z;
+    if (d.three_d) {
+      Z = axis_slot<kM>(M, d, c.m, 2, c.ic[2] + q - 1, c.x[2], dz, idz, ellz, invz, c.L[2]);
+      if (q == 0) wz[0] = Z.w; else if (q == 1) wz[1] = Z.w; else wz[2] = Z.w;
+    } else {
+      if (q != 1) continue;
+      Z.w = 1.0; Z.g = 0.0; Z.e = 0.0; Z.dx = 1.0; Z.y = 1.0; Z.o = 0;
+    }
+    if (Z.w == 0.0 && (!kM || Z.g == 0.0)) continue;
+    const int kk = d.three_d ? d.ks + c.ic[2] + q - 1 - Z.o * d.nx3 : d.ks;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      if (Y[b].w == 0.0 && (!kM || Y[b].g == 0.0)) continue;
+      const double w23 = Y[b].w * Z.w;
+      const int jj = d.js + c.ic[1] + b - 1 - Y[b].o * d.nx2;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        if (X[a].w == 0.0 && (!kM || X[a].g == 0.0)) continue;
+        const double w = w23 * X[a].w;
+        if (!kM && w == 0.0) continue;
+        const int ii = d.is + c.ic[0] + a - 1 - X[a].o * d.nx1;
+        const int blk = c.inside ? c.m : cloud_owner(M, d, c.m, X[a].o, Y[b].o, Z.o);
+        if (blk < 0) { if (err) report(err, DUSTB_ERR_CLOUD); continue; }
+        if (kM) {
+          const double *g = f + ((((long long)blk * d.n3 + kk) * d.n2 + jj) * d.n1 + ii) * 12;
+          const double cx = div_by(0.5 * (w23 * X[a].g + X[a].e * w), X[a].dx, X[a].y);
+          const double cy = div_by(0.5 * (X[a].w * Y[b].g * Z.w + Y[b].e * w), Y[b].dx, Y[b].y);
+          if (d.three_d) {
+            const double cz = div_by(0.5 * (X[a].w * Y[b].w * Z.g + Z.e * w), Z.dx, Z.y);
+            ug[0] += w * g[0] + cx * g[3] + cy * g[6] + cz * g[9];
+            ug[1] += w * g[1] + cx * g[4] + cy * g[7] + cz * g[10];
+            ug[2] += w * g[2] + cx * g[5] + cy * g[8] + cz * g[11];
+          } else {
+            ug[0] += w * g[0] + cx * g[3] + cy * g[6];
+            ug[1] += w * g[1] + cx * g[4] + cy * g[7];
+            ug[2] += w * g[2] + cx * g[5] + cy * g[8];
+          }
+        } else {
+          const double *g = f + d.at(blk, nvar, 0, kk, jj, ii);
+          const long long vs = d.cells();
+          ug[0] += w * g[0]; ug[1] += w * g[vs]; ug[2] += w * g[2 * vs];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 3; ++t) { wx[t] = X[t].w; wy[t] = Y[t].w; }
+}
+
+// the slots' weights alone
+__device__ __forceinline__ void slot_weights(const MCtx &M, const Ind &d, const CloudPos &c,
+                                             double wx[3], double wy[3], double wz[3]) {
+  AxisSlot s[3];
+  cloud_slots<false>(M, d, c, 0, s);
+#pragma unroll
+  for (int t = 0; t < 3; ++t) wx[t] = s[t].w;
+  cloud_slots<false>(M, d, c, 1, s);
+#pragma unroll
+  for (int t = 0; t < 3; ++t) wy[t] = s[t].w;
+  wz[0] = wz[2] = 0.0; wz[1] = 1.0;
+  if (d.three_d) {
+    cloud_slots<false>(M, d, c, 2, s);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) wz[t] = s[t].w;
+  }
+}
+
+// every cloud of the launch through cloud(p, position, stencil) and its deposit into variable v0
+// on of an nvar-variable field, cells beyond a block in the owning neighbour's active cells
+// (report: a cell no block owns sets the error bit)
+template <int NV, bool ONE, typename F>
+__device__ __forceinline__ void deposit_clouds(const MCtx &M, int npart, int nb, const Ind &d,
+                                               double *field, int nvar, int v0, unsigned *err,
+                                               F &&cloud) {
+  __shared__ WarpStage s_stage[kDepWarps];
+  WarpStage &st = s_stage[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  CellDeposit<NV, ONE> dep;
+  dep.init(d.three_d);
+  const long long vs = d.cells();
+  double *mine = field + ((long long)(dep.c * d.n2 + dep.b) * d.n1 + dep.a);
+  // the anchor's index is doubled: its low bit says that the window lies inside the block
+  auto at = [&](long long k2) -> double * {
+    if (k2 & 1) return mine + (k2 >> 1);
+    const unsigned cells = (unsigned)vs;
+    unsigned r = (unsigned)((k2 >> 1) / ((long long)nvar * cells));
+    const int m = (int)r;
+    r = (unsigned)((k2 >> 1) - ((long long)m * nvar + v0) * cells);
+    int k = (int)(r / (unsigned)(d.n1 * d.n2));
+    r -= (unsigned)(k * d.n1 * d.n2);
+    int j = (int)(r / (unsigned)d.n1), i = (int)(r - (unsigned)(j * d.n1));
+    i += dep.a - d.is; j += dep.b - d.js; k += dep.c - d.ks;
+    const int ox = (i < 0) ? -1 : ((i >= d.nx1) ? 1 : 0), oy = (j < 0) ? -1 : ((j >= d.nx2) ? 1 : 0);
+    const int oz = d.three_d ? ((k < 0) ? -1 : ((k >= d.nx3) ? 1 : 0)) : 0;
+    const int b = cloud_owner(M, d, m, ox, oy, oz);
+    if (b < 0) {
+      bool any = false;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) any = any || dep.acc[v] != 0.0;
+      if (any && err) report(err, DUSTB_ERR_CLOUD);
+      return nullptr;
+    }
+    return field + d.at(b, nvar, v0, d.ks + k - oz * d.nx3, d.js + j - oy * d.nx2, d.is + i - ox * d.nx1);
+  };
+  const long long first = ((long long)blockIdx.x * kDepWarps + (threadIdx.x >> 5)) * nb * 32;
+  for (int b = 0; b < nb; ++b) {
+    const long long p0 = first + 32LL * b;
+    if (p0 >= npart) break;
+    Stencil t;
+    CloudPos c;
+    c.L[0] = M.x1max - M.x1min; c.L[1] = M.x2max - M.x2min; c.L[2] = M.x3max - M.x3min;
+    const bool live = p0 + lane < npart && cloud((int)(p0 + lane), c, t);
+    unsigned key = kNoCell;
+    long long kb = 0;
+    if (live) {
+      const int k = d.ks + c.ic[2], j = d.js + c.ic[1], i = d.is + c.ic[0];
+      key = (unsigned)d.at(c.m, 1, 0, k, j, i);
+      kb = 2 * d.at(c.m, nvar, v0, k, j, i) + (c.inside ? 1 : 0);
+    }
+    const int slot = warp_rank(key, live);
+    double sum = 0.0;
+    if (live) {
+      st.put(slot, t.wx, t.wy, t.wz, t.fac, t.q, key, kb);
+#pragma unroll
+      for (int v = 0; v < NV - (ONE ? 1 : 0); ++v) sum += t.q[v];
+    }
+    const int n = __popc(__ballot_sync(0xffffffffu, live));
+    const bool check = __any_sync(0xffffffffu, !isfinite(sum));
+    __syncwarp();
+    dep.walk(st, n, check, vs, at);
+    __syncwarp();
+  }
+  dep.flush(vs, at);
+}
+
+// the stage position, block, level and cell of a cloud (cloud_load)
+__device__ __forceinline__ bool cloud_here(const PCtx &P, const MCtx &M, const Ind &d, int p,
+                                           double sh, CloudPos &c, unsigned *err) {
+  if (!cloud_load(P, M, d, p, sh, c.L, c.m, c.x, c.lev)) {
+    if (err) report(err, DUSTB_ERR_CLOUD);
+    return false;
+  }
+  cloud_cell(M, d, c);
+  return true;
+}
+
+__global__ void __launch_bounds__(32 * kDepWarps, 4)
+k_cloud_deposit_s(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh, unsigned *err, int nb) {
+  deposit_clouds<4, true>(M, P.npart, nb, d, qdep, 5, 0, err, [&](int p, CloudPos &c, Stencil &t) {
+    if (!cloud_here(P, M, d, p, sh, c, err)) return false;
+    slot_weights(M, d, c, t.wx, t.wy, t.wz);
+    const double mass_c = d.three_d ? P.r(DUSTB_IPM, p) * a_dt / (P.r(DUSTB_IPTS, p) + a_dt)
+                                    : P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt));
+    t.fac = mass_c / cloud_measure(M, d, c.m);
+    t.q[0] = P.r(DUSTB_IPVX, p); t.q[1] = P.r(DUSTB_IPVY, p); t.q[2] = P.r(DUSTB_IPVZ, p);
+    t.q[3] = 0.0;
+    return true;
+  });
+}
+
+__global__ void __launch_bounds__(32 * kDepWarps, 4)
+k_cloud_gather_kick_s(PCtx P, MCtx M, Ind d, const double *gp, double *dmom, double a_dt, double sh,
+                      int br, unsigned *err, int nb) {
+  deposit_clouds<3, false>(M, P.npart, nb, d, dmom, 3, 0, nullptr, [&](int p, CloudPos &c, Stencil &t) {
+    if (!cloud_here(P, M, d, p, sh, c, err)) return false;
+    double ug[3];
+    slot_gather<true>(M, d, c, gp, 0, ug, t.wx, t.wy, t.wz, err);
+    const double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
+    const double vx = P.r(DUSTB_IPVX, p), vy = P.r(DUSTB_IPVY, p), vz = P.r(DUSTB_IPVZ, p);
+    const double dvx = cj * (ug[0] - vx), dvy = cj * (ug[1] - vy), dvz = cj * (ug[2] - vz);
+    P.r(DUSTB_IPVX, p) = vx + dvx; P.r(DUSTB_IPVY, p) = vy + dvy; P.r(DUSTB_IPVZ, p) = vz + dvz;
+    P.r(DUSTB_IPRX, p) = dvx / a_dt; P.r(DUSTB_IPRY, p) = dvy / a_dt; P.r(DUSTB_IPRZ, p) = dvz / a_dt;
+    if (!br) return false;
+    t.fac = -P.r(DUSTB_IPM, p) / cloud_measure(M, d, c.m);
+    t.q[0] = dvx; t.q[1] = dvy; t.q[2] = dvz; t.q[3] = 0.0;
+    return true;
+  });
+}
+
+__global__ void __launch_bounds__(32 * kDepWarps, 4)
+k_cloud_operator_s(PCtx P, MCtx M, Ind d, const double *gp, double *result, double a_dt, double sh,
+                   unsigned *err, int nb) {
+  deposit_clouds<3, false>(M, P.npart, nb, d, result, 3, 0, nullptr, [&](int p, CloudPos &c, Stencil &t) {
+    if (!cloud_here(P, M, d, p, sh, c, err)) return false;
+    slot_gather<true>(M, d, c, gp, 0, t.q, t.wx, t.wy, t.wz, err);
+    t.fac = P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt)) / cloud_measure(M, d, c.m);
+    t.q[3] = 0.0;
+    return true;
+  });
+}
+
 // CloudDepositImplicitT (src/dust/dust_imex3d.cpp:61-99): Q = m c W / V, P = Q v
 template <int LF>
 __device__ __forceinline__ void k_cloud_deposit_body(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh,
@@ -2401,6 +2705,23 @@ __global__ void k_cloud_consistent_dust_u(PCtx P, MCtx M, Ind d, const double *r
 __global__ void __launch_bounds__(kThreads, 2) k_cloud_consistent_dust_l(PCtx P, MCtx M, Ind d, const double *res, double a_dt,
                                         double sh, int x3phys) { k_cloud_consistent_dust_body<1>(P, M, d, res, a_dt, sh, x3phys); }
 
+__global__ void k_cloud_consistent_dust_s(PCtx P, MCtx M, Ind d, const double *res, double a_dt,
+                                          double sh) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= P.npart) return;
+  if (P.r(DUSTB_IPM, p) <= 0.0) return;
+  CloudPos c;
+  c.L[0] = M.x1max - M.x1min; c.L[1] = M.x2max - M.x2min; c.L[2] = M.x3max - M.x3min;
+  if (!cloud_here(P, M, d, p, sh, c, nullptr)) return;
+  double rv[3], wx[3], wy[3], wz[3];
+  slot_gather<false>(M, d, c, res, 4, rv, wx, wy, wz, nullptr);
+  const double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
+  P.r(DUSTB_IPVX, p) += cj * rv[0]; P.r(DUSTB_IPVY, p) += cj * rv[1]; P.r(DUSTB_IPVZ, p) += cj * rv[2];
+  P.r(DUSTB_IPRX, p) += cj * rv[0] / a_dt;
+  P.r(DUSTB_IPRY, p) += cj * rv[1] / a_dt;
+  P.r(DUSTB_IPRZ, p) += cj * rv[2] / a_dt;
+}
+
 // ---- the clouds' pc2 (src/dust/dust_cloud3d.cpp:1362-1538, CloudPC2Push :76-150) ----------
 // PackGasGather3D: the gas velocity u1 momentum / density in every cell
 __global__ void k_gas_velocity_all(Ind d, const double *u, int nv, double *uv) {
@@ -2443,18 +2764,31 @@ __global__ void k_cloud_pc2_predictor_u(PCtx P, MCtx M, Ind d, const double *gp,
 __global__ void __launch_bounds__(kThreads, 2) k_cloud_pc2_predictor_l(PCtx P, MCtx M, Ind d, const double *gp, double *qdep,
                                       double dt, int rate_dep, int x3phys, unsigned *err) { k_cloud_pc2_predictor_body<1>(P, M, d, gp, qdep, dt, rate_dep, x3phys, err); }
 
+__global__ void __launch_bounds__(32 * kDepWarps, 4)
+k_cloud_pc2_predictor_s(PCtx P, MCtx M, Ind d, const double *gp, double *qdep, double dt,
+                        int rate_dep, unsigned *err, int nb) {
+  deposit_clouds<4, false>(M, P.npart, nb, d, qdep, 5, 1, nullptr, [&](int p, CloudPos &c, Stencil &t) {
+    if (!cloud_here(P, M, d, p, 0.0, c, err)) return false;
+    double ug[3];
+    slot_gather<true>(M, d, c, gp, 0, ug, t.wx, t.wy, t.wz, err);
+    const double mass_rate = P.r(DUSTB_IPM, p) / P.r(DUSTB_IPTS, p);
+    t.fac = 1.0 / cloud_measure(M, d, c.m);
+    t.q[0] = -dt * mass_rate * (ug[0] - P.r(DUSTB_IPVX, p));
+    t.q[1] = -dt * mass_rate * (ug[1] - P.r(DUSTB_IPVY, p));
+    t.q[2] = -dt * mass_rate * (ug[2] - P.r(DUSTB_IPVZ, p));
+    t.q[3] = rate_dep ? mass_rate : 0.0;
+    return true;
+  });
+}
+
 // CloudAdvanceT with CloudPC2Push's Midpoint / Kick / Drift
-template <int LF>
-__device__ __forceinline__ void k_cloud_pc2_advance_body(PCtx P, MCtx M, Ind d, const double *gp, double *dmom,
-                                    double dt, int br, int sbox, int strat, double q, double om,
-                                    double aphi, int x3phys, unsigned *err) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
-  const double L[3] = {M.x1max - M.x1min, M.x2max - M.x2min, M.x3max - M.x3min};
-  const int m = P.i(DUSTB_PGID, p) - M.gids, lev = P.i(DUSTB_PLEV, p);
-  const double x0[3] = {P.r(DUSTB_IPX1, p), P.r(DUSTB_IPY1, p), d.three_d ? P.r(DUSTB_IPZ1, p) : 0.0};
-  const double v0[3] = {P.r(DUSTB_IPVX1, p), P.r(DUSTB_IPVY1, p), P.r(DUSTB_IPVZ1, p)};
-  double xh[3], xg[3];
+// CloudPC2Push's Midpoint: the half-step position and the position the gas is gathered at
+struct CloudHalf { double x0[3], v0[3], xh[3], xg[3]; };
+__device__ __forceinline__ void cloud_midpoint(const PCtx &P, const Ind &d, int p, double dt,
+                                               int sbox, double q, double om, CloudHalf &H) {
+  double (&x0)[3] = H.x0, (&v0)[3] = H.v0, (&xh)[3] = H.xh, (&xg)[3] = H.xg;
+  x0[0] = P.r(DUSTB_IPX1, p); x0[1] = P.r(DUSTB_IPY1, p); x0[2] = d.three_d ? P.r(DUSTB_IPZ1, p) : 0.0;
+  v0[0] = P.r(DUSTB_IPVX1, p); v0[1] = P.r(DUSTB_IPVY1, p); v0[2] = P.r(DUSTB_IPVZ1, p);
   if (d.three_d) {
     xh[0] = x0[0] + 0.5 * dt * v0[0];
     xh[1] = x0[1] + 0.5 * dt * (v0[1] - (sbox ? q * om * x0[0] : 0.0));
@@ -2468,10 +2802,14 @@ __device__ __forceinline__ void k_cloud_pc2_advance_body(PCtx P, MCtx M, Ind d, 
     xh[2] = x0[2];
     xg[0] = xh[0]; xg[1] = xh[1]; xg[2] = xh[2];
   }
-  double x[3] = {xg[0], xg[1], xg[2]};
-  if (!cloud_frame_ok(M, d, m, lev, L, x, 1.0)) { report(err, DUSTB_ERR_CLOUD); return; }
-  double ug[3];
-  cloud_gather<LF>(M, d, m, x, lev, L, x3phys, gp, ug, err);
+}
+
+// ... its Kick and Drift from the gathered velocity; the impulse per mass in dv
+__device__ __forceinline__ void cloud_advance(const PCtx &P, const Ind &d, int p, double dt,
+                                              int sbox, int strat, double q, double om,
+                                              double aphi, const CloudHalf &H,
+                                              const double ug[3], double dv[3]) {
+  const double (&x0)[3] = H.x0, (&v0)[3] = H.v0, (&xh)[3] = H.xh;
   const double h = 0.5 * dt;
   const double lambda = h / P.r(DUSTB_IPTS, p);
   const double aa = 1.0 + lambda;
@@ -2516,14 +2854,52 @@ __device__ __forceinline__ void k_cloud_pc2_advance_body(PCtx P, MCtx M, Ind d, 
   const double dvy = dt * (ug[1] - vh[1]) / P.r(DUSTB_IPTS, p);
   const double dvz = dt * (ug[2] - vh[2]) / P.r(DUSTB_IPTS, p);
   P.r(DUSTB_IPRX, p) = dvx; P.r(DUSTB_IPRY, p) = dvy; P.r(DUSTB_IPRZ, p) = dvz;
+  dv[0] = dvx; dv[1] = dvy; dv[2] = dvz;
+}
+
+template <int LF>
+__device__ __forceinline__ void k_cloud_pc2_advance_body(PCtx P, MCtx M, Ind d, const double *gp, double *dmom,
+                                    double dt, int br, int sbox, int strat, double q, double om,
+                                    double aphi, int x3phys, unsigned *err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= P.npart) return;
+  const double L[3] = {M.x1max - M.x1min, M.x2max - M.x2min, M.x3max - M.x3min};
+  const int m = P.i(DUSTB_PGID, p) - M.gids, lev = P.i(DUSTB_PLEV, p);
+  CloudHalf H;
+  cloud_midpoint(P, d, p, dt, sbox, q, om, H);
+  double x[3] = {H.xg[0], H.xg[1], H.xg[2]};
+  if (!cloud_frame_ok(M, d, m, lev, L, x, 1.0)) { report(err, DUSTB_ERR_CLOUD); return; }
+  double ug[3], dv[3];
+  cloud_gather<LF>(M, d, m, x, lev, L, x3phys, gp, ug, err);
+  cloud_advance(P, d, p, dt, sbox, strat, q, om, aphi, H, ug, dv);
   if (!br) return;
   const double mass = -P.r(DUSTB_IPM, p);
   cloud_leaves<false, LF>(M, d, m, x, lev, L, x3phys, [&](const CloudLeaf &lf) {
     const double dw = mass * lf.w / cloud_measure(M, d, lf.b);
-    atomicAdd(&dmom[d.at(lf.b, 3, 0, lf.k, lf.j, lf.i)], dw * dvx);
-    atomicAdd(&dmom[d.at(lf.b, 3, 1, lf.k, lf.j, lf.i)], dw * dvy);
-    atomicAdd(&dmom[d.at(lf.b, 3, 2, lf.k, lf.j, lf.i)], dw * dvz);
+    atomicAdd(&dmom[d.at(lf.b, 3, 0, lf.k, lf.j, lf.i)], dw * dv[0]);
+    atomicAdd(&dmom[d.at(lf.b, 3, 1, lf.k, lf.j, lf.i)], dw * dv[1]);
+    atomicAdd(&dmom[d.at(lf.b, 3, 2, lf.k, lf.j, lf.i)], dw * dv[2]);
   }, nullptr);
+}
+__global__ void __launch_bounds__(32 * kDepWarps, 4)
+k_cloud_pc2_advance_s(PCtx P, MCtx M, Ind d, const double *gp, double *dmom, double dt, int br,
+                      int sbox, int strat, double q, double om, double aphi, unsigned *err, int nb) {
+  deposit_clouds<3, false>(M, P.npart, nb, d, dmom, 3, 0, nullptr, [&](int p, CloudPos &c, Stencil &t) {
+    c.m = P.i(DUSTB_PGID, p) - M.gids; c.lev = P.i(DUSTB_PLEV, p);
+    CloudHalf H;
+    cloud_midpoint(P, d, p, dt, sbox, q, om, H);
+    c.x[0] = H.xg[0]; c.x[1] = H.xg[1]; c.x[2] = H.xg[2];
+    // (a gather position up to a cell beyond the block)
+    if (!cloud_frame_ok(M, d, c.m, c.lev, c.L, c.x, 1.0)) { report(err, DUSTB_ERR_CLOUD); return false; }
+    cloud_cell(M, d, c);
+    double ug[3];
+    slot_gather<true>(M, d, c, gp, 0, ug, t.wx, t.wy, t.wz, err);
+    cloud_advance(P, d, p, dt, sbox, strat, q, om, aphi, H, ug, t.q);
+    if (!br) return false;
+    t.fac = -P.r(DUSTB_IPM, p) / cloud_measure(M, d, c.m);
+    t.q[3] = 0.0;
+    return true;
+  });
 }
 __global__ void k_cloud_pc2_advance_u(PCtx P, MCtx M, Ind d, const double *gp, double *dmom,
                                     double dt, int br, int sbox, int strat, double q, double om,
@@ -2929,7 +3305,8 @@ int dustb_cloud_deposit_qp(const dustb_ctx *c, double a_dt, double sh, void *str
   cudaMemsetAsync(c->f.qdep, 0, (size_t)(n_all(d) * 5) * sizeof(double), S(stream));
   if (c->part.npart > 0) {
     if (c->mesh.leaf) k_cloud_deposit_l<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, cloud_x3phys(c), c->err);
-    else k_cloud_deposit_u<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, cloud_x3phys(c), c->err);
+    else if (cloud_x3phys(c)) k_cloud_deposit_u<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, cloud_x3phys(c), c->err);
+    else k_cloud_deposit_s<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, c->err, NB(c));
   }
   return launch_status("cloud_deposit_qp");
 }
@@ -2945,8 +3322,10 @@ int dustb_cloud_gather_kick(const dustb_ctx *c, double a_dt, double sh, double *
   if (c->part.npart > 0) {
     if (c->mesh.leaf) k_cloud_gather_kick_l<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, a_dt, sh,
                                       c->phys.back_reaction, cloud_x3phys(c), c->err);
-    else k_cloud_gather_kick_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, a_dt, sh,
+    else if (cloud_x3phys(c)) k_cloud_gather_kick_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, a_dt, sh,
                                       c->phys.back_reaction, cloud_x3phys(c), c->err);
+    else k_cloud_gather_kick_s<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.dmom, a_dt, sh,
+                                      c->phys.back_reaction, c->err, NB(c));
   }
   return launch_status("cloud_gather_kick");
 }
@@ -2964,8 +3343,9 @@ int dustb_cloud_dc1_sweep(const dustb_ctx *c, double a_dt, double sh, double *gp
   if (c->part.npart > 0) {
     if (c->mesh.leaf) k_cloud_operator_l<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.work, a_dt, sh,
                                    cloud_x3phys(c), c->err);
-    else k_cloud_operator_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.work, a_dt, sh,
+    else if (cloud_x3phys(c)) k_cloud_operator_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.work, a_dt, sh,
                                    cloud_x3phys(c), c->err);
+    else k_cloud_operator_s<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.work, a_dt, sh, c->err, NB(c));
   }
   k_dc_correct<<<blocks_for(n_active(d)), kThreads, 0, S(stream)>>>(d, c->f.u0, c->f.nvar_gas,
                                                                     c->f.qdep, c->f.work,
@@ -2985,8 +3365,9 @@ int dustb_cloud_apply_pmbr(const dustb_ctx *c, double a_dt, double sh, void *str
   if (c->part.npart > 0) {
     if (c->mesh.leaf) k_cloud_consistent_dust_l<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt, sh,
                                           cloud_x3phys(c));
-    else k_cloud_consistent_dust_u<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt, sh,
+    else if (cloud_x3phys(c)) k_cloud_consistent_dust_u<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt, sh,
                                           cloud_x3phys(c));
+    else k_cloud_consistent_dust_s<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt, sh);
   }
   return launch_status("cloud_apply_pmbr");
 }
@@ -3005,8 +3386,9 @@ int dustb_cloud_pc2_predictor(const dustb_ctx *c, double dt, int rate_dep, doubl
   if (c->part.npart > 0) {
     if (c->mesh.leaf) k_cloud_pc2_predictor_l<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, rate_dep,
                                         cloud_x3phys(c), c->err);
-    else k_cloud_pc2_predictor_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, rate_dep,
+    else if (cloud_x3phys(c)) k_cloud_pc2_predictor_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, rate_dep,
                                         cloud_x3phys(c), c->err);
+    else k_cloud_pc2_predictor_s<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, rate_dep, c->err, NB(c));
   }
   return launch_status("cloud_pc2_predictor");
 }
@@ -3023,9 +3405,12 @@ int dustb_cloud_pc2_advance(const dustb_ctx *c, double dt, double *gpack, void *
     if (c->mesh.leaf) k_cloud_pc2_advance_l<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, dt,
                                       ph.back_reaction, ph.shearing_box, ph.stratified,
                                       ph.qshear, ph.omega0, ph.const_accel_phi, cloud_x3phys(c), c->err);
-    else k_cloud_pc2_advance_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, dt,
+    else if (cloud_x3phys(c)) k_cloud_pc2_advance_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, dt,
                                       ph.back_reaction, ph.shearing_box, ph.stratified,
                                       ph.qshear, ph.omega0, ph.const_accel_phi, cloud_x3phys(c), c->err);
+    else k_cloud_pc2_advance_s<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.dmom, dt,
+                                      ph.back_reaction, ph.shearing_box, ph.stratified,
+                                      ph.qshear, ph.omega0, ph.const_accel_phi, c->err, NB(c));
   }
   return launch_status("cloud_pc2_advance");
 }
