@@ -1140,35 +1140,70 @@ __global__ void k_pc2_commit(Ind d, double *u0, int nv, const double *dmom, cons
 // ---- ParticleHistory (the phst row), src/dust/dust_science.cpp:391-482 ------------------
 constexpr int kPhstChunk = 4096, kPhstSums = 7;
 
-// the particle sums of one chunk of 4096 particles, in particle order (dust_science.cpp:400-413)
-__global__ void k_phst_chunks(PCtx P, int zc, double *part, int nchunk) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nchunk) return;
-  double a[kPhstSums] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  const int p0 = c * kPhstChunk, p1 = min(p0 + kPhstChunk, P.npart);
-  for (int p = p0; p < p1; ++p) {
-    const double m = P.r(DUSTB_IPM, p);
-    if (m == 0.0) continue;                        // outflow tombstones
-    const double v1 = P.r(DUSTB_IPVX, p), v2 = P.r(DUSTB_IPVY, p), v3 = P.r(DUSTB_IPVZ, p);
-    const double z = P.r(zc, p);
-    a[0] += 1.0;
-    a[1] += m;
-    a[2] += m * v1; a[3] += m * v2; a[4] += m * v3;
-    a[5] += 0.5 * m * (v1 * v1 + v2 * v2 + v3 * v3);
-    a[6] += m * z * z;
+// the particle sums of one chunk of 4096 particles, in particle order (dust_science.cpp:400-413).
+// One CTA per chunk: four warps load 128 particles at a time, coalesced, and leave their seven
+// terms in shared memory; seven lanes of a fifth warp add the tile before in particle order, so
+// that the loads run beside the serial chain of additions, which bounds it.  (A term of a
+// massless particle is zero.)  3.5 M particles: 3.52 -> 0.06 ms against one thread per chunk.
+constexpr int kPhstTile = 128;
+__global__ void __launch_bounds__(kPhstTile + 32)
+k_phst_chunks(PCtx P, int zc, double *part) {
+  __shared__ double s_t[2][kPhstSums][kPhstTile + 2];
+  const int p0 = blockIdx.x * kPhstChunk, n = min(kPhstChunk, P.npart - p0);
+  const int nt = (n + kPhstTile - 1) / kPhstTile;
+  const int t = threadIdx.x, q = t - kPhstTile;
+  double sum = 0.0;
+  for (int k = 0; k <= nt; ++k) {
+    if (t < kPhstTile) {
+      if (k < nt) {
+        double a[kPhstSums] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        const int p = k * kPhstTile + t;
+        if (p < n) {
+          const double m = P.r(DUSTB_IPM, p0 + p);
+          if (m != 0.0) {                            // (outflow tombstones: no term)
+            const double v1 = P.r(DUSTB_IPVX, p0 + p), v2 = P.r(DUSTB_IPVY, p0 + p);
+            const double v3 = P.r(DUSTB_IPVZ, p0 + p), z = P.r(zc, p0 + p);
+            a[0] = 1.0;
+            a[1] = m;
+            a[2] = m * v1; a[3] = m * v2; a[4] = m * v3;
+            a[5] = 0.5 * m * (v1 * v1 + v2 * v2 + v3 * v3);
+            a[6] = m * z * z;
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < kPhstSums; ++c) s_t[k & 1][c][t] = a[c];
+      }
+    } else if (k > 0 && q < kPhstSums) {
+      const double *r = s_t[(k - 1) & 1][q];
+#pragma unroll 16
+      for (int x = 0; x < kPhstTile; ++x) sum += r[x];
+    }
+    __syncthreads();
   }
-  for (int q = 0; q < kPhstSums; ++q) part[(long long)c * kPhstSums + q] = a[q];
+  if (q >= 0 && q < kPhstSums) part[(long long)blockIdx.x * kPhstSums + q] = sum;
 }
 
-// the chunks summed in order (the host loop of dust_science.cpp:415-416), one thread
-__global__ void k_phst_sums(const double *part, int nchunk, const double *chi, int br,
-                            double *row) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  double s[kPhstSums] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int c = 0; c < nchunk; ++c)
-    for (int q = 0; q < kPhstSums; ++q) s[q] += part[(long long)c * kPhstSums + q];
-  for (int q = 0; q < 6; ++q) row[q] = s[q];
-  row[6] = (s[1] > 0.0) ? sqrt(s[6] / s[1]) : 0.0;
+// the chunks summed in order (the host loop of dust_science.cpp:415-416): one thread per sum,
+// the chunks' values staged by the CTA
+__global__ void __launch_bounds__(256)
+k_phst_sums(const double *part, int nchunk, const double *chi, int br, double *row) {
+  __shared__ double s_p[256 * kPhstSums];
+  __shared__ double s_s[kPhstSums];
+  double sum = 0.0;
+  for (int c0 = 0; c0 < nchunk; c0 += 256) {
+    const int n = min(256, nchunk - c0) * kPhstSums;
+    for (int x = threadIdx.x; x < n; x += 256) s_p[x] = part[(long long)c0 * kPhstSums + x];
+    __syncthreads();
+    if (threadIdx.x < kPhstSums)
+#pragma unroll 8
+      for (int x = threadIdx.x; x < n; x += kPhstSums) sum += s_p[x];
+    __syncthreads();
+  }
+  if (threadIdx.x < kPhstSums) s_s[threadIdx.x] = sum;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int q = 0; q < 6; ++q) row[q] = s_s[q];
+  row[6] = (s_s[1] > 0.0) ? sqrt(s_s[6] / s_s[1]) : 0.0;
   row[12] = (br && chi) ? *chi : -1.0;
   row[13] = -1.0;
   row[14] = 0.0;
@@ -1221,12 +1256,17 @@ __global__ void k_argmax_blocks(Ind d, const double *f, double *bval, long long 
   }
   if (threadIdx.x == 0) { bval[blockIdx.x] = sv[0]; bloc[blockIdx.x] = sq[0]; }
 }
-__global__ void k_argmax_final(Ind d, MCtx M, const double *bval, const long long *bloc,
-                               int nb, double *row) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
+__global__ void __launch_bounds__(256)
+k_argmax_final(Ind d, MCtx M, const double *bval, const long long *bloc, int nb, double *row) {
+  __shared__ double sv[256];
+  __shared__ long long sq[256];
   double v = 0.0;
   long long q = -1;
-  for (int b = 0; b < nb; ++b) if (bloc[b] >= 0) better(v, q, bval[b], bloc[b]);
+  for (int b = threadIdx.x; b < nb; b += 256) if (bloc[b] >= 0) better(v, q, bval[b], bloc[b]);
+  sv[threadIdx.x] = v; sq[threadIdx.x] = q;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int t = 1; t < 256; ++t) if (sq[t] >= 0) better(v, q, sv[t], sq[t]);
   row[7] = (q >= 0 && v > 0.0) ? v : 0.0;
   row[8] = row[9] = row[10] = 0.0;
   row[11] = -1.0;
@@ -3254,15 +3294,15 @@ int dustb_phst(const dustb_ctx *c, const double *chi_max, double *row, void *scr
   double *bval = (double *)b;
   long long *bloc = (long long *)(b + 1024 * 8);
   cudaMemsetAsync(part, 0, (size_t)nchunk * kPhstSums * 8, S(stream));
-  if (np > 0) k_phst_chunks<<<blocks_for(nchunk), kThreads, 0, S(stream)>>>(pview(c), DUSTB_IPZ, part, nchunk);
-  k_phst_sums<<<1, 1, 0, S(stream)>>>(part, nchunk, chi_max, c->phys.back_reaction, row);
+  if (np > 0) k_phst_chunks<<<nchunk, kPhstTile + 32, 0, S(stream)>>>(pview(c), DUSTB_IPZ, part);
+  k_phst_sums<<<1, 256, 0, S(stream)>>>(part, nchunk, chi_max, c->phys.back_reaction, row);
   cudaMemsetAsync(field, 0, (size_t)d.cells() * d.nmb * 8, S(stream));
   if (np > 0) k_mass_deposit<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, field, c->err, NB(c));
   int rc = dustb_ghost_add(c, field, 1, stream);
   if (rc) return rc;
   const int nb = 1024;
   k_argmax_blocks<<<nb, 256, 0, S(stream)>>>(d, field, bval, bloc);
-  k_argmax_final<<<1, 1, 0, S(stream)>>>(d, mview(c), bval, bloc, nb, row);
+  k_argmax_final<<<1, 256, 0, S(stream)>>>(d, mview(c), bval, bloc, nb, row);
   return launch_status("phst");
 }
 
