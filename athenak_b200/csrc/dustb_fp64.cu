@@ -112,16 +112,40 @@ __global__ void k_reg_copy(PCtx P) {
   P.r(DUSTB_IPVZ1, p) = P.r(DUSTB_IPVZ, p);
 }
 
-// active-cell loop helper: idx over nmb*nx3*nx2*nx1
+// active-cell loop helper: idx over nmb*nx3*nx2*nx1 (32-bit divisions where the count allows:
+// the 64-bit ones were most of a small cell kernel's instructions)
 __device__ __forceinline__ bool active_cell(const Ind &d, long long idx, int &m, int &k, int &j,
                                             int &i) {
-  long long n = (long long)d.nmb * d.nx3 * d.nx2 * d.nx1;
+  const long long n = (long long)d.nmb * d.nx3 * d.nx2 * d.nx1;
   if (idx >= n) return false;
+  if (n <= 0x7fffffffLL) {
+    unsigned u = (unsigned)idx, q = u / (unsigned)d.nx1;
+    i = (int)(u - q * (unsigned)d.nx1) + d.is; u = q;
+    q = u / (unsigned)d.nx2;
+    j = (int)(u - q * (unsigned)d.nx2) + d.js; u = q;
+    q = u / (unsigned)d.nx3;
+    k = (int)(u - q * (unsigned)d.nx3) + d.ks;
+    m = (int)q;
+    return true;
+  }
   i = (int)(idx % d.nx1) + d.is; idx /= d.nx1;
   j = (int)(idx % d.nx2) + d.js; idx /= d.nx2;
   k = (int)(idx % d.nx3) + d.ks; idx /= d.nx3;
   m = (int)idx;
   return true;
+}
+
+// block m and padded cell c of idx over nmb * per padded cells
+__device__ __forceinline__ void block_cell(long long idx, long long per, long long total, int &m,
+                                           long long &c) {
+  if (total <= 0x7fffffffLL) {
+    const unsigned q = (unsigned)idx / (unsigned)per;
+    m = (int)q;
+    c = (unsigned)idx - q * (unsigned)per;
+  } else {
+    m = (int)(idx / per);
+    c = idx - (long long)m * per;
+  }
 }
 
 __global__ void k_gas_rk(Ind d, double *u0, const double *u1, int nv, double g0, double g1) {
@@ -350,11 +374,13 @@ __device__ double shear_add_sum(const SBox &B, const Ind &d, const double *a, in
             const long long sj = Y - (long long)sb2 * B.nx2 + d.js;
             if (sj < 0 || sj >= d.n2) continue;
             const double ya = (double)Y + sh, yb = (double)(Y + 1) + sh;
-            for (int im = -2; im <= 2; ++im) {
-              const double clo = (double)(J + im * N2), chi = clo + 1.0;
-              const double o = fmin(yb, chi) - fmax(ya, clo);
-              if (o > 0.0) sum += o * a[d.at(S, nvar, v, sk, (int)sj, si)];
-            }
+            // the one image of this row that the interval can overlap: the nearest (the rows
+            // are a cell wide and their images N2 >= 2 cells apart)
+            const int im = __double2int_rn((ya - (double)J) / (double)N2);
+            if (im < -2 || im > 2) continue;
+            const double clo = (double)(J + im * N2), chi = clo + 1.0;
+            const double o = fmin(yb, chi) - fmax(ya, clo);
+            if (o > 0.0) sum += o * a[d.at(S, nvar, v, sk, (int)sj, si)];
           }
       }
     }
@@ -619,7 +645,7 @@ k_scatter(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh, unsigned 
 // cells reach), enumerated per block: the near x3 planes whole (zn of them), then in each of
 // the zin inner planes its near x2 rows whole (yn) and, in each of its yin inner rows, the xn
 // cells near the x1 faces.  A dimension the mesh lacks has no near part (zn = 0, zin = nx3).
-struct Shell { int zn, zin, yn, yin, xn, xin, zoff, yoff; long long per; };
+struct Shell { int zn, zin, yn, yin, xn, xin, zoff, yoff, per; };
 
 __host__ __device__ inline Shell make_shell(const Ind &d) {
   Shell h;
@@ -632,96 +658,99 @@ __host__ __device__ inline Shell make_shell(const Ind &d) {
   h.zin = d.nx3 - h.zn;
   h.yoff = d.multi_d ? d.ng : 0;
   h.zoff = d.three_d ? d.ng : 0;
-  h.per = (long long)h.zn * d.nx2 * d.nx1 +
-          (long long)h.zin * ((long long)h.yn * d.nx1 + (long long)h.yin * h.xn);
+  h.per = h.zn * d.nx2 * d.nx1 + h.zin * (h.yn * d.nx1 + h.yin * h.xn);
   return h;
 }
 
 // t in [0, per) -> the cell's offsets from (ks, js, is)
-__device__ __forceinline__ void shell_cell(const Ind &d, const Shell &h, long long t, int &k,
-                                           int &j, int &i) {
-  const long long plane = (long long)d.nx2 * d.nx1;
-  if (t < (long long)h.zn * plane) {
-    const int z = (int)(t / plane);
-    const long long r = t - z * plane;
+__device__ __forceinline__ void shell_cell(const Ind &d, const Shell &h, int t, int &k, int &j,
+                                           int &i) {
+  const int plane = d.nx2 * d.nx1;
+  if (t < h.zn * plane) {
+    const int z = t / plane, r = t - z * plane;
     k = z < d.ng ? z : z + h.zin;
-    j = (int)(r / d.nx1);
-    i = (int)(r - (long long)j * d.nx1);
+    j = r / d.nx1;
+    i = r - j * d.nx1;
     return;
   }
-  t -= (long long)h.zn * plane;
-  const long long inner = (long long)h.yn * d.nx1 + (long long)h.yin * h.xn;
-  const int z = (int)(t / inner);
-  long long r = t - z * inner;
+  t -= h.zn * plane;
+  const int inner = h.yn * d.nx1 + h.yin * h.xn;
+  const int z = t / inner;
+  int r = t - z * inner;
   k = h.zoff + z;
-  if (r < (long long)h.yn * d.nx1) {
-    const int y = (int)(r / d.nx1);
+  if (r < h.yn * d.nx1) {
+    const int y = r / d.nx1;
     j = y < d.ng ? y : y + h.yin;
-    i = (int)(r - (long long)y * d.nx1);
+    i = r - y * d.nx1;
     return;
   }
-  r -= (long long)h.yn * d.nx1;
-  const int y = (int)(r / h.xn);
-  const int u = (int)(r - (long long)y * h.xn);
+  r -= h.yn * d.nx1;
+  const int y = r / h.xn;
+  const int u = r - y * h.xn;
   j = h.yoff + y;
   i = u < d.ng ? u : u + h.xin;
 }
 
-// fold: fold the ghost deposits beyond physical x3 faces back into the mirrored active cells
-__global__ void k_ghost_add(Ind d, const int *nghbr, int gids, double *a, int nvar, int fold,
-                            SBox B) {
-  int m, k, j, i;
-  const Shell sh = make_shell(d);
-  long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long ncell = (long long)d.nmb * sh.per;
-  int v = (int)(idx / ncell);
-  if (v >= nvar) return;
-  {
-    const long long r = idx - (long long)v * ncell;
-    m = (int)(r / sh.per);
-    shell_cell(d, sh, r - (long long)m * sh.per, k, j, i);
-    k += d.ks; j += d.js; i += d.is;
-  }
+// fold: fold the ghost deposits beyond physical x3 faces back into the mirrored active cells.
+// Grid: x over the shell cells of a block, y over blocks and variables.  The directions are
+// unrolled, so that each one's test is a combination of six flags of the cell (looped over the
+// table in constant memory with 64-bit index divisions, an exchange of 64^3 cells and five
+// variables took 28 us against 8)
+__global__ void __launch_bounds__(kThreads)
+k_ghost_add(Ind d, const int *nghbr, int gids, double *a, int nvar, int fold, SBox B, Shell sh) {
+  constexpr signed char kDir[26][3] = {
+      {-1, 0, 0}, {1, 0, 0}, {0, -1, 0}, {0, 1, 0},
+      {-1, -1, 0}, {1, -1, 0}, {-1, 1, 0}, {1, 1, 0},
+      {0, 0, -1}, {0, 0, 1},
+      {-1, 0, -1}, {1, 0, -1}, {-1, 0, 1}, {1, 0, 1},
+      {0, -1, -1}, {0, 1, -1}, {0, -1, 1}, {0, 1, 1},
+      {-1, -1, -1}, {1, -1, -1}, {-1, 1, -1}, {1, 1, -1},
+      {-1, -1, 1}, {1, -1, 1}, {-1, 1, 1}, {1, 1, 1}};     // kDirOrder
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= sh.per) return;
+  int k, j, i;
+  shell_cell(d, sh, t, k, j, i);
+  k += d.ks; j += d.js; i += d.is;
   const int ng1 = d.ng - 1;
-  const int ndir = d.three_d ? 26 : (d.multi_d ? 8 : 2);
-  const long long at = d.at(m, nvar, v, k, j, i);
-  double val = a[at];
-  for (int n = 0; n < ndir; ++n) {
-    const int o1 = kDirOrder[n][0], o2 = kDirOrder[n][1], o3 = kDirOrder[n][2];
-    if (o1 > 0 && i < d.ie - ng1) continue;
-    if (o1 < 0 && i > d.is + ng1) continue;
-    if (o2 > 0 && j < d.je - ng1) continue;
-    if (o2 < 0 && j > d.js + ng1) continue;
-    if (o3 > 0 && k < d.ke - ng1) continue;
-    if (o3 < 0 && k > d.ks + ng1) continue;
-    const int src = nghbr[(long long)m * 27 + dir_slot(o1, o2, o3)] - gids;
-    if (src < 0 || src >= d.nmb || B.crossing(m, o1)) continue;
-    val += a[d.at(src, nvar, v, k - o3 * d.nx3, j - o2 * d.nx2, i - o1 * d.nx1)];
-  }
-  if (fold && d.three_d) {
-    // a physical x3 face (no neighbour across it): the ghost plane ks-1-t (ke+1+t) folds into
-    // the active plane ks+t (ke-t); the block's own column, then its x1/x2 neighbours'
-    // ghost strips that face this cell, in NeighborIndex order
-    for (int side = 0; side < 2; ++side) {
-      const int o3 = side ? 1 : -1;
-      if (side == 0 ? (k > d.ks + ng1) : (k < d.ke - ng1)) continue;
-      if (nghbr[(long long)m * 27 + dir_slot(0, 0, o3)] >= 0) continue;
-      const int kg = side ? 2 * d.ke + 1 - k : 2 * d.ks - 1 - k;
-      val += a[d.at(m, nvar, v, kg, j, i)];
-      for (int n = 0; n < ndir; ++n) {
-        const int o1 = kDirOrder[n][0], o2 = kDirOrder[n][1];
-        if (kDirOrder[n][2] != 0) continue;
-        if (o1 > 0 && i < d.ie - ng1) continue;
-        if (o1 < 0 && i > d.is + ng1) continue;
-        if (o2 > 0 && j < d.je - ng1) continue;
-        if (o2 < 0 && j > d.js + ng1) continue;
-        const int src = nghbr[(long long)m * 27 + dir_slot(o1, o2, 0)] - gids;
-        if (src < 0 || src >= d.nmb || B.crossing(m, o1)) continue;
-        val += a[d.at(src, nvar, v, kg, j - o2 * d.nx2, i - o1 * d.nx1)];
+  const bool near[3][3] = {{i <= d.is + ng1, true, i >= d.ie - ng1},
+                           {j <= d.js + ng1, true, j >= d.je - ng1},
+                           {k <= d.ks + ng1, true, k >= d.ke - ng1}};
+  for (int mv = blockIdx.y; mv < d.nmb * nvar; mv += gridDim.y) {
+    const int m = mv / nvar, v = mv - m * nvar;
+    const int *nb = nghbr + (long long)m * 27;
+    const long long at = d.at(m, nvar, v, k, j, i);
+    double val = a[at];
+    const bool cm = B.crossing(m, -1), cp = B.crossing(m, 1);
+#pragma unroll
+    for (int n = 0; n < 26; ++n) {
+      const int o1 = kDir[n][0], o2 = kDir[n][1], o3 = kDir[n][2];
+      if ((o3 != 0 && !d.three_d) || (o2 != 0 && !d.multi_d)) continue;
+      if (!(near[0][o1 + 1] && near[1][o2 + 1] && near[2][o3 + 1])) continue;
+      const int src = nb[dir_slot(o1, o2, o3)] - gids;
+      if (src < 0 || src >= d.nmb || (o1 < 0 && cm) || (o1 > 0 && cp)) continue;
+      val += a[d.at(src, nvar, v, k - o3 * d.nx3, j - o2 * d.nx2, i - o1 * d.nx1)];
+    }
+    if (fold && d.three_d) {
+      // a physical x3 face (no neighbour across it): the ghost plane ks-1-t (ke+1+t) folds into
+      // the active plane ks+t (ke-t); the block's own column, then its x1/x2 neighbours'
+      // ghost strips that face this cell, in NeighborIndex order
+      for (int side = 0; side < 2; ++side) {
+        if (!near[2][side ? 2 : 0]) continue;
+        if (nb[dir_slot(0, 0, side ? 1 : -1)] >= 0) continue;
+        const int kg = side ? 2 * d.ke + 1 - k : 2 * d.ks - 1 - k;
+        val += a[d.at(m, nvar, v, kg, j, i)];
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+          const int o1 = kDir[n][0], o2 = kDir[n][1];
+          if (!(near[0][o1 + 1] && near[1][o2 + 1])) continue;
+          const int src = nb[dir_slot(o1, o2, 0)] - gids;
+          if (src < 0 || src >= d.nmb || (o1 < 0 && cm) || (o1 > 0 && cp)) continue;
+          val += a[d.at(src, nvar, v, kg, j - o2 * d.nx2, i - o1 * d.nx1)];
+        }
       }
     }
+    a[at] = val;
   }
-  a[at] = val;
 }
 
 // shear-periodic x1 faces: the remapped ghost cells beyond them, their sum added as
@@ -751,42 +780,46 @@ __global__ void k_shear_add(Ind d, SBox B, double *a, int nvar) {
 // the general deposit remap of a refined mesh (GeneralApply, bvals_dep_general.cpp:1135-1175):
 // one thread per (target cell, variable), its sources summed in list order and added once.
 // Sources are ghost cells and targets active cells, so no thread reads what another writes.
+// (32-bit divisions: an entry's cell index is an int)
 __global__ void k_dep_plan_apply(int nseg, const int *__restrict__ tgt, const int *__restrict__ ptr,
                                  const int *__restrict__ src, const double *__restrict__ w,
-                                 double *a, int nvar, long long ncell) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= (long long)nseg * nvar) return;
-  const int s = (int)(t / nvar), v = (int)(t - (long long)s * nvar);
+                                 double *a, int nvar, unsigned ncell) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x, v = blockIdx.y;
+  if (s >= nseg) return;
   double sum = 0.0;
   for (int e = ptr[s]; e < ptr[s + 1]; ++e) {
-    const long long q = src[e];
-    const long long sm = q / ncell;
-    sum += w[e] * a[(sm * nvar + v) * ncell + (q - sm * ncell)];
+    const unsigned q = (unsigned)src[e], sm = q / ncell;
+    sum += w[e] * a[((long long)sm * nvar + v) * ncell + (q - sm * ncell)];
   }
-  const long long c = tgt[s];
-  const long long tm = c / ncell;
-  a[(tm * nvar + v) * ncell + (c - tm * ncell)] += sum;
+  const unsigned c = (unsigned)tgt[s], tm = c / ncell;
+  a[((long long)tm * nvar + v) * ncell + (c - tm * ncell)] += sum;
 }
 
-// copy exchange: every ghost cell <- the neighbour's active cell at index - o*nx
-__global__ void k_ghost_copy(Ind d, const int *nghbr, int gids, double *a, int nvar) {
-  long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  long long per = d.cells();
-  long long tot = per * d.nmb;
-  if (idx >= tot) return;
-  int m = (int)(idx / per);
-  long long r = idx - (long long)m * per;
-  int i = (int)(r % d.n1); r /= d.n1;
-  int j = (int)(r % d.n2);
-  int k = (int)(r / d.n2);
-  int o1 = (i < d.is) ? -1 : ((i > d.ie) ? 1 : 0);
-  int o2 = (j < d.js) ? -1 : ((j > d.je) ? 1 : 0);
-  int o3 = (k < d.ks) ? -1 : ((k > d.ke) ? 1 : 0);
-  if (o1 == 0 && o2 == 0 && o3 == 0) return;
-  const int src = nghbr[(long long)m * 27 + dir_slot(o1, o2, o3)] - gids;
-  if (src < 0 || src >= d.nmb) return;
-  for (int v = 0; v < nvar; ++v)
-    a[d.at(m, nvar, v, k, j, i)] = a[d.at(src, nvar, v, k - o3 * d.nx3, j - o2 * d.nx2, i - o1 * d.nx1)];
+// copy exchange: every ghost cell <- the neighbour's active cell at index - o*nx.  One warp per
+// row of a block: the whole row in a ghost row, the 2 ng ghost columns (of all variables at
+// once) in the others, so that no thread is started for an active cell (a thread per padded
+// cell with 64-bit index divisions: 42 us against 10 for 4 variables of eight blocks of 64^3)
+__global__ void __launch_bounds__(kThreads)
+k_ghost_copy(Ind d, const int *nghbr, int gids, double *a, int nvar) {
+  const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= d.n2 * d.n3) return;
+  const int k = row / d.n2, j = row - k * d.n2;
+  const int o2 = (j < d.js) ? -1 : ((j > d.je) ? 1 : 0);
+  const int o3 = (k < d.ks) ? -1 : ((k > d.ke) ? 1 : 0);
+  const bool inner = o2 == 0 && o3 == 0;
+  const int cols = inner ? 2 * d.ng : d.n1;
+  for (int m = blockIdx.y; m < d.nmb; m += gridDim.y) {
+    const int *nb = nghbr + (long long)m * 27;
+    for (int x = lane; x < cols * nvar; x += 32) {
+      const int v = x / cols, c = x - v * cols;
+      const int i = (inner && c >= d.ng) ? c + d.nx1 : c;
+      const int o1 = (i < d.is) ? -1 : ((i > d.ie) ? 1 : 0);
+      const int src = nb[dir_slot(o1, o2, o3)] - gids;
+      if (src < 0 || src >= d.nmb) continue;
+      a[d.at(m, nvar, v, k, j, i)] =
+          a[d.at(src, nvar, v, k - o3 * d.nx3, j - o2 * d.nx2, i - o1 * d.nx1)];
+    }
+  }
 }
 
 // UstarX3BCs, src/dust/dust_tasks.cpp:445-469
@@ -1061,10 +1094,11 @@ __global__ void k_pc2_apply(Ind d, double *u0, int nv, double *qdep, double dt, 
 // dust_gas_midpoint, dust_push.cpp:53-59 (ghosts included)
 __global__ void k_pc2_midpoint(Ind d, const double *u0, const double *u1, int nv, double *us) {
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  long long per = d.cells();
+  const long long per = d.cells();
   if (idx >= per * d.nmb) return;
-  int m = (int)(idx / per);
-  long long c = idx - (long long)m * per;
+  int m;
+  long long c;
+  block_cell(idx, per, per * d.nmb, m, c);
   const long long b0 = ((long long)m * nv) * per + c;
   double inv = 1.0 / (u1[b0] + u0[b0]);
   for (int v = 0; v < 3; ++v) {
@@ -2768,8 +2802,9 @@ __global__ void k_gas_velocity_all(Ind d, const double *u, int nv, double *uv) {
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long per = d.cells();
   if (idx >= per * d.nmb) return;
-  const int m = (int)(idx / per);
-  const long long r = idx - (long long)m * per;
+  int m;
+  long long r;
+  block_cell(idx, per, per * d.nmb, m, r);
   const long long base = (long long)m * nv * per;
   const double invrho = 1.0 / u[base + r];
   for (int v = 0; v < 3; ++v) uv[((long long)m * 3 + v) * per + r] = u[base + (1 + v) * per + r] * invrho;
@@ -3104,8 +3139,10 @@ int dustb_ghost_add(const dustb_ctx *c, double *field, int nvar, void *stream) {
   Ind d = make_ind(c->mesh);
   const int fold = d.three_d && c->mesh.x3bc != DUSTB_X3_PERIODIC && !c->phys.x3_deposit_drop;
   const SBox B = sbview(c);
-  k_ghost_add<<<blocks_for(make_shell(d).per * d.nmb * nvar), kThreads, 0, S(stream)>>>(d, c->mesh.nghbr, c->mesh.gids, field, nvar, fold,
-                                                                          B);
+  const Shell sh = make_shell(d);
+  const long long nmv = (long long)d.nmb * nvar;
+  k_ghost_add<<<dim3(blocks_for(sh.per), (unsigned)(nmv < 65535 ? nmv : 65535)), kThreads, 0, S(stream)>>>(
+      d, c->mesh.nghbr, c->mesh.gids, field, nvar, fold, B, sh);
   if (B.on) {
     if (!B.sb_gid || B.nb2 <= 0 || B.nb3 <= 0) return DUSTB_EINVAL;
     k_shear_add<<<blocks_for((long long)d.nmb * nvar * d.nx3 * d.nx2 * 2 * d.ng), kThreads, 0, S(stream)>>>(
@@ -3121,9 +3158,9 @@ int dustb_ghost_add_plan(const dustb_ctx *c, const dustb_dep_plan *plan, double 
   if (plan->nseg == 0) return DUSTB_OK;
   if (!plan->seg_tgt || !plan->seg_ptr || !plan->ent_src || !plan->ent_w) return DUSTB_EINVAL;
   Ind d = make_ind(c->mesh);
-  k_dep_plan_apply<<<blocks_for((long long)plan->nseg * nvar), kThreads, 0, S(stream)>>>(
+  k_dep_plan_apply<<<dim3(blocks_for(plan->nseg), (unsigned)nvar), kThreads, 0, S(stream)>>>(
       plan->nseg, plan->seg_tgt, plan->seg_ptr, plan->ent_src, plan->ent_w, field, nvar,
-      d.cells());
+      (unsigned)d.cells());
   return launch_status("ghost_add_plan");
 }
 
@@ -3132,7 +3169,9 @@ int dustb_ghost_copy(const dustb_ctx *c, double *field, int nvar, int x3_bcs, vo
   if (!field || nvar <= 0) return DUSTB_EINVAL;
   if (c->mesh.nghbr_ml) return DUSTB_EUNSUP;        // (no prolongation across levels)
   Ind d = make_ind(c->mesh);
-  k_ghost_copy<<<blocks_for(n_all(d)), kThreads, 0, S(stream)>>>(d, c->mesh.nghbr, c->mesh.gids, field, nvar);
+  k_ghost_copy<<<dim3((unsigned)((d.n2 * d.n3 + kThreads / 32 - 1) / (kThreads / 32)),
+                      (unsigned)(d.nmb < 65535 ? d.nmb : 65535)), kThreads, 0, S(stream)>>>(
+      d, c->mesh.nghbr, c->mesh.gids, field, nvar);
   const SBox B = sbview(c);
   if (B.on) {
     // the shearing box remap of the x1 ghost strips, after the plain copy and before the
