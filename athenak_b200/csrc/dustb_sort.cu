@@ -51,7 +51,7 @@ __global__ void k_keys(const double *pr, const int *pi, long long stride, int np
   atomicAdd(&count[c], 1);
 }
 
-// ---- exclusive scan of n ints in place (three kernels) ---------------------------------
+// ---- exclusive scan of n ints in place ---------------------------------------------------
 __device__ __forceinline__ int block_excl_scan(int v, int *sh, int &total) {
   // warp inclusive scan
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -105,8 +105,20 @@ __global__ void k_scan_sums(int *bsum, int nb) {
   }
 }
 
-__global__ void k_scan_apply(int *a, long long n, const int *bsum) {
+// scanned: bsum holds the exclusive sums of the tiles; else their totals, and the CTA adds up
+// those before its own (copy: a second array that takes the result, or null)
+__global__ void k_scan_apply(int *a, long long n, const int *bsum, int scanned, int *copy) {
   __shared__ int sh[32];
+  __shared__ int s_base;
+  if (scanned) {
+    if (threadIdx.x == 0) s_base = bsum[blockIdx.x];
+  } else {
+    int t = 0, total;
+    for (int x = threadIdx.x; x < (int)blockIdx.x; x += kScanT) t += bsum[x];
+    block_excl_scan(t, sh, total);
+    if (threadIdx.x == 0) s_base = total;
+  }
+  __syncthreads();
   long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
   int v[kScanItems];
   int s = 0;
@@ -116,10 +128,13 @@ __global__ void k_scan_apply(int *a, long long n, const int *bsum) {
     s += v[r];
   }
   int total;
-  int ex = block_excl_scan(s, sh, total) + bsum[blockIdx.x];
+  int ex = block_excl_scan(s, sh, total) + s_base;
   for (int r = 0; r < kScanItems; ++r) {
     long long idx = base + r;
-    if (idx < n) a[idx] = ex;
+    if (idx < n) {
+      a[idx] = ex;
+      if (copy) copy[idx] = ex;
+    }
     ex += v[r];
   }
 }
@@ -155,14 +170,16 @@ __device__ void sift_down(int *a, int root, int n) {
   }
 }
 
+// (a thread per cell; runs of 49 to 1024 are k_sort_long's)
+constexpr int kRunLane = 48, kRunWarp = 1024;
 __global__ void k_sort_runs(const int *cstart, long long ncell, int *order) {
   long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= ncell) return;
   int b = cstart[c], e = cstart[c + 1];
   int n = e - b;
-  if (n < 2) return;
+  if (n < 2 || (n > kRunLane && n <= kRunWarp)) return;
   int *a = order + b;
-  if (n <= 48) {
+  if (n <= kRunLane) {
     for (int x = 1; x < n; ++x) {
       int v = a[x];
       int y = x - 1;
@@ -176,6 +193,38 @@ __global__ void k_sort_runs(const int *cstart, long long ncell, int *order) {
     int t = a[0]; a[0] = a[x]; a[x] = t;
     sift_down(a, 0, x);
   }
+}
+
+// the long runs of clumped cells, a warp per cell: every lane counts the smaller elements of
+// each of its NT, which is its place in the run (n^2 / 32 comparisons without a dependent
+// step; one thread's heap sort of 220 particles took 0.26 ms of a stratified layer's sort)
+template <int NT>
+__device__ __forceinline__ void rank_run(int *a, int n, int lane) {
+  int v[NT], place[NT];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    place[t] = 0;
+    v[t] = (t * 32 + lane < n) ? a[t * 32 + lane] : 0x7fffffff;
+  }
+#pragma unroll 4
+  for (int y = 0; y < n; ++y) {
+    const int w = a[y];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) place[t] += w < v[t];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+    if (t * 32 + lane < n) a[place[t]] = v[t];
+}
+__global__ void k_sort_long(const int *cstart, long long ncell, int *order) {
+  const long long c = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  if (c >= ncell) return;
+  const int b = cstart[c], n = cstart[c + 1] - b, lane = threadIdx.x & 31;
+  if (n <= kRunLane || n > kRunWarp) return;
+  if (n <= 128) rank_run<4>(order + b, n, lane);
+  else if (n <= 256) rank_run<8>(order + b, n, lane);
+  else rank_run<32>(order + b, n, lane);
 }
 
 // every row of particle order[k] into slot k of the spare arrays
@@ -201,11 +250,15 @@ long long csr_scratch_bytes(long long ncell, long long n) {
                      align256(sizeof(int) * (size_t)(nb + 1)));
 }
 
-int exclusive_scan(int *a, long long n, int *bsum, cudaStream_t st) {
-  long long nb = (n + kScanTile - 1) / kScanTile;
+int exclusive_scan(int *a, long long n, int *bsum, cudaStream_t st, int *copy) {
+  const long long nb = (n + kScanTile - 1) / kScanTile;
+  // up to 4096 tiles (16.8 M ints) every CTA adds up the tiles before its own, at most four
+  // loads a thread, and the launch over the sums is left out (a launch is 2.5 us of the 7 us a
+  // scan of 32 K ints takes); beyond that the sums are scanned once
+  const bool two = nb <= 4096;
   k_scan_reduce<<<(unsigned)nb, kScanT, 0, st>>>(a, n, bsum);
-  k_scan_sums<<<1, kScanT, 0, st>>>(bsum, (int)nb);
-  k_scan_apply<<<(unsigned)nb, kScanT, 0, st>>>(a, n, bsum);
+  if (!two) k_scan_sums<<<1, kScanT, 0, st>>>(bsum, (int)nb);
+  k_scan_apply<<<(unsigned)nb, kScanT, 0, st>>>(a, n, bsum, two ? 0 : 1, copy);
   return dustb_host::launch_status("exclusive_scan");
 }
 
@@ -213,11 +266,14 @@ int exclusive_scan(int *a, long long n, int *bsum, cudaStream_t st) {
 // per-cell counts on entry; cursor (ncell + 1 ints) and bsum are scratch.
 int csr_build(const int *key, int n, long long ncell, int *cstart, int *order, int *cursor,
               int *bsum, bool ordered_runs, cudaStream_t st) {
-  int rc = exclusive_scan(cstart, ncell + 1, bsum, st);
+  int rc = exclusive_scan(cstart, ncell + 1, bsum, st, cursor);
   if (rc) return rc;
-  cudaMemcpyAsync(cursor, cstart, sizeof(int) * (size_t)(ncell + 1), cudaMemcpyDeviceToDevice, st);
   if (n > 0) k_fill<<<nblk(n), kT, 0, st>>>(key, n, cursor, order);
-  if (ordered_runs) k_sort_runs<<<nblk(ncell), kT, 0, st>>>(cstart, ncell, order);
+  if (ordered_runs) {
+    k_sort_runs<<<nblk(ncell), kT, 0, st>>>(cstart, ncell, order);
+    // (no cell of a set of 48 particles holds a long run)
+    if (n > kRunLane) k_sort_long<<<nblk(ncell * 32), kT, 0, st>>>(cstart, ncell, order);
+  }
   return dustb_host::launch_status("csr_build");
 }
 

@@ -6,8 +6,9 @@
 namespace dustb {
 // scratch bytes of csr_from_keys for ncell cells and n particles
 long long csr_scratch_bytes(long long ncell, long long n);
-// in-place exclusive scan of n ints (bsum: (n + 4095)/4096 + 1 ints of scratch)
-int exclusive_scan(int *a, long long n, int *bsum, cudaStream_t st);
+// in-place exclusive scan of n ints (bsum: (n + 4095)/4096 + 1 ints of scratch), with a second
+// copy of the result in copy unless that is null
+int exclusive_scan(int *a, long long n, int *bsum, cudaStream_t st, int *copy = nullptr);
 // order/cstart from per-particle keys with explicit scratch (cursor: ncell + 1 ints, bsum:
 // scan_bsum_ints(ncell + 1) ints); ordered_runs: order every cell's run by particle index
 int csr_build(const int *key, int n, long long ncell, int *cstart, int *order, int *cursor,
