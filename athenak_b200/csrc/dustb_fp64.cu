@@ -157,17 +157,123 @@ __global__ void k_gas_rk(Ind d, double *u0, const double *u1, int nv, double g0,
   }
 }
 
-// (f2: a second 3-variable rate field added after dmom, in the same pass; null: none)
-__global__ void k_history(Ind d, double *u0, int nv, const double *dmom, const double *f2,
-                          double atw_dt) {
+__global__ void k_history(Ind d, double *u0, int nv, const double *dmom, double atw_dt) {
   int m, k, j, i;
   if (!active_cell(d, blockIdx.x * (long long)blockDim.x + threadIdx.x, m, k, j, i)) return;
   for (int v = 0; v < 3; ++v) {
     const long long a = d.at(m, nv, 1 + v, k, j, i), b = d.at(m, 3, v, k, j, i);
-    double u = u0[a] + atw_dt * dmom[b];
-    if (f2) u = u + atw_dt * f2[b];
-    u0[a] = u;
+    u0[a] = u0[a] + atw_dt * dmom[b];
   }
+}
+
+// ---- the cell work of a mixed imex stage, fused -------------------------------------------
+// The stage's start over the padded cells: the register copy u1 <- u0 (copy), the zero-flux RK
+// combination of the active cells, the history terms (dmom, f2; null: none), and the deposit
+// field zeroed (qdep, 5 variables; null: left alone).  The operations of k_gas_rk and k_history
+// in their order, in one pass over the gas instead of four.
+__global__ void k_stage_start(Ind d, double *u0, double *u1, int nv, int copy, double g0,
+                              double g1, const double *dmom, const double *f2, double atw_dt,
+                              double *qdep) {
+  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long per = d.cells();
+  if (idx >= per * d.nmb) return;
+  int m;
+  long long c;
+  block_cell(idx, per, per * d.nmb, m, c);
+  const unsigned n12 = (unsigned)(d.n1 * d.n2);
+  const int k = (int)((unsigned)c / n12), r = (int)((unsigned)c - (unsigned)k * n12);
+  const int j = r / d.n1, i = r - j * d.n1;
+  const bool act = i >= d.is && i <= d.ie && j >= d.js && j <= d.je && k >= d.ks && k <= d.ke;
+  for (int v = 0; v < nv; ++v) {
+    const long long a = ((long long)m * nv + v) * per + c;
+    double u = 0.0, w = 0.0;
+    if (copy || act) u = u0[a];
+    if (copy) { w = u; u1[a] = w; } else if (act) { w = u1[a]; }
+    if (act) {
+      u = g0 * u + g1 * w;
+      if (v >= 1 && v <= 3) {
+        const long long b = ((long long)m * 3 + (v - 1)) * per + c;
+        if (dmom) u = u + atw_dt * dmom[b];
+        if (f2) u = u + atw_dt * f2[b];
+      }
+      u0[a] = u;
+    }
+  }
+  if (qdep) {
+#pragma unroll
+    for (int v = 0; v < 5; ++v) qdep[((long long)m * 5 + v) * per + c] = 0.0;
+  }
+}
+
+// the gather window of a 3-D mesh without physical faces (dustb_mixed.cu): float4 cells, a layer
+// around every block
+struct WinView { float4 *w; const int *nghbr; int gids, W1, W2, W3; };
+
+// u* of active cell (k, j, i) of block m into the window: its own cell and, next to a face, the
+// layer of the blocks across it (a neighbour table holds each pair of blocks both ways)
+__device__ __forceinline__ void window_put(const Ind &d, const WinView &W, int m, int k, int j,
+                                           int i, float4 v) {
+  const int kc = k - d.ks, jc = j - d.js, ic = i - d.is;
+  W.w[(((long long)m * W.W3 + kc + 1) * W.W2 + jc + 1) * W.W1 + ic + 1] = v;
+  const int a1 = (ic == 0) ? -1 : ((ic == d.nx1 - 1) ? 1 : 0);
+  const int a2 = (jc == 0) ? -1 : ((jc == d.nx2 - 1) ? 1 : 0);
+  const int a3 = (kc == 0) ? -1 : ((kc == d.nx3 - 1) ? 1 : 0);
+  if ((a1 | a2 | a3) == 0) return;
+  const int *nb = W.nghbr + (long long)m * 27;
+#pragma unroll
+  for (int t = 1; t < 8; ++t) {
+    const int o1 = (t & 1) ? a1 : 0, o2 = (t & 2) ? a2 : 0, o3 = (t & 4) ? a3 : 0;
+    if (((t & 1) && !a1) || ((t & 2) && !a2) || ((t & 4) && !a3)) continue;
+    const int s = nb[dir_slot(o1, o2, o3)] - W.gids;
+    if (s < 0 || s >= d.nmb) continue;
+    W.w[(((long long)s * W.W3 + kc + 1 - o3 * d.nx3) * W.W2 + jc + 1 - o2 * d.nx2) * W.W1 + ic + 1 -
+        o1 * d.nx1] = v;
+  }
+}
+
+// k_solve_ustar, the gather window of the result (W.w null: none) and the next deposits' fields
+// zeroed (z0, z1: 3 variables each, or null); flag: an int set to 0 (or null)
+__global__ void k_solve_stage(Ind d, const double *u0, int nv, const double *qdep, double *us,
+                              int br, WinView W, double *z0, double *z1, int *flag) {
+  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (idx == 0 && flag) *flag = 0;
+  int m, k, j, i;
+  if (!active_cell(d, idx, m, k, j, i)) return;
+  const double q0 = br ? qdep[d.at(m, 5, 0, k, j, i)] : 0.0;
+  const double denom = 1.0 / (u0[d.at(m, nv, 0, k, j, i)] + q0);
+  double x[3];
+#pragma unroll
+  for (int v = 0; v < 3; ++v) {
+    const double qv = br ? qdep[d.at(m, 5, 1 + v, k, j, i)] : 0.0;
+    const long long a = d.at(m, 3, v, k, j, i);
+    x[v] = (u0[d.at(m, nv, 1 + v, k, j, i)] + qv) * denom;
+    us[a] = x[v];
+    if (z0) z0[a] = 0.0;
+    if (z1) z1[a] = 0.0;
+  }
+  if (W.w) window_put(d, W, m, k, j, i, make_float4((float)x[0], (float)x[1], (float)x[2], 0.0f));
+}
+
+// k_dc_correct with the window of the corrected field; the operator's result zeroed behind the
+// read (the next sweep's, or the ledger's, field) and z0 too (3 variables, or null)
+__global__ void k_correct_stage(Ind d, const double *u0, int nv, const double *qdep,
+                                double *result, double *field, WinView W, double *z0) {
+  int m, k, j, i;
+  if (!active_cell(d, blockIdx.x * (long long)blockDim.x + threadIdx.x, m, k, j, i)) return;
+  const double rho = u0[d.at(m, nv, 0, k, j, i)];
+  const double pinv = 1.0 / (rho + qdep[d.at(m, 5, 0, k, j, i)]);
+  double x[3];
+#pragma unroll
+  for (int v = 0; v < 3; ++v) {
+    const long long a = d.at(m, 3, v, k, j, i);
+    const double av = result[a] + rho * field[a];
+    const double rv = u0[d.at(m, nv, 1 + v, k, j, i)] + qdep[d.at(m, 5, 1 + v, k, j, i)] - av;
+    x[v] = field[a] + pinv * rv;
+    field[a] = x[v];
+    result[a] = 0.0;
+    if (z0) z0[a] = 0.0;
+  }
+  if (W.w) window_put(d, W, m, k, j, i, make_float4((float)x[0], (float)x[1], (float)x[2], 0.0f));
 }
 
 // ---- ExplicitPush imex, src/dust/dust_push.cpp:262-297 ----------------------------------
@@ -368,11 +474,14 @@ __device__ double shear_add_sum(const SBox &B, const Ind &d, const double *a, in
         seen[db + 1] = sb2;
         const int S = B.block(sface, sb3, sb2);
         if (S < 0) continue;
-        for (long long Yc = F - 1; Yc <= F + 1; ++Yc)
-          for (int q = -2; q <= 2; ++q) {
-            const long long Y = Yc + q * N2;
-            const long long sj = Y - (long long)sb2 * B.nx2 + d.js;
-            if (sj < 0 || sj >= d.n2) continue;
+        for (int e = -1; e <= 1; ++e) {
+          // the rows of the block (ghost rows included) that are row F + e or an image of it
+          const long long t = F + e - (long long)sb2 * B.nx2 + d.js;
+          int q = -(int)floor((double)t / (double)N2);
+          long long sj = t + q * N2;                 // (0 <= sj < N2)
+          for (; sj < d.n2; sj += N2, ++q) {
+            if (q < -2 || q > 2) continue;
+            const long long Y = F + e + q * N2;
             const double ya = (double)Y + sh, yb = (double)(Y + 1) + sh;
             // the one image of this row that the interval can overlap: the nearest (the rows
             // are a cell wide and their images N2 >= 2 cells apart)
@@ -382,6 +491,7 @@ __device__ double shear_add_sum(const SBox &B, const Ind &d, const double *a, in
             const double o = fmin(yb, chi) - fmax(ya, clo);
             if (o > 0.0) sum += o * a[d.at(S, nvar, v, sk, (int)sj, si)];
           }
+        }
       }
     }
   }
@@ -691,65 +801,103 @@ __device__ __forceinline__ void shell_cell(const Ind &d, const Shell &h, int t, 
   i = u < d.ng ? u : u + h.xin;
 }
 
-// fold: fold the ghost deposits beyond physical x3 faces back into the mirrored active cells.
-// Grid: x over the shell cells of a block, y over blocks and variables.  The directions are
-// unrolled, so that each one's test is a combination of six flags of the cell (looped over the
-// table in constant memory with 64-bit index divisions, an exchange of 64^3 cells and five
-// variables took 28 us against 8)
-__global__ void __launch_bounds__(kThreads)
-k_ghost_add(Ind d, const int *nghbr, int gids, double *a, int nvar, int fold, SBox B, Shell sh) {
-  constexpr signed char kDir[26][3] = {
+// the directions (indices of kDirOrder) with component o along axis a
+constexpr unsigned dir_mask(int a, int o) {
+  constexpr signed char t[26][3] = {
       {-1, 0, 0}, {1, 0, 0}, {0, -1, 0}, {0, 1, 0},
       {-1, -1, 0}, {1, -1, 0}, {-1, 1, 0}, {1, 1, 0},
       {0, 0, -1}, {0, 0, 1},
       {-1, 0, -1}, {1, 0, -1}, {-1, 0, 1}, {1, 0, 1},
       {0, -1, -1}, {0, 1, -1}, {0, -1, 1}, {0, 1, 1},
       {-1, -1, -1}, {1, -1, -1}, {-1, 1, -1}, {1, 1, -1},
-      {-1, -1, 1}, {1, -1, 1}, {-1, 1, 1}, {1, 1, 1}};     // kDirOrder
+      {-1, -1, 1}, {1, -1, 1}, {-1, 1, 1}, {1, 1, 1}};       // kDirOrder
+  unsigned m = 0;
+  for (int n = 0; n < 26; ++n)
+    if (t[n][a] == o) m |= 1u << n;
+  return m;
+}
+
+constexpr unsigned kXlo = dir_mask(0, -1), kXhi = dir_mask(0, 1), kYlo = dir_mask(1, -1);
+constexpr unsigned kYhi = dir_mask(1, 1), kZlo = dir_mask(2, -1), kZhi = dir_mask(2, 1);
+
+// fold: fold the ghost deposits beyond physical x3 faces back into the mirrored active cells.
+// Grid: x over the shell cells of a block, y over the blocks; a thread takes NV variables of
+// its cell at a time.  The directions whose ghost cells reach the cell are the bits of a mask
+// (one for most cells), taken in NeighborIndex order; each one's neighbour is looked up once
+// for all variables.  (A thread per cell and variable that tested all 26 directions took 600
+// instructions: 88 us for 5 variables of eight blocks of 64^3.)
+template <int NV>
+__device__ __forceinline__ void ghost_add_cell(const Ind &d, const int *nb, int gids, double *a,
+                                               int nvar, int v0, int m, int k, int j, int i,
+                                               unsigned dirs, unsigned fold_lo, unsigned fold_hi) {
+  const long long vs = d.cells();
+  double *at = a + d.at(m, nvar, v0, k, j, i);
+  double val[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) val[v] = at[v * vs];
+  auto take = [&](int src, int kk, int jj, int ii) {
+    const double *f = a + d.at(src, nvar, v0, kk, jj, ii);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) val[v] += f[v * vs];
+  };
+  for (unsigned r = dirs; r; r &= r - 1) {
+    const int n = __ffs(r) - 1;
+    const int o1 = kDirOrder[n][0], o2 = kDirOrder[n][1], o3 = kDirOrder[n][2];
+    const int src = nb[dir_slot(o1, o2, o3)] - gids;
+    if (src >= 0 && src < d.nmb) take(src, k - o3 * d.nx3, j - o2 * d.nx2, i - o1 * d.nx1);
+  }
+  // a physical x3 face (no neighbour across it): the ghost plane ks-1-t (ke+1+t) folds into the
+  // active plane ks+t (ke-t); the block's own column (bit 31), then its x1/x2 neighbours' ghost
+  // strips that face this cell, in NeighborIndex order
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    const unsigned f = side ? fold_hi : fold_lo;
+    if (!f) continue;
+    const int kg = side ? 2 * d.ke + 1 - k : 2 * d.ks - 1 - k;
+    take(m, kg, j, i);
+    for (unsigned r = f & 0x7fffffffu; r; r &= r - 1) {
+      const int n = __ffs(r) - 1;
+      const int o1 = kDirOrder[n][0], o2 = kDirOrder[n][1];
+      const int src = nb[dir_slot(o1, o2, 0)] - gids;
+      if (src >= 0 && src < d.nmb) take(src, kg, j - o2 * d.nx2, i - o1 * d.nx1);
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < NV; ++v) at[v * vs] = val[v];
+}
+
+__global__ void __launch_bounds__(kThreads)
+k_ghost_add(Ind d, const int *nghbr, int gids, double *a, int nvar, int fold, SBox B, Shell sh) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= sh.per) return;
   int k, j, i;
   shell_cell(d, sh, t, k, j, i);
   k += d.ks; j += d.js; i += d.is;
   const int ng1 = d.ng - 1;
-  const bool near[3][3] = {{i <= d.is + ng1, true, i >= d.ie - ng1},
-                           {j <= d.js + ng1, true, j >= d.je - ng1},
-                           {k <= d.ks + ng1, true, k >= d.ke - ng1}};
-  for (int mv = blockIdx.y; mv < d.nmb * nvar; mv += gridDim.y) {
-    const int m = mv / nvar, v = mv - m * nvar;
+  unsigned dirs = d.three_d ? 0x3ffffffu : 0xffu;
+  if (i > d.is + ng1) dirs &= ~kXlo;
+  if (i < d.ie - ng1) dirs &= ~kXhi;
+  if (j > d.js + ng1) dirs &= ~kYlo;
+  if (j < d.je - ng1) dirs &= ~kYhi;
+  const unsigned flat = dirs & 0xffu;              // (the directions within the plane)
+  if (k > d.ks + ng1) dirs &= ~kZlo;
+  if (k < d.ke - ng1) dirs &= ~kZhi;
+  for (int m = blockIdx.y; m < d.nmb; m += gridDim.y) {
     const int *nb = nghbr + (long long)m * 27;
-    const long long at = d.at(m, nvar, v, k, j, i);
-    double val = a[at];
-    const bool cm = B.crossing(m, -1), cp = B.crossing(m, 1);
-#pragma unroll
-    for (int n = 0; n < 26; ++n) {
-      const int o1 = kDir[n][0], o2 = kDir[n][1], o3 = kDir[n][2];
-      if ((o3 != 0 && !d.three_d) || (o2 != 0 && !d.multi_d)) continue;
-      if (!(near[0][o1 + 1] && near[1][o2 + 1] && near[2][o3 + 1])) continue;
-      const int src = nb[dir_slot(o1, o2, o3)] - gids;
-      if (src < 0 || src >= d.nmb || (o1 < 0 && cm) || (o1 > 0 && cp)) continue;
-      val += a[d.at(src, nvar, v, k - o3 * d.nx3, j - o2 * d.nx2, i - o1 * d.nx1)];
+    unsigned off = 0;                              // (shear faces are remapped, not exchanged)
+    if (B.on) {
+      if (B.crossing(m, -1)) off |= kXlo;
+      if (B.crossing(m, 1)) off |= kXhi;
     }
+    unsigned lo = 0, hi = 0;
     if (fold && d.three_d) {
-      // a physical x3 face (no neighbour across it): the ghost plane ks-1-t (ke+1+t) folds into
-      // the active plane ks+t (ke-t); the block's own column, then its x1/x2 neighbours'
-      // ghost strips that face this cell, in NeighborIndex order
-      for (int side = 0; side < 2; ++side) {
-        if (!near[2][side ? 2 : 0]) continue;
-        if (nb[dir_slot(0, 0, side ? 1 : -1)] >= 0) continue;
-        const int kg = side ? 2 * d.ke + 1 - k : 2 * d.ks - 1 - k;
-        val += a[d.at(m, nvar, v, kg, j, i)];
-#pragma unroll
-        for (int n = 0; n < 8; ++n) {
-          const int o1 = kDir[n][0], o2 = kDir[n][1];
-          if (!(near[0][o1 + 1] && near[1][o2 + 1])) continue;
-          const int src = nb[dir_slot(o1, o2, 0)] - gids;
-          if (src < 0 || src >= d.nmb || (o1 < 0 && cm) || (o1 > 0 && cp)) continue;
-          val += a[d.at(src, nvar, v, kg, j - o2 * d.nx2, i - o1 * d.nx1)];
-        }
-      }
+      if (k <= d.ks + ng1 && nb[dir_slot(0, 0, -1)] < 0) lo = 0x80000000u | (flat & ~off);
+      if (k >= d.ke - ng1 && nb[dir_slot(0, 0, 1)] < 0) hi = 0x80000000u | (flat & ~off);
     }
-    a[at] = val;
+    int v = 0;
+    for (; v + 5 <= nvar; v += 5) ghost_add_cell<5>(d, nb, gids, a, nvar, v, m, k, j, i, dirs & ~off, lo, hi);
+    for (; v + 3 <= nvar; v += 3) ghost_add_cell<3>(d, nb, gids, a, nvar, v, m, k, j, i, dirs & ~off, lo, hi);
+    for (; v < nvar; ++v) ghost_add_cell<1>(d, nb, gids, a, nvar, v, m, k, j, i, dirs & ~off, lo, hi);
   }
 }
 
@@ -3035,18 +3183,6 @@ void gas_rk(const dustb_ctx *c, double g0, double g1, cudaStream_t st) {
   Ind d = make_ind(c->mesh);
   k_gas_rk<<<blocks_for(n_active(d)), kThreads, 0, st>>>(d, c->f.u0, c->f.u1, c->f.nvar_gas, g0, g1);
 }
-void history(const dustb_ctx *c, double atw_dt, cudaStream_t st) {
-  Ind d = make_ind(c->mesh);
-  k_history<<<blocks_for(n_active(d)), kThreads, 0, st>>>(d, c->f.u0, c->f.nvar_gas, c->f.dmom,
-                                                          nullptr, atw_dt);
-}
-// u0.m += atw_dt dmom, then u0.m += atw_dt f for a 3-variable field f (the mixed form's rate
-// ledger), in one pass: the same sums as two history launches
-void history_field(const dustb_ctx *c, const double *f, double atw_dt, cudaStream_t st) {
-  Ind d = make_ind(c->mesh);
-  k_history<<<blocks_for(n_active(d)), kThreads, 0, st>>>(d, c->f.u0, c->f.nvar_gas, c->f.dmom, f,
-                                                          atw_dt);
-}
 void dc_correct(const dustb_ctx *c, cudaStream_t st) {
   Ind d = make_ind(c->mesh);
   k_dc_correct<<<blocks_for(n_active(d)), kThreads, 0, st>>>(d, c->f.u0, c->f.nvar_gas, c->f.qdep,
@@ -3062,6 +3198,28 @@ void pmbr(const dustb_ctx *c, double a_dt, cudaStream_t st) {
   k_pmbr<<<blocks_for(n_active(d)), kThreads, 0, st>>>(d, c->f.u0, c->f.nvar_gas, c->f.dmom, 1.0 / a_dt);
 }
 bool ctx_valid(const dustb_ctx *c) { return ctx_cells_ok(c); }
+static WinView win_view(const dustb_ctx *c, const Ind &d, void *win) {
+  return WinView{(float4 *)win, c->mesh.nghbr, c->mesh.gids, d.nx1 + 2, d.nx2 + 2, d.nx3 + 2};
+}
+void stage_start(const dustb_ctx *c, int copy, double g0, double g1, const double *dmom,
+                 const double *f2, double atw_dt, bool zero_qdep, cudaStream_t st) {
+  Ind d = make_ind(c->mesh);
+  k_stage_start<<<blocks_for(n_all(d)), kThreads, 0, st>>>(
+      d, c->f.u0, c->f.u1, c->f.nvar_gas, copy, g0, g1, dmom, f2, atw_dt,
+      zero_qdep ? c->f.qdep : nullptr);
+}
+void solve_stage(const dustb_ctx *c, void *win, double *z0, double *z1, int *flag,
+                 cudaStream_t st) {
+  Ind d = make_ind(c->mesh);
+  k_solve_stage<<<blocks_for(n_active(d)), kThreads, 0, st>>>(
+      d, c->f.u0, c->f.nvar_gas, c->f.qdep, c->f.ustar, c->phys.back_reaction,
+      win_view(c, d, win), z0, z1, flag);
+}
+void correct_stage(const dustb_ctx *c, void *win, double *z0, cudaStream_t st) {
+  Ind d = make_ind(c->mesh);
+  k_correct_stage<<<blocks_for(n_active(d)), kThreads, 0, st>>>(
+      d, c->f.u0, c->f.nvar_gas, c->f.qdep, c->f.work, c->f.ustar, win_view(c, d, win), z0);
+}
 }  // namespace dustb_cells
 
 #define CHECK_CTX(c) do { if (!ctx_ok(c)) { return DUSTB_EINVAL; } } while (0)
@@ -3096,7 +3254,7 @@ int dustb_gas_rk_noflux(const dustb_ctx *c, double gam0, double gam1, void *stre
 int dustb_history_gas(const dustb_ctx *c, double atw_dt, void *stream) {
   CHECK_CELLS(c);
   Ind d = make_ind(c->mesh);
-  k_history<<<blocks_for(n_active(d)), kThreads, 0, S(stream)>>>(d, c->f.u0, c->f.nvar_gas, c->f.dmom, nullptr, atw_dt);
+  k_history<<<blocks_for(n_active(d)), kThreads, 0, S(stream)>>>(d, c->f.u0, c->f.nvar_gas, c->f.dmom, atw_dt);
   return launch_status("history_gas");
 }
 
@@ -3140,8 +3298,7 @@ int dustb_ghost_add(const dustb_ctx *c, double *field, int nvar, void *stream) {
   const int fold = d.three_d && c->mesh.x3bc != DUSTB_X3_PERIODIC && !c->phys.x3_deposit_drop;
   const SBox B = sbview(c);
   const Shell sh = make_shell(d);
-  const long long nmv = (long long)d.nmb * nvar;
-  k_ghost_add<<<dim3(blocks_for(sh.per), (unsigned)(nmv < 65535 ? nmv : 65535)), kThreads, 0, S(stream)>>>(
+  k_ghost_add<<<dim3(blocks_for(sh.per), (unsigned)(d.nmb < 65535 ? d.nmb : 65535)), kThreads, 0, S(stream)>>>(
       d, c->mesh.nghbr, c->mesh.gids, field, nvar, fold, B, sh);
   if (B.on) {
     if (!B.sb_gid || B.nb2 <= 0 || B.nb3 <= 0) return DUSTB_EINVAL;

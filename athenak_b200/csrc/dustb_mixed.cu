@@ -43,8 +43,11 @@
 
 namespace dustb_cells {
 void gas_rk(const dustb_ctx *c, double g0, double g1, cudaStream_t st);
-void history(const dustb_ctx *c, double atw_dt, cudaStream_t st);
-void history_field(const dustb_ctx *c, const double *f, double atw_dt, cudaStream_t st);
+void stage_start(const dustb_ctx *c, int copy, double g0, double g1, const double *dmom,
+                 const double *f2, double atw_dt, bool zero_qdep, cudaStream_t st);
+void solve_stage(const dustb_ctx *c, void *win, double *z0, double *z1, int *flag,
+                 cudaStream_t st);
+void correct_stage(const dustb_ctx *c, void *win, double *z0, cudaStream_t st);
 void dc_correct(const dustb_ctx *c, cudaStream_t st);
 void consistent_gas(const dustb_ctx *c, double a_dt, cudaStream_t st);
 void pmbr(const dustb_ctx *c, double a_dt, cudaStream_t st);
@@ -819,7 +822,7 @@ __device__ __forceinline__ int advance(const Geo &G, const PushArgs &P, int &m, 
 // SP: 0 a periodic single-level mesh, 1 physical x3 or shear-periodic x1 faces, 2 a refined
 // (periodic) mesh
 template <int KIND, int SP>
-__global__ void __launch_bounds__(kT) k_count(PBuf S, int *key_out, int *count,
+__global__ void __launch_bounds__(kT, SP == 2 ? 5 : 8) k_count(PBuf S, int *key_out, int *count,
                                               const __grid_constant__ Geo G, int n,
                                               const __grid_constant__ PushArgs P) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -974,8 +977,10 @@ __device__ __forceinline__ void move_particle(const PBuf &S, const PBuf &D, cons
   D.f[F_TS][q] = ts; D.f[F_M][q] = mass; D.f[F_CC][q] = cc;
 }
 
+// (held to 64 registers, four CTAs per SM: the level carry of SP 2, which few particles take, had
+// it at 87, two CTAs and 24 % of the DRAM rate; 5.0 M particles 0.29 -> 0.21 ms)
 template <int KIND, int SP>
-__global__ void __launch_bounds__(kT) k_move(PBuf S, PBuf D, const int *key_in, int *cursor,
+__global__ void __launch_bounds__(kT, 4) k_move(PBuf S, PBuf D, const int *key_in, int *cursor,
                                              const __grid_constant__ Geo G, int n,
                                              const __grid_constant__ PushArgs P) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1852,27 +1857,41 @@ __global__ void __maxnreg__(168) k_tile(PBuf S, Geo G, TileArgs T,
 // heaviest first (buckets of equal log2 count, in descending order; a tile's place inside its
 // bucket does not matter), so that the persistent tile launches start the long tiles first
 // and finish on short ones.  One CTA; also clears the stage's queue counters.
-__global__ void __launch_bounds__(1024) k_tile_order(const int *cstart, Geo G, int tj, int tpp,
-                                                     int ntiles, int *order, int *qhead) {
+// (tile t is cells t nct .. (t + 1) nct - 1 of the sort.  The tiles of a uniform mesh all fall
+// into one bucket: lanes with the same bucket add once, or the counter's address serialises
+// them -- 16384 tiles 43 us)
+__global__ void __launch_bounds__(1024) k_tile_order(const int *cstart, int nct, int ntiles,
+                                                     int *order, int *qhead) {
   __shared__ int hist[33], base[33];
-  const int nct = tj * G.nx1, per_block = G.nx3 * tpp;
   auto bucket = [&](int t) {
-    const int m = t / per_block, r = t - m * per_block, k = r / tpp, j0 = (r - k * tpp) * tj;
-    const int c0 = encode(G, m, k, j0, 0);
-    const int cost = cstart[c0 + nct] - cstart[c0];
-    return cost > 0 ? __clz(cost) : 32;           // 32 - log2 size: heavy tiles first
+    if (t >= ntiles) return 33;                    // (no tile)
+    const int cost = cstart[(long long)(t + 1) * nct] - cstart[(long long)t * nct];
+    return cost > 0 ? __clz(cost) : 32;            // 32 - log2 size: heavy tiles first
   };
-  for (int b = threadIdx.x; b < 33; b += blockDim.x) hist[b] = 0;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 33) hist[threadIdx.x] = 0;
   if (threadIdx.x < kQueues) qhead[threadIdx.x] = 0;
   __syncthreads();
-  for (int t = threadIdx.x; t < ntiles; t += blockDim.x) atomicAdd(&hist[bucket(t)], 1);
+  for (int t0 = 0; t0 < ntiles; t0 += 1024) {
+    const int b = bucket(t0 + (int)threadIdx.x);
+    const unsigned peers = __match_any_sync(0xffffffffu, b);
+    if (b < 33 && lane == __ffs(peers) - 1) atomicAdd(&hist[b], __popc(peers));
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     int run = 0;
     for (int b = 0; b < 33; ++b) { base[b] = run; run += hist[b]; }
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < ntiles; t += blockDim.x) order[atomicAdd(&base[bucket(t)], 1)] = t;
+  for (int t0 = 0; t0 < ntiles; t0 += 1024) {
+    const int t = t0 + (int)threadIdx.x, b = bucket(t);
+    const unsigned peers = __match_any_sync(0xffffffffu, b);
+    const int lead = __ffs(peers) - 1;
+    int at = 0;
+    if (b < 33 && lane == lead) at = atomicAdd(&base[b], __popc(peers));
+    at = __shfl_sync(0xffffffffu, at, lead) + __popc(peers & ((1u << lane) - 1u));
+    if (b < 33) order[at] = t;
+  }
 }
 
 // m/rho of a gas field on every cell, ghosts included: the predictor's gather field
@@ -2183,7 +2202,7 @@ int build_queue(const MState &S, const Geo &G, const Cfg &cf, TileArgs &T, cudaS
   T.order = nullptr; T.qhead = nullptr;
   if (cf.grid) return DUSTB_OK;
   T.ntiles = G.nmb * G.nx3 * cf.tpp;
-  k_tile_order<<<1, 1024, 0, st>>>(S.cstart, G, cf.tj, cf.tpp, T.ntiles, S.tile_order, S.qhead);
+  k_tile_order<<<1, 1024, 0, st>>>(S.cstart, cf.tj * G.nx1, T.ntiles, S.tile_order, S.qhead);
   T.order = S.tile_order;
   T.qhead = S.qhead;
   return dustb_host::launch_status("mixed tile queue");
@@ -2254,9 +2273,8 @@ int sort_into(const MState &S, const PBuf &src, const PBuf &dst, const dustb_mes
   const long long ncell = ncell_of(ms);
   cudaMemsetAsync(S.cstart, 0, 4 * (size_t)nbins(ncell), st);
   if (n > 0) k_hist<<<nblk(n), kT, 0, st>>>(src.cell, n, S.cstart);
-  int rc = exclusive_scan(S.cstart, nbins(ncell), S.bsum, st);
+  int rc = exclusive_scan(S.cstart, nbins(ncell), S.bsum, st, S.cursor);
   if (rc) return rc;
-  cudaMemcpyAsync(S.cursor, S.cstart, 4 * (size_t)nbins(ncell), cudaMemcpyDeviceToDevice, st);
   if (n > 0) k_sortmove<<<nblk(n), kT, 0, st>>>(src, dst, n, S.cursor);
   return dustb_host::launch_status("mixed sort");
 }
@@ -2345,8 +2363,7 @@ int push_sort(const MState &S, const PBuf &src, const PBuf &dst, const Geo &G, i
   }
   {
     Scope sc(DUSTB_K_FILL, st);
-    if ((rc = exclusive_scan(S.cstart, nbins(ncell), S.bsum, st))) return rc;
-    cudaMemcpyAsync(S.cursor, S.cstart, 4 * (size_t)nbins(ncell), cudaMemcpyDeviceToDevice, st);
+    if ((rc = exclusive_scan(S.cstart, nbins(ncell), S.bsum, st, S.cursor))) return rc;
   }
   Scope sc(DUSTB_K_MOVE, st);
   if (n > 0) {
@@ -2391,12 +2408,14 @@ int dustb_mixed_import(const dustb_ctx *c, const dustb_mixed_params *mp, void *w
   const int n = c->part.npart;
   const long long ncell = ncell_of(c->mesh);
   cudaMemsetAsync(S.head, 0, sizeof(MHead), st);   // the rows carry every kick so far
+  // (the layer cells of the gather window that no block owns stay zero: the cycle's cell kernels
+  // write the window from the active cells)
+  if (nwin(c->mesh) > 0) cudaMemsetAsync(S.win, 0, 16 * (size_t)nwin(c->mesh), st);
   cudaMemsetAsync(S.cstart, 0, 4 * (size_t)nbins(ncell), st);
   if (n > 0)
     k_import<<<nblk(n), kT, 0, st>>>(c->part.pr, c->part.pi, c->part.stride, n, S.B, S.cstart, G, c->err);
-  int rc = exclusive_scan(S.cstart, nbins(ncell), S.bsum, st);
+  int rc = exclusive_scan(S.cstart, nbins(ncell), S.bsum, st, S.cursor);
   if (rc) return rc;
-  cudaMemcpyAsync(S.cursor, S.cstart, 4 * (size_t)nbins(ncell), cudaMemcpyDeviceToDevice, st);
   if (n > 0) k_sortmove<<<nblk(n), kT, 0, st>>>(S.B, S.A, n, S.cursor);
   return dustb_host::launch_status("mixed_import");
 }
@@ -2550,16 +2569,13 @@ int dustb_mixed_imex_cycle(const dustb_ctx *c, const dustb_mixed_params *mp, voi
     const PBuf &cur = (stage == 1) ? S.B : S.A;
     {
       Scope sc(DUSTB_K_CELLS, st);
-      if (stage == 1) cudaMemcpyAsync(c->f.u1, c->f.u0, fbytes * c->f.nvar_gas, cudaMemcpyDeviceToDevice, st);
-      dustb_cells::gas_rk(c, gam0[stage - 1], gam1[stage - 1], st);
-      if (stage == 2 && br) {
-        // with the ledger, the rate's FP32 rounding the stage-1 kick tiles recorded follows the
-        // gas rate in the same pass
-        if (!(mp->variant & DUSTB_MIXED_NO_LEDGER))
-          dustb_cells::history_field(c, c->f.work, atw22 * dt, st);
-        else
-          dustb_cells::history(c, atw22 * dt, st);
-      }
+      // with the ledger, the rate's FP32 rounding the stage-1 kick tiles recorded follows the gas
+      // rate of the history term
+      const bool hist = stage == 2 && br;
+      dustb_cells::stage_start(c, stage == 1, gam0[stage - 1], gam1[stage - 1],
+                               hist ? c->f.dmom : nullptr,
+                               hist && !(mp->variant & DUSTB_MIXED_NO_LEDGER) ? c->f.work : nullptr,
+                               atw22 * dt, br != 0, st);
     }
     PushArgs P{};
     P.kind = PK_IMEX;
@@ -2590,7 +2606,6 @@ int dustb_mixed_imex_cycle(const dustb_ctx *c, const dustb_mixed_params *mp, voi
     }
     P.inv_adt = 1.0 / a_dt;
     RUN(push_sort(S, src, cur, G, n, ncell, P, st));
-    if (stage == 1) cudaMemsetAsync(&S.head->pending, 0, sizeof(int), st);   // applied
     TileArgs T{};
     T.a_dt = a_dt; T.err = c->err; T.deposit = 1; T.shy = P.shy;
     RUN(build_queue(S, G, cf, T, st));                // the stage's tiles, heaviest first
@@ -2598,7 +2613,6 @@ int dustb_mixed_imex_cycle(const dustb_ctx *c, const dustb_mixed_params *mp, voi
     if (br) {
       {
         Scope sc(DUSTB_K_DEPOSIT_QP, st);
-        cudaMemsetAsync(c->f.qdep, 0, fbytes * 5, st);
         T.dfield = c->f.qdep; T.dnvar = 5; T.res = c->f.resid;
         RUN(launch_tile<MODE_QP>(S, cur, G, cf, T, st, Q_QP));
         if (shift) RUN(launch_shift_edge<MODE_QP>(S, cur, G, T, st));
@@ -2606,17 +2620,45 @@ int dustb_mixed_imex_cycle(const dustb_ctx *c, const dustb_mixed_params *mp, voi
       Scope sc(DUSTB_K_CELLS, st);
       RUN(ghost_add_if(c, G, c->f.qdep, 5, st, mp));
     }
-    // periodic meshes: the deposits go straight into the owners' active cells and the
-    // gathers read ghost cells from their owners, so no ghost exchange is needed
-    {
-      Scope sc(DUSTB_K_CELLS, st);
-      RUN(dustb_solve_ustar(c, st));
-    }
-    if (br && c->phys.drag_solver >= DUSTB_SOLVER_DC1) {
-      const int nsw = (c->phys.drag_solver == DUSTB_SOLVER_DC2) ? 2 : 1;
+    // periodic meshes: the deposits go straight into the owners' active cells and the gathers
+    // read ghost cells from their owners, so no ghost exchange is needed; the solve and the
+    // sweeps then write the gather window themselves and zero the next deposits' fields as they
+    // pass (in ghost mode the exchanges come between).  Stage 1 has applied the pending kick
+    int *applied = stage == 1 ? &S.head->pending : nullptr;
+    const int nsw = (br && c->phys.drag_solver >= DUSTB_SOLVER_DC1)
+                        ? ((c->phys.drag_solver == DUSTB_SOLVER_DC2) ? 2 : 1) : 0;
+    // (the fields the kick adds to: dmom, and in stage 1 the ledger's rate rounding in work)
+    double *kd = br ? c->f.dmom : nullptr;
+    double *kh = (ledger && stage == 1) ? c->f.work : nullptr;
+    if (!G.ghost) {
+      void *win = G.three_d ? (void *)S.win : nullptr;
+      T.win4 = S.win;
+      {
+        Scope sc(DUSTB_K_CELLS, st);
+        dustb_cells::solve_stage(c, win, nsw ? c->f.work : kd, nsw ? nullptr : kh, applied, st);
+        RUN(dustb_host::launch_status("mixed solve"));
+      }
+      for (int w = 0; w < nsw; ++w) {
+        {
+          Scope sc(DUSTB_K_OPERATOR, st);
+          T.gfield = c->f.ustar; T.dfield = c->f.work; T.dnvar = 3;
+          RUN(launch_tile<MODE_OP>(S, cur, G, cf, T, st, Q_OP + w));
+          if (shift) RUN(launch_shift_edge<MODE_OP>(S, cur, G, T, st));
+        }
+        Scope sc(DUSTB_K_CELLS, st);
+        dustb_cells::correct_stage(c, win, w == nsw - 1 ? kd : nullptr, st);
+        RUN(dustb_host::launch_status("mixed correct"));
+      }
+    } else {
+      {
+        Scope sc(DUSTB_K_CELLS, st);
+        dustb_cells::solve_stage(c, nullptr, nullptr, nullptr, applied, st);
+        RUN(dustb_host::launch_status("mixed solve"));
+      }
       for (int w = 0; w < nsw; ++w) {
         { Scope sc(DUSTB_K_CELLS, st);
           RUN(ghost_copy_if(c, G, c->f.ustar, st, mp)); }
+        // (the block's own ghost cells take deposits: the whole field is zeroed)
         cudaMemsetAsync(c->f.work, 0, fbytes * 3, st);
         RUN(gather_window(S, G, c->mesh, c->f.ustar, T, st));
         { Scope sc(DUSTB_K_OPERATOR, st);
@@ -2627,16 +2669,14 @@ int dustb_mixed_imex_cycle(const dustb_ctx *c, const dustb_mixed_params *mp, voi
           RUN(ghost_add_if(c, G, c->f.work, 3, st, mp));
           dustb_cells::dc_correct(c, st); }
       }
+      {
+        Scope sc(DUSTB_K_CELLS, st);
+        RUN(ghost_copy_if(c, G, c->f.ustar, st, mp));
+      }
+      if (kd) cudaMemsetAsync(kd, 0, fbytes * 3, st);
+      if (kh) cudaMemsetAsync(kh, 0, fbytes * 3, st);
+      RUN(gather_window(S, G, c->mesh, c->f.ustar, T, st));
     }
-    {
-      Scope sc(DUSTB_K_CELLS, st);
-      RUN(ghost_copy_if(c, G, c->f.ustar, st, mp));
-    }
-    if (br) cudaMemsetAsync(c->f.dmom, 0, fbytes * 3, st);
-    // stage 1: the kick tiles record the rate's rounding in work for stage 2's history term
-    // (work is free from here: the operator sweeps are done)
-    if (ledger && stage == 1) cudaMemsetAsync(c->f.work, 0, fbytes * 3, st);
-    RUN(gather_window(S, G, c->mesh, c->f.ustar, T, st));
     {
       Scope sc(DUSTB_K_KICK, st);
       T.gfield = c->f.ustar; T.dfield = c->f.dmom; T.dnvar = 3; T.deposit = br;
