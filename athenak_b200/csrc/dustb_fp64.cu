@@ -2459,10 +2459,15 @@ __device__ void cloud_gather(const MCtx &M, const Ind &d, int m, const double x[
   }, err);
 }
 
-// Every cloud kernel below is a body templated on the traversal form and two kernels: _u over
-// the uniform-mesh traversal (no launch bounds: the compiler keeps it near 120 registers and 16
-// warps per SM), _l over the leaf tables of refined meshes (held to 128 registers, 2 CTAs of 256
-// threads per SM: about 15 % faster than its unbounded 230 registers, which allow one CTA).
+
+// Every cloud kernel below has a body, templated on the traversal form, for one cloud in the
+// general traversal, and three kernels: _u, a thread per cloud through the uniform-mesh
+// traversal (meshes with physical x3 faces, whose clouds have a mirrored part); _l, over the
+// leaf tables of refined meshes (held to 128 registers, 2 CTAs of 256 threads per SM: about 15 %
+// faster than its unbounded 230 registers, which allow one CTA); and _s, the slots of the next
+// section.  (The slots for the clouds inside their block on refined meshes, the others listed
+// per CTA and put through the leaf traversal at the end, ran at half the speed of _l: 41
+// against 21 ms per pass of 1.9 M clouds -- the listed clouds lose their neighbours.)
 
 // ---- the uniform traversal as three slots per direction ---------------------------------
 // On a uniform mesh without physical x3 faces a plain cloud of any level reaches at most the
@@ -2551,14 +2556,22 @@ __device__ __forceinline__ void cloud_cell(const MCtx &M, const Ind &d, CloudPos
   }
 }
 
+// the hat along direction a: the block's cell width and its reciprocal, the half-width and its
+// reciprocal
+struct AxisHat { double dx, idx, ell, inv; };
+__device__ __forceinline__ AxisHat axis_hat(const MCtx &M, const CloudPos &c, int a) {
+  AxisHat h;
+  h.dx = M.s(c.m, DX1 + a);
+  h.idx = 1.0 / h.dx;
+  h.ell = ldexp(h.dx, -c.lev);
+  h.inv = ldexp(h.idx, c.lev);
+  return h;
+}
+
 template <bool kM>
-__device__ __forceinline__ void cloud_slots(const MCtx &M, const Ind &d, const CloudPos &c, int a,
-                                            AxisSlot s[3]) {
-  const double dx = M.s(c.m, DX1 + a), idx = 1.0 / dx;
-  const double ell = ldexp(dx, -c.lev), inv = ldexp(idx, c.lev);
-#pragma unroll
-  for (int t = 0; t < 3; ++t)
-    s[t] = axis_slot<kM>(M, d, c.m, a, c.ic[a] + t - 1, c.x[a], dx, idx, ell, inv, c.L[a]);
+__device__ __forceinline__ AxisSlot slot_of(const MCtx &M, const Ind &d, const CloudPos &c, int a,
+                                            int t, const AxisHat &h) {
+  return axis_slot<kM>(M, d, c.m, a, c.ic[a] + t - 1, c.x[a], h.dx, h.idx, h.ell, h.inv, c.L[a]);
 }
 
 // cloud_gather over the slots (kM), or the sum of weights times a field of nvar variables
@@ -2568,18 +2581,34 @@ __device__ __forceinline__ void slot_gather(const MCtx &M, const Ind &d, const C
                                             const double *f, int nvar, double ug[3],
                                             double wx[3], double wy[3], double wz[3],
                                             unsigned *err) {
+  // (only the leaves of a row are unrolled, and the owner of a cell beyond the block is looked up
+  // once per row and for the row's ends: with a plane of nine unrolled and a lookup per leaf
+  // the gather's warps waited for instructions most of the time, 2.6 ms for 3.1 M clouds)
   AxisSlot X[3], Y[3];
-  cloud_slots<kM>(M, d, c, 0, X);
-  cloud_slots<kM>(M, d, c, 1, Y);
-  const double dz = M.s(c.m, DX3), idz = 1.0 / dz;
-  const double ellz = ldexp(dz, -c.lev), invz = ldexp(idz, c.lev);
+  {
+    const AxisHat h = axis_hat(M, c, 0);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) X[t] = slot_of<kM>(M, d, c, 0, t, h);
+  }
+  {
+    const AxisHat h = axis_hat(M, c, 1);
+#pragma unroll 1
+    for (int t = 0; t < 3; ++t) Y[t] = slot_of<kM>(M, d, c, 1, t, h);
+  }
+  const AxisHat hz = axis_hat(M, c, 2);
+  const long long vs = d.cells();
+  const int st = kM ? 12 : 1;                      // the distance of neighbouring cells in f
+  auto cell = [&](int blk, int kk, int jj, int ii) -> const double * {
+    return kM ? f + ((((long long)blk * d.n3 + kk) * d.n2 + jj) * d.n1 + ii) * 12
+              : f + d.at(blk, nvar, 0, kk, jj, ii);
+  };
   ug[0] = ug[1] = ug[2] = 0.0;
   wz[0] = wz[2] = 0.0; wz[1] = 1.0;
 #pragma unroll 1
   for (int q = 0; q < 3; ++q) {
     AxisSlot Z;
     if (d.three_d) {
-      Z = axis_slot<kM>(M, d, c.m, 2, c.ic[2] + q - 1, c.x[2], dz, idz, ellz, invz, c.L[2]);
+      Z = slot_of<kM>(M, d, c, 2, q, hz);
       if (q == 0) wz[0] = Z.w; else if (q == 1) wz[1] = Z.w; else wz[2] = Z.w;
     } else {
       if (q != 1) continue;
@@ -2587,25 +2616,23 @@ __device__ __forceinline__ void slot_gather(const MCtx &M, const Ind &d, const C
     }
     if (Z.w == 0.0 && (!kM || Z.g == 0.0)) continue;
     const int kk = d.three_d ? d.ks + c.ic[2] + q - 1 - Z.o * d.nx3 : d.ks;
-#pragma unroll
+#pragma unroll 1
     for (int b = 0; b < 3; ++b) {
-      if (Y[b].w == 0.0 && (!kM || Y[b].g == 0.0)) continue;
-      const double w23 = Y[b].w * Z.w;
-      const int jj = d.js + c.ic[1] + b - 1 - Y[b].o * d.nx2;
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        if (X[a].w == 0.0 && (!kM || X[a].g == 0.0)) continue;
-        const double w = w23 * X[a].w;
-        if (!kM && w == 0.0) continue;
-        const int ii = d.is + c.ic[0] + a - 1 - X[a].o * d.nx1;
-        const int blk = c.inside ? c.m : cloud_owner(M, d, c.m, X[a].o, Y[b].o, Z.o);
-        if (blk < 0) { if (err) report(err, DUSTB_ERR_CLOUD); continue; }
+      const AxisSlot &S = Y[b];
+      const double w2 = S.w, g2 = S.g;
+      if (w2 == 0.0 && (!kM || g2 == 0.0)) continue;
+      const double w23 = w2 * Z.w;
+      const int jj = d.js + c.ic[1] + b - 1 - S.o * d.nx2;
+      const int rb = cloud_owner(M, d, c.m, 0, S.o, Z.o);
+      const double *row = cell(rb < 0 ? c.m : rb, kk, jj, d.is + c.ic[0] - 1);
+      const double ey = S.e, dy = S.dx, yy = S.y;
+      auto leaf = [&](const AxisSlot &x, const double *g) {
+        const double w = w23 * x.w;
         if (kM) {
-          const double *g = f + ((((long long)blk * d.n3 + kk) * d.n2 + jj) * d.n1 + ii) * 12;
-          const double cx = div_by(0.5 * (w23 * X[a].g + X[a].e * w), X[a].dx, X[a].y);
-          const double cy = div_by(0.5 * (X[a].w * Y[b].g * Z.w + Y[b].e * w), Y[b].dx, Y[b].y);
+          const double cx = div_by(0.5 * (w23 * x.g + x.e * w), x.dx, x.y);
+          const double cy = div_by(0.5 * (x.w * g2 * Z.w + ey * w), dy, yy);
           if (d.three_d) {
-            const double cz = div_by(0.5 * (X[a].w * Y[b].w * Z.g + Z.e * w), Z.dx, Z.y);
+            const double cz = div_by(0.5 * (x.w * w2 * Z.g + Z.e * w), Z.dx, Z.y);
             ug[0] += w * g[0] + cx * g[3] + cy * g[6] + cz * g[9];
             ug[1] += w * g[1] + cx * g[4] + cy * g[7] + cz * g[10];
             ug[2] += w * g[2] + cx * g[5] + cy * g[8] + cz * g[11];
@@ -2615,10 +2642,21 @@ __device__ __forceinline__ void slot_gather(const MCtx &M, const Ind &d, const C
             ug[2] += w * g[2] + cx * g[5] + cy * g[8];
           }
         } else {
-          const double *g = f + d.at(blk, nvar, 0, kk, jj, ii);
-          const long long vs = d.cells();
           ug[0] += w * g[0]; ug[1] += w * g[vs]; ug[2] += w * g[2 * vs];
         }
+      };
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        if (X[a].w == 0.0 && (!kM || X[a].g == 0.0)) continue;
+        if (!kM && w23 * X[a].w == 0.0) continue;
+        const double *g = row + a * st;
+        int blk = rb;
+        if (X[a].o != 0) {
+          blk = cloud_owner(M, d, c.m, X[a].o, S.o, Z.o);
+          if (blk >= 0) g = cell(blk, kk, jj, d.is + c.ic[0] + a - 1 - X[a].o * d.nx1);
+        }
+        if (blk < 0) { if (err) report(err, DUSTB_ERR_CLOUD); continue; }
+        leaf(X[a], g);
       }
     }
   }
@@ -2629,18 +2667,12 @@ __device__ __forceinline__ void slot_gather(const MCtx &M, const Ind &d, const C
 // the slots' weights alone
 __device__ __forceinline__ void slot_weights(const MCtx &M, const Ind &d, const CloudPos &c,
                                              double wx[3], double wy[3], double wz[3]) {
-  AxisSlot s[3];
-  cloud_slots<false>(M, d, c, 0, s);
+  const AxisHat hx = axis_hat(M, c, 0), hy = axis_hat(M, c, 1), hz = axis_hat(M, c, 2);
 #pragma unroll
-  for (int t = 0; t < 3; ++t) wx[t] = s[t].w;
-  cloud_slots<false>(M, d, c, 1, s);
-#pragma unroll
-  for (int t = 0; t < 3; ++t) wy[t] = s[t].w;
-  wz[0] = wz[2] = 0.0; wz[1] = 1.0;
-  if (d.three_d) {
-    cloud_slots<false>(M, d, c, 2, s);
-#pragma unroll
-    for (int t = 0; t < 3; ++t) wz[t] = s[t].w;
+  for (int t = 0; t < 3; ++t) {
+    wx[t] = slot_of<false>(M, d, c, 0, t, hx).w;
+    wy[t] = slot_of<false>(M, d, c, 1, t, hy).w;
+    wz[t] = d.three_d ? slot_of<false>(M, d, c, 2, t, hz).w : (t == 1 ? 1.0 : 0.0);
   }
 }
 
@@ -2723,57 +2755,10 @@ __device__ __forceinline__ bool cloud_here(const PCtx &P, const MCtx &M, const I
   return true;
 }
 
-__global__ void __launch_bounds__(32 * kDepWarps, 4)
-k_cloud_deposit_s(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh, unsigned *err, int nb) {
-  deposit_clouds<4, true>(M, P.npart, nb, d, qdep, 5, 0, err, [&](int p, CloudPos &c, Stencil &t) {
-    if (!cloud_here(P, M, d, p, sh, c, err)) return false;
-    slot_weights(M, d, c, t.wx, t.wy, t.wz);
-    const double mass_c = d.three_d ? P.r(DUSTB_IPM, p) * a_dt / (P.r(DUSTB_IPTS, p) + a_dt)
-                                    : P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt));
-    t.fac = mass_c / cloud_measure(M, d, c.m);
-    t.q[0] = P.r(DUSTB_IPVX, p); t.q[1] = P.r(DUSTB_IPVY, p); t.q[2] = P.r(DUSTB_IPVZ, p);
-    t.q[3] = 0.0;
-    return true;
-  });
-}
-
-__global__ void __launch_bounds__(32 * kDepWarps, 4)
-k_cloud_gather_kick_s(PCtx P, MCtx M, Ind d, const double *gp, double *dmom, double a_dt, double sh,
-                      int br, unsigned *err, int nb) {
-  deposit_clouds<3, false>(M, P.npart, nb, d, dmom, 3, 0, nullptr, [&](int p, CloudPos &c, Stencil &t) {
-    if (!cloud_here(P, M, d, p, sh, c, err)) return false;
-    double ug[3];
-    slot_gather<true>(M, d, c, gp, 0, ug, t.wx, t.wy, t.wz, err);
-    const double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
-    const double vx = P.r(DUSTB_IPVX, p), vy = P.r(DUSTB_IPVY, p), vz = P.r(DUSTB_IPVZ, p);
-    const double dvx = cj * (ug[0] - vx), dvy = cj * (ug[1] - vy), dvz = cj * (ug[2] - vz);
-    P.r(DUSTB_IPVX, p) = vx + dvx; P.r(DUSTB_IPVY, p) = vy + dvy; P.r(DUSTB_IPVZ, p) = vz + dvz;
-    P.r(DUSTB_IPRX, p) = dvx / a_dt; P.r(DUSTB_IPRY, p) = dvy / a_dt; P.r(DUSTB_IPRZ, p) = dvz / a_dt;
-    if (!br) return false;
-    t.fac = -P.r(DUSTB_IPM, p) / cloud_measure(M, d, c.m);
-    t.q[0] = dvx; t.q[1] = dvy; t.q[2] = dvz; t.q[3] = 0.0;
-    return true;
-  });
-}
-
-__global__ void __launch_bounds__(32 * kDepWarps, 4)
-k_cloud_operator_s(PCtx P, MCtx M, Ind d, const double *gp, double *result, double a_dt, double sh,
-                   unsigned *err, int nb) {
-  deposit_clouds<3, false>(M, P.npart, nb, d, result, 3, 0, nullptr, [&](int p, CloudPos &c, Stencil &t) {
-    if (!cloud_here(P, M, d, p, sh, c, err)) return false;
-    slot_gather<true>(M, d, c, gp, 0, t.q, t.wx, t.wy, t.wz, err);
-    t.fac = P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt)) / cloud_measure(M, d, c.m);
-    t.q[3] = 0.0;
-    return true;
-  });
-}
-
 // CloudDepositImplicitT (src/dust/dust_imex3d.cpp:61-99): Q = m c W / V, P = Q v
 template <int LF>
-__device__ __forceinline__ void k_cloud_deposit_body(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh,
+__device__ __forceinline__ void k_cloud_deposit_body(int p, const PCtx &P, const MCtx &M, const Ind &d, double *qdep, double a_dt, double sh,
                                 int x3phys, unsigned *err) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
   const double L[3] = {M.x1max - M.x1min, M.x2max - M.x2min, M.x3max - M.x3min};
   int m, lev;
   double x[3];
@@ -2790,9 +2775,15 @@ __device__ __forceinline__ void k_cloud_deposit_body(PCtx P, MCtx M, Ind d, doub
   }, err);
 }
 __global__ void k_cloud_deposit_u(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh,
-                                int x3phys, unsigned *err) { k_cloud_deposit_body<0>(P, M, d, qdep, a_dt, sh, x3phys, err); }
+                                int x3phys, unsigned *err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_deposit_body<0>(p, P, M, d, qdep, a_dt, sh, x3phys, err);
+}
 __global__ void __launch_bounds__(kThreads, 2) k_cloud_deposit_l(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh,
-                                int x3phys, unsigned *err) { k_cloud_deposit_body<1>(P, M, d, qdep, a_dt, sh, x3phys, err); }
+                                int x3phys, unsigned *err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_deposit_body<1>(p, P, M, d, qdep, a_dt, sh, x3phys, err);
+}
 
 // PackGatherField3D (src/dust/dust_cloud3d.cpp:1319-1340): the velocity and its central
 // differences, gp(m, k, j, i, 0..11), over the padded interior (the outer layer zero); 2-D
@@ -2823,10 +2814,8 @@ __global__ void k_gather_pack(Ind d, const double *v, double *gp) {
 // + cz du/dz, cx = (m1x + MinImage(x - xc) w) / (2 dx); dv = c (ubar - v), v += dv,
 // R = dv / a_dt; with back-reaction -m w dv / V into dmom over the leaves of nonzero weight
 template <int LF>
-__device__ __forceinline__ void k_cloud_gather_kick_body(PCtx P, MCtx M, Ind d, const double *gp, double *dmom,
+__device__ __forceinline__ void k_cloud_gather_kick_body(int p, const PCtx &P, const MCtx &M, const Ind &d, const double *gp, double *dmom,
                                     double a_dt, double sh, int br, int x3phys, unsigned *err) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
   const double L[3] = {M.x1max - M.x1min, M.x2max - M.x2min, M.x3max - M.x3min};
   int m, lev;
   double x[3];
@@ -2849,17 +2838,21 @@ __device__ __forceinline__ void k_cloud_gather_kick_body(PCtx P, MCtx M, Ind d, 
   }, nullptr);
 }
 __global__ void k_cloud_gather_kick_u(PCtx P, MCtx M, Ind d, const double *gp, double *dmom,
-                                    double a_dt, double sh, int br, int x3phys, unsigned *err) { k_cloud_gather_kick_body<0>(P, M, d, gp, dmom, a_dt, sh, br, x3phys, err); }
+                                    double a_dt, double sh, int br, int x3phys, unsigned *err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_gather_kick_body<0>(p, P, M, d, gp, dmom, a_dt, sh, br, x3phys, err);
+}
 __global__ void __launch_bounds__(kThreads, 2) k_cloud_gather_kick_l(PCtx P, MCtx M, Ind d, const double *gp, double *dmom,
-                                    double a_dt, double sh, int br, int x3phys, unsigned *err) { k_cloud_gather_kick_body<1>(P, M, d, gp, dmom, a_dt, sh, br, x3phys, err); }
+                                    double a_dt, double sh, int br, int x3phys, unsigned *err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_gather_kick_body<1>(p, P, M, d, gp, dmom, a_dt, sh, br, x3phys, err);
+}
 
 // CloudOperatorKernelT (src/dust/dust_cloud_imex_kernels.hpp:20-70): the clouds' m c W ubar / V
 // with ubar their linear gather of the packed field, into result (the operator of dc1 / dc2)
 template <int LF>
-__device__ __forceinline__ void k_cloud_operator_body(PCtx P, MCtx M, Ind d, const double *gp, double *result,
+__device__ __forceinline__ void k_cloud_operator_body(int p, const PCtx &P, const MCtx &M, const Ind &d, const double *gp, double *result,
                                  double a_dt, double sh, int x3phys, unsigned *err) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
   const double L[3] = {M.x1max - M.x1min, M.x2max - M.x2min, M.x3max - M.x3min};
   int m, lev;
   double x[3];
@@ -2875,9 +2868,60 @@ __device__ __forceinline__ void k_cloud_operator_body(PCtx P, MCtx M, Ind d, con
   }, nullptr);
 }
 __global__ void k_cloud_operator_u(PCtx P, MCtx M, Ind d, const double *gp, double *result,
-                                 double a_dt, double sh, int x3phys, unsigned *err) { k_cloud_operator_body<0>(P, M, d, gp, result, a_dt, sh, x3phys, err); }
+                                 double a_dt, double sh, int x3phys, unsigned *err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_operator_body<0>(p, P, M, d, gp, result, a_dt, sh, x3phys, err);
+}
 __global__ void __launch_bounds__(kThreads, 2) k_cloud_operator_l(PCtx P, MCtx M, Ind d, const double *gp, double *result,
-                                 double a_dt, double sh, int x3phys, unsigned *err) { k_cloud_operator_body<1>(P, M, d, gp, result, a_dt, sh, x3phys, err); }
+                                 double a_dt, double sh, int x3phys, unsigned *err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_operator_body<1>(p, P, M, d, gp, result, a_dt, sh, x3phys, err);
+}
+
+__global__ void __launch_bounds__(32 * kDepWarps, 4)
+k_cloud_deposit_s(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh, unsigned *err, int nb) {
+  deposit_clouds<4, true>(M, P.npart, nb, d, qdep, 5, 0, err, [&](int p, CloudPos &c, Stencil &t) {
+    if (!cloud_here(P, M, d, p, sh, c, err)) return false;
+    slot_weights(M, d, c, t.wx, t.wy, t.wz);
+    const double mass_c = d.three_d ? P.r(DUSTB_IPM, p) * a_dt / (P.r(DUSTB_IPTS, p) + a_dt)
+                                    : P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt));
+    t.fac = mass_c / cloud_measure(M, d, c.m);
+    t.q[0] = P.r(DUSTB_IPVX, p); t.q[1] = P.r(DUSTB_IPVY, p); t.q[2] = P.r(DUSTB_IPVZ, p);
+    t.q[3] = 0.0;
+    return true;
+  });
+}
+
+__global__ void __launch_bounds__(32 * kDepWarps, 3)
+k_cloud_gather_kick_s(PCtx P, MCtx M, Ind d, const double *gp, double *dmom, double a_dt, double sh,
+                      int br, unsigned *err, int nb) {
+  deposit_clouds<3, false>(M, P.npart, nb, d, dmom, 3, 0, nullptr, [&](int p, CloudPos &c, Stencil &t) {
+    if (!cloud_here(P, M, d, p, sh, c, err)) return false;
+    double ug[3];
+    slot_gather<true>(M, d, c, gp, 0, ug, t.wx, t.wy, t.wz, err);
+    const double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
+    const double vx = P.r(DUSTB_IPVX, p), vy = P.r(DUSTB_IPVY, p), vz = P.r(DUSTB_IPVZ, p);
+    const double dvx = cj * (ug[0] - vx), dvy = cj * (ug[1] - vy), dvz = cj * (ug[2] - vz);
+    P.r(DUSTB_IPVX, p) = vx + dvx; P.r(DUSTB_IPVY, p) = vy + dvy; P.r(DUSTB_IPVZ, p) = vz + dvz;
+    P.r(DUSTB_IPRX, p) = dvx / a_dt; P.r(DUSTB_IPRY, p) = dvy / a_dt; P.r(DUSTB_IPRZ, p) = dvz / a_dt;
+    if (!br) return false;
+    t.fac = -P.r(DUSTB_IPM, p) / cloud_measure(M, d, c.m);
+    t.q[0] = dvx; t.q[1] = dvy; t.q[2] = dvz; t.q[3] = 0.0;
+    return true;
+  });
+}
+
+__global__ void __launch_bounds__(32 * kDepWarps, 3)
+k_cloud_operator_s(PCtx P, MCtx M, Ind d, const double *gp, double *result, double a_dt, double sh,
+                   unsigned *err, int nb) {
+  deposit_clouds<3, false>(M, P.npart, nb, d, result, 3, 0, nullptr, [&](int p, CloudPos &c, Stencil &t) {
+    if (!cloud_here(P, M, d, p, sh, c, err)) return false;
+    slot_gather<true>(M, d, c, gp, 0, t.q, t.wx, t.wy, t.wz, err);
+    t.fac = P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt)) / cloud_measure(M, d, c.m);
+    t.q[3] = 0.0;
+    return true;
+  });
+}
 
 // CloudImplicitConsistencyOverlapT (src/dust/dust_imex3d.cpp:669-790), the cells: g = rho u* -
 // M, r = (D - g) / (rho + Q) (by the reciprocal), the gas takes g + rho r, dmom its rate, r
@@ -2903,10 +2947,8 @@ __global__ void k_cloud_consistent_gas(Ind d, double *u0, int nv, const double *
 
 // ... the clouds: v += c sum W r, R += c sum W r / a_dt with the deposit's weights
 template <int LF>
-__device__ __forceinline__ void k_cloud_consistent_dust_body(PCtx P, MCtx M, Ind d, const double *res, double a_dt,
+__device__ __forceinline__ void k_cloud_consistent_dust_body(int p, const PCtx &P, const MCtx &M, const Ind &d, const double *res, double a_dt,
                                         double sh, int x3phys) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
   if (P.r(DUSTB_IPM, p) <= 0.0) return;
   const double L[3] = {M.x1max - M.x1min, M.x2max - M.x2min, M.x3max - M.x3min};
   int m, lev;
@@ -2923,13 +2965,20 @@ __device__ __forceinline__ void k_cloud_consistent_dust_body(PCtx P, MCtx M, Ind
   P.r(DUSTB_IPRZ, p) += cj * rv[2] / a_dt;
 }
 __global__ void k_cloud_consistent_dust_u(PCtx P, MCtx M, Ind d, const double *res, double a_dt,
-                                        double sh, int x3phys) { k_cloud_consistent_dust_body<0>(P, M, d, res, a_dt, sh, x3phys); }
-__global__ void __launch_bounds__(kThreads, 2) k_cloud_consistent_dust_l(PCtx P, MCtx M, Ind d, const double *res, double a_dt,
-                                        double sh, int x3phys) { k_cloud_consistent_dust_body<1>(P, M, d, res, a_dt, sh, x3phys); }
-
-__global__ void k_cloud_consistent_dust_s(PCtx P, MCtx M, Ind d, const double *res, double a_dt,
-                                          double sh) {
+                                        double sh, int x3phys) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_consistent_dust_body<0>(p, P, M, d, res, a_dt, sh, x3phys);
+}
+__global__ void __launch_bounds__(kThreads, 2) k_cloud_consistent_dust_l(PCtx P, MCtx M, Ind d, const double *res, double a_dt,
+                                        double sh, int x3phys) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_consistent_dust_body<1>(p, P, M, d, res, a_dt, sh, x3phys);
+}
+
+__global__ void __launch_bounds__(128) k_cloud_consistent_dust_s(PCtx P, MCtx M, Ind d,
+                                                                 const double *res, double a_dt,
+                                                                 double sh) {
+  const int p = blockIdx.x * 128 + threadIdx.x;
   if (p >= P.npart) return;
   if (P.r(DUSTB_IPM, p) <= 0.0) return;
   CloudPos c;
@@ -2960,10 +3009,8 @@ __global__ void k_gas_velocity_all(Ind d, const double *u, int nv, double *uv) {
 
 // CloudPredictorT: g = -dt (m / t_s) (ubar - v) into qdep 1-3, m / t_s into qdep 4 (rate_dep)
 template <int LF>
-__device__ __forceinline__ void k_cloud_pc2_predictor_body(PCtx P, MCtx M, Ind d, const double *gp, double *qdep,
+__device__ __forceinline__ void k_cloud_pc2_predictor_body(int p, const PCtx &P, const MCtx &M, const Ind &d, const double *gp, double *qdep,
                                       double dt, int rate_dep, int x3phys, unsigned *err) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
   const double L[3] = {M.x1max - M.x1min, M.x2max - M.x2min, M.x3max - M.x3min};
   int m, lev;
   double x[3];
@@ -2983,11 +3030,17 @@ __device__ __forceinline__ void k_cloud_pc2_predictor_body(PCtx P, MCtx M, Ind d
   }, nullptr);
 }
 __global__ void k_cloud_pc2_predictor_u(PCtx P, MCtx M, Ind d, const double *gp, double *qdep,
-                                      double dt, int rate_dep, int x3phys, unsigned *err) { k_cloud_pc2_predictor_body<0>(P, M, d, gp, qdep, dt, rate_dep, x3phys, err); }
+                                      double dt, int rate_dep, int x3phys, unsigned *err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_pc2_predictor_body<0>(p, P, M, d, gp, qdep, dt, rate_dep, x3phys, err);
+}
 __global__ void __launch_bounds__(kThreads, 2) k_cloud_pc2_predictor_l(PCtx P, MCtx M, Ind d, const double *gp, double *qdep,
-                                      double dt, int rate_dep, int x3phys, unsigned *err) { k_cloud_pc2_predictor_body<1>(P, M, d, gp, qdep, dt, rate_dep, x3phys, err); }
+                                      double dt, int rate_dep, int x3phys, unsigned *err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_pc2_predictor_body<1>(p, P, M, d, gp, qdep, dt, rate_dep, x3phys, err);
+}
 
-__global__ void __launch_bounds__(32 * kDepWarps, 4)
+__global__ void __launch_bounds__(32 * kDepWarps, 3)
 k_cloud_pc2_predictor_s(PCtx P, MCtx M, Ind d, const double *gp, double *qdep, double dt,
                         int rate_dep, unsigned *err, int nb) {
   deposit_clouds<4, false>(M, P.npart, nb, d, qdep, 5, 1, nullptr, [&](int p, CloudPos &c, Stencil &t) {
@@ -3081,11 +3134,9 @@ __device__ __forceinline__ void cloud_advance(const PCtx &P, const Ind &d, int p
 }
 
 template <int LF>
-__device__ __forceinline__ void k_cloud_pc2_advance_body(PCtx P, MCtx M, Ind d, const double *gp, double *dmom,
+__device__ __forceinline__ void k_cloud_pc2_advance_body(int p, const PCtx &P, const MCtx &M, const Ind &d, const double *gp, double *dmom,
                                     double dt, int br, int sbox, int strat, double q, double om,
                                     double aphi, int x3phys, unsigned *err) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
   const double L[3] = {M.x1max - M.x1min, M.x2max - M.x2min, M.x3max - M.x3min};
   const int m = P.i(DUSTB_PGID, p) - M.gids, lev = P.i(DUSTB_PLEV, p);
   CloudHalf H;
@@ -3104,7 +3155,7 @@ __device__ __forceinline__ void k_cloud_pc2_advance_body(PCtx P, MCtx M, Ind d, 
     atomicAdd(&dmom[d.at(lf.b, 3, 2, lf.k, lf.j, lf.i)], dw * dv[2]);
   }, nullptr);
 }
-__global__ void __launch_bounds__(32 * kDepWarps, 4)
+__global__ void __launch_bounds__(32 * kDepWarps, 3)
 k_cloud_pc2_advance_s(PCtx P, MCtx M, Ind d, const double *gp, double *dmom, double dt, int br,
                       int sbox, int strat, double q, double om, double aphi, unsigned *err, int nb) {
   deposit_clouds<3, false>(M, P.npart, nb, d, dmom, 3, 0, nullptr, [&](int p, CloudPos &c, Stencil &t) {
@@ -3126,10 +3177,16 @@ k_cloud_pc2_advance_s(PCtx P, MCtx M, Ind d, const double *gp, double *dmom, dou
 }
 __global__ void k_cloud_pc2_advance_u(PCtx P, MCtx M, Ind d, const double *gp, double *dmom,
                                     double dt, int br, int sbox, int strat, double q, double om,
-                                    double aphi, int x3phys, unsigned *err) { k_cloud_pc2_advance_body<0>(P, M, d, gp, dmom, dt, br, sbox, strat, q, om, aphi, x3phys, err); }
+                                    double aphi, int x3phys, unsigned *err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_pc2_advance_body<0>(p, P, M, d, gp, dmom, dt, br, sbox, strat, q, om, aphi, x3phys, err);
+}
 __global__ void __launch_bounds__(kThreads, 2) k_cloud_pc2_advance_l(PCtx P, MCtx M, Ind d, const double *gp, double *dmom,
                                     double dt, int br, int sbox, int strat, double q, double om,
-                                    double aphi, int x3phys, unsigned *err) { k_cloud_pc2_advance_body<1>(P, M, d, gp, dmom, dt, br, sbox, strat, q, om, aphi, x3phys, err); }
+                                    double aphi, int x3phys, unsigned *err) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) k_cloud_pc2_advance_body<1>(p, P, M, d, gp, dmom, dt, br, sbox, strat, q, om, aphi, x3phys, err);
+}
 
 long long n_active(const Ind &d) { return (long long)d.nmb * d.nx3 * d.nx2 * d.nx1; }
 long long n_all(const Ind &d) { return d.cells() * d.nmb; }
@@ -3603,7 +3660,7 @@ int dustb_cloud_apply_pmbr(const dustb_ctx *c, double a_dt, double sh, void *str
                                           cloud_x3phys(c));
     else if (cloud_x3phys(c)) k_cloud_consistent_dust_u<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt, sh,
                                           cloud_x3phys(c));
-    else k_cloud_consistent_dust_s<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt, sh);
+    else k_cloud_consistent_dust_s<<<(unsigned)((c->part.npart + 127) / 128), 128, 0, S(stream)>>>(pview(c), mview(c), d, c->f.resid, a_dt, sh);
   }
   return launch_status("cloud_apply_pmbr");
 }
