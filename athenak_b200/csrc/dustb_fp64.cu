@@ -277,10 +277,24 @@ __global__ void k_correct_stage(Ind d, const double *u0, int nv, const double *q
 }
 
 // ---- ExplicitPush imex, src/dust/dust_push.cpp:262-297 ----------------------------------
-__global__ void k_push_imex(PCtx P, int three_d, int sbox, int strat, double q, double om,
-                            double gam0, double gam1, double beta_dt, double atw_dt) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
+struct PushCoef { int three_d, sbox, strat; double q, om, gam0, gam1, beta_dt, atw_dt; };
+
+// one particle's rows as values: the fused push reads them once and writes them once.  r() has
+// the rows' names, so the push and the routing below serve the rows in memory and these alike
+// (every index is a constant: the array stays in registers)
+struct LocalRow {
+  double a[15];
+  double *mass;
+  int gid;
+  __device__ __forceinline__ double &r(int c, int) { return c == DUSTB_IPM ? *mass : a[c]; }
+  __device__ __forceinline__ int &i(int, int) { return gid; }
+};
+
+template <typename Row>
+__device__ __forceinline__ void push_one(Row &P, int p, const PushCoef &C) {
+  const int three_d = C.three_d, sbox = C.sbox, strat = C.strat;
+  const double q = C.q, om = C.om, gam0 = C.gam0, gam1 = C.gam1;
+  const double beta_dt = C.beta_dt, atw_dt = C.atw_dt;
   double x_old = P.r(DUSTB_IPX, p), y_old = P.r(DUSTB_IPY, p), z_old = P.r(DUSTB_IPZ, p);
   double vx_old = P.r(DUSTB_IPVX, p), vy_old = P.r(DUSTB_IPVY, p), vz_old = P.r(DUSTB_IPVZ, p);
   double fx = 0.0, fy = 0.0, fz = 0.0;
@@ -302,6 +316,11 @@ __global__ void k_push_imex(PCtx P, int three_d, int sbox, int strat, double q, 
   P.r(DUSTB_IPX, p) = gam0 * x_old + gam1 * P.r(DUSTB_IPX1, p) + beta_dt * vx_old;
   P.r(DUSTB_IPY, p) = gam0 * y_old + gam1 * P.r(DUSTB_IPY1, p) + beta_dt * ydot;
   if (three_d) P.r(DUSTB_IPZ, p) = gam0 * z_old + gam1 * P.r(DUSTB_IPZ1, p) + beta_dt * vz_old;
+}
+
+__global__ void k_push_imex(PCtx P, PushCoef C) {
+  int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) push_one(P, p, C);
 }
 
 // ---- shear-periodic x1 faces (3-D shearing box) ------------------------------------------
@@ -506,9 +525,9 @@ __device__ int route_slot_ml(const MCtx &M, int m, int ix, int iy, int iz, int f
 }
 
 // ---- SetNewPrtclGID, src/bvals/bvals_part.cpp:159-429 (any levels with M.nml) -------------
-__global__ void k_route(PCtx P, MCtx M, Ind d, int x3bc, double *x3rem, unsigned *err, SBox B) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npart) return;
+template <typename Row>
+__device__ __forceinline__ void route_one(Row &P, int p, const MCtx &M, const Ind &d, int x3bc,
+                                          double *x3rem, unsigned *err, const SBox &B) {
   int m = P.i(DUSTB_PGID, p) - M.gids;
   if (!block_ok(d, m)) { report(err, DUSTB_ERR_PGID); return; }
   const double z3a = M.x3min, z3b = M.x3max;
@@ -606,6 +625,41 @@ __global__ void k_route(PCtx P, MCtx M, Ind d, int x3bc, double *x3rem, unsigned
   else if (hi2) { P.r(DUSTB_IPY, p) -= Ly; P.r(DUSTB_IPY1, p) -= Ly; }
   if (lo3) { P.r(DUSTB_IPZ, p) += Lz; P.r(DUSTB_IPZ1, p) += Lz; }
   else if (hi3) { P.r(DUSTB_IPZ, p) -= Lz; P.r(DUSTB_IPZ1, p) -= Lz; }
+}
+
+__global__ void k_route(PCtx P, MCtx M, Ind d, int x3bc, double *x3rem, unsigned *err, SBox B) {
+  int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < P.npart) route_one(P, p, M, d, x3bc, x3rem, err, B);
+}
+
+// FirstTwoImpRK's register copy (first), the imex push and the routing of an imex stage in one
+// pass over the rows, the operations of the three kernels in their order.  Bound by the rows it
+// reads and writes: 172 B per particle instead of 292 (stage 1) and 196 (stage 2).
+__global__ void __launch_bounds__(kThreads, 3) k_push_route(PCtx P, PushCoef C, int first, MCtx M, Ind d, int x3bc,
+                             double *x3rem, unsigned *err, SBox B) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= P.npart) return;
+  LocalRow R;
+  const int gid = P.i(DUSTB_PGID, p);
+  R.gid = gid;
+  R.mass = &P.r(DUSTB_IPM, p);
+#pragma unroll
+  for (int c = DUSTB_IPX; c <= DUSTB_IPVZ; ++c) R.a[c] = P.r(c, p);
+#pragma unroll
+  for (int c = DUSTB_IPRX; c <= DUSTB_IPRZ; ++c) R.a[c] = P.r(c, p);
+#pragma unroll
+  for (int c = 0; c < 6; ++c) R.a[DUSTB_IPX1 + c] = first ? R.a[c] : P.r(DUSTB_IPX1 + c, p);
+  double reg[6];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) reg[c] = R.a[DUSTB_IPX1 + c];
+  push_one(R, p, C);
+  route_one(R, p, M, d, x3bc, x3rem, err, B);
+#pragma unroll
+  for (int c = DUSTB_IPX; c <= DUSTB_IPVZ; ++c) P.r(c, p) = R.a[c];
+#pragma unroll
+  for (int c = 0; c < 6; ++c)
+    if (first || R.a[DUSTB_IPX1 + c] != reg[c]) P.r(DUSTB_IPX1 + c, p) = R.a[DUSTB_IPX1 + c];
+  if (R.gid != gid) P.i(DUSTB_PGID, p) = R.gid;
 }
 
 // ---- deposits: a warp's particles combined per cell (dustb_deposit.cuh) -------------------
@@ -3315,27 +3369,58 @@ int dustb_history_gas(const dustb_ctx *c, double atw_dt, void *stream) {
   return launch_status("history_gas");
 }
 
+static PushCoef push_coef(const dustb_ctx *c, double gam0, double gam1, double beta_dt,
+                          double atw_dt) {
+  return PushCoef{c->mesh.three_d, c->phys.shearing_box, c->phys.stratified, c->phys.qshear,
+                  c->phys.omega0, gam0, gam1, beta_dt, atw_dt};
+}
+
 int dustb_push_imex(const dustb_ctx *c, double gam0, double gam1, double beta_dt, double atw_dt,
                     void *stream) {
   CHECK_CTX(c);
   if (c->part.npart == 0) return DUSTB_OK;
-  k_push_imex<<<PGRID(c)>>>(pview(c), c->mesh.three_d, c->phys.shearing_box, c->phys.stratified,
-                            c->phys.qshear, c->phys.omega0, gam0, gam1, beta_dt, atw_dt);
+  k_push_imex<<<PGRID(c)>>>(pview(c), push_coef(c, gam0, gam1, beta_dt, atw_dt));
   return launch_status("push_imex");
 }
 
-int dustb_route(const dustb_ctx *c, double *x3_removed, void *stream) {
-  CHECK_CTX(c);
+// the checks of a routing: DUSTB_OK, or why it cannot run
+static int route_check(const dustb_ctx *c, double *x3_removed, const SBox &B) {
   if (c->mesh.x3bc == DUSTB_X3_OUTFLOW && !x3_removed) return DUSTB_EINVAL;
   if (c->part.npart == 0) return DUSTB_OK;
-  Ind d = make_ind(c->mesh);
-  const SBox B = sbview(c);
   if (B.on && (!B.sb_gid || B.nb2 <= 0 || B.nb3 <= 0)) return DUSTB_EINVAL;
   // refined meshes: 3-D, both tables, no shear-periodic faces (their maps are single-level)
   if ((c->mesh.nghbr_ml != nullptr) != (c->mesh.mb_lev != nullptr)) return DUSTB_EINVAL;
   if (c->mesh.nghbr_ml && (!c->mesh.three_d || B.on)) return DUSTB_EUNSUP;
-  k_route<<<PGRID(c)>>>(pview(c), mview(c), d, c->mesh.x3bc, x3_removed, c->err, B);
+  return DUSTB_OK;
+}
+
+int dustb_route(const dustb_ctx *c, double *x3_removed, void *stream) {
+  CHECK_CTX(c);
+  const SBox B = sbview(c);
+  const int rc = route_check(c, x3_removed, B);
+  if (rc || c->part.npart == 0) return rc;
+  k_route<<<PGRID(c)>>>(pview(c), mview(c), make_ind(c->mesh), c->mesh.x3bc, x3_removed, c->err, B);
   return launch_status("route");
+}
+
+// the register copy (stage 1), push and routing of an imex stage
+static int imex_push(const dustb_ctx *c, int stage, double gam0, double gam1, double beta_dt,
+                     double atw_dt, double *x3_removed, void *stream) {
+  const SBox B = sbview(c);
+  const int rc = route_check(c, x3_removed, B);
+  if (rc || c->part.npart == 0) return rc;
+  k_push_route<<<PGRID(c)>>>(pview(c), push_coef(c, gam0, gam1, beta_dt, atw_dt), stage == 1,
+                             mview(c), make_ind(c->mesh), c->mesh.x3bc, x3_removed, c->err, B);
+  return launch_status("push and route");
+}
+
+// the gas register of stage 1 (dustb_register_copy without the particles)
+static int gas_register(const dustb_ctx *c, void *stream) {
+  const Ind d = make_ind(c->mesh);
+  const cudaError_t e = cudaMemcpyAsync(c->f.u1, c->f.u0, (size_t)n_all(d) * c->f.nvar_gas * sizeof(double),
+                                        cudaMemcpyDeviceToDevice, S(stream));
+  if (e != cudaSuccess) { dustb_host::set_error("gas_register", e); return DUSTB_ELAUNCH; }
+  return DUSTB_OK;
 }
 
 int dustb_deposit_qp(const dustb_ctx *c, double a_dt, double sh, void *stream) {
@@ -3863,12 +3948,11 @@ int dustb_imex_cycle(const dustb_ctx *c, const dustb_imex_coeffs *co, double *x3
   int rc;
 #define RUN(x) do { rc = (x); if (rc) return rc; } while (0)
   for (int stage = 1; stage <= 2; ++stage) {
-    if (stage == 1) RUN(dustb_register_copy(c, stream));
+    if (stage == 1) RUN(gas_register(c, stream));
     RUN(dustb_gas_rk_noflux(c, gam0[stage - 1], gam1[stage - 1], stream));
     if (stage == 2 && br) RUN(dustb_history_gas(c, atw22 * dt, stream));
-    RUN(dustb_push_imex(c, gam0[stage - 1], gam1[stage - 1], beta[stage - 1] * dt,
-                        (stage == 2) ? atw22 * dt : 0.0, stream));
-    RUN(dustb_route(c, x3_removed, stream));
+    RUN(imex_push(c, stage, gam0[stage - 1], gam1[stage - 1], beta[stage - 1] * dt,
+                  (stage == 2) ? atw22 * dt : 0.0, x3_removed, stream));
     const double sh = co->sh[stage - 1];
     if (br) {
       RUN(dustb_deposit_qp(c, a_dt, sh, stream));
@@ -3928,12 +4012,11 @@ int dustb_refined_imex_cycle(const dustb_ctx *c, const dustb_dep_plan *plan,
   Ind d = make_ind(c->mesh);
   int rc;
   for (int stage = 1; stage <= 2; ++stage) {
-    if (stage == 1) RUN(dustb_register_copy(c, stream));
+    if (stage == 1) RUN(gas_register(c, stream));
     RUN(dustb_gas_rk_noflux(c, gam0[stage - 1], gam1[stage - 1], stream));
     if (stage == 2 && br) RUN(dustb_history_gas(c, atw22 * dt, stream));
-    RUN(dustb_push_imex(c, gam0[stage - 1], gam1[stage - 1], beta[stage - 1] * dt,
-                        (stage == 2) ? atw22 * dt : 0.0, stream));
-    RUN(dustb_route(c, x3_removed, stream));
+    RUN(imex_push(c, stage, gam0[stage - 1], gam1[stage - 1], beta[stage - 1] * dt,
+                  (stage == 2) ? atw22 * dt : 0.0, x3_removed, stream));
     if (br) {
       RUN(dustb_deposit_qp(c, a_dt, 0.0, stream));
       RUN(dustb_ghost_add_plan(c, plan, c->f.qdep, 5, stream));
@@ -3976,12 +4059,11 @@ static int cloud_imex_cycle(const dustb_ctx *c, const dustb_imex_coeffs *co, dou
   const int br = c->phys.back_reaction;
   int rc;
   for (int stage = 1; stage <= 2; ++stage) {
-    if (stage == 1) RUN(dustb_register_copy(c, stream));
+    if (stage == 1) RUN(gas_register(c, stream));
     RUN(dustb_gas_rk_noflux(c, gam0[stage - 1], gam1[stage - 1], stream));
     if (stage == 2 && br) RUN(dustb_history_gas(c, atw22 * dt, stream));
-    RUN(dustb_push_imex(c, gam0[stage - 1], gam1[stage - 1], beta[stage - 1] * dt,
-                        (stage == 2) ? atw22 * dt : 0.0, stream));
-    RUN(dustb_route(c, x3_removed, stream));
+    RUN(imex_push(c, stage, gam0[stage - 1], gam1[stage - 1], beta[stage - 1] * dt,
+                  (stage == 2) ? atw22 * dt : 0.0, x3_removed, stream));
     const double sh = co->sh[stage - 1];
     if (br) RUN(dustb_cloud_deposit_qp(c, a_dt, sh, stream));
     RUN(dustb_solve_ustar(c, stream));
