@@ -89,15 +89,16 @@ __device__ __forceinline__ int warp_rank(unsigned key, bool live) {
 // NV values per cell; ONE: the first is the weight itself, the others the weight times q[0],
 // q[1], ...
 // at(k): the field address (variable 0) of this lane's window cell about the anchor with field
-// index k, null if no block owns it; variables vs apart
-template <int NV, bool ONE>
+// index k, null if no block owns it; variables vs apart.  CEN: lane 27, which has no window
+// cell, sums q[3] of the anchor cell's particles instead
+template <int NV, bool ONE, bool CEN = false>
 struct CellDeposit {
   static constexpr int NQ = NV - (ONE ? 1 : 0);
   double acc[NV];
   long long base;               // the field index of the current anchor cell
   unsigned cur;                 // the current anchor cell (kNoCell: none)
   int a, b, c;                  // this lane's cell of the window, -1..1 each
-  bool on;
+  bool on, centre;
 
   // lane = 9 (a + 1) + 3 (c + 1) + b + 1: a column is nine consecutive lanes
   __device__ __forceinline__ void init(bool three_d) {
@@ -105,6 +106,7 @@ struct CellDeposit {
     const int r = l % 9;
     a = l / 9 - 1; c = r / 3 - 1; b = r % 3 - 1;
     on = lane < 27 && (three_d || c == 0);
+    centre = CEN && lane == 27;
     cur = kNoCell;
     base = 0;
 #pragma unroll
@@ -112,12 +114,12 @@ struct CellDeposit {
   }
   template <typename At>
   __device__ __forceinline__ void put(bool who, long long vs, At &&at) {
-    if (!who) return;
+    if (!(who || centre)) return;
     double *t = at(base);
     if (!t) return;
 #pragma unroll
     for (int v = 0; v < NV; ++v)
-      if (acc[v] != 0.0) atomicAdd(t + v * vs, acc[v]);
+      if (acc[v] != 0.0 && (v == 0 || !centre)) atomicAdd(t + v * vs, acc[v]);
   }
   template <typename At>
   __device__ __forceinline__ void flush(long long vs, At &&at) {
@@ -162,14 +164,15 @@ struct CellDeposit {
 #pragma unroll 4
         for (int p = lo; p < hi; ++p) {
           const double w = wyz[p] * wx[p];
-          if (ONE) acc[0] += w;
+          if (ONE) acc[0] += centre ? s.q[p][3] : w;
 #pragma unroll
           for (int v = 0; v < NQ; ++v)
             acc[v + (ONE ? 1 : 0)] = __fma_rn(w, s.q[p][v], acc[v + (ONE ? 1 : 0)]);
         }
       } else {
         for (int p = lo; p < hi; ++p) {
-          if (wyz[p] == 0.0) continue;
+          if (CEN && centre) acc[0] += s.q[p][3];
+          if (wyz[p] == 0.0 || (CEN && centre)) continue;
           const double w = wyz[p] * wx[p];
           if (ONE) acc[0] += w;
 #pragma unroll

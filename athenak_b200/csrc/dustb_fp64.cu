@@ -689,17 +689,25 @@ struct BlockScale {
 
 // every particle of the launch through particle(p, stencil, scale), which returns whether it
 // deposits, and its deposit into variable v0 on of an nvar-variable field
-template <int NV, bool ONE, typename F>
+// (cen, CEN: a field that takes q[3] of every particle at its anchor cell, one variable of nvc)
+template <int NV, bool ONE, bool CEN = false, typename F>
 __device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &d, double *field,
-                                                  int nvar, int v0, F &&particle) {
+                                                  int nvar, int v0, F &&particle,
+                                                  double *cen = nullptr, int nvc = 0) {
   __shared__ WarpStage s_stage[kDepWarps];
   WarpStage &st = s_stage[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  CellDeposit<NV, ONE> dep;
+  CellDeposit<NV, ONE, CEN> dep;
   dep.init(d.three_d);
   const long long vs = d.cells();
   double *mine = field + ((long long)(dep.c * d.n2 + dep.b) * d.n1 + dep.a);
-  auto at = [&](long long k) { return mine + k; };
+  auto at = [&](long long k) -> double * {
+    if (CEN && dep.centre) {
+      const unsigned cells = (unsigned)vs, m = dep.cur / cells;
+      return cen + (long long)m * nvc * vs + (dep.cur - m * cells);
+    }
+    return mine + k;
+  };
   BlockScale bs;
   const long long first = ((long long)blockIdx.x * kDepWarps + (threadIdx.x >> 5)) * nb * 32;
   for (int b = 0; b < nb; ++b) {
@@ -787,17 +795,22 @@ __device__ __forceinline__ bool place(const PCtx &P, const MCtx &M, const Ind &d
 }
 
 // ---- DepositDrag imex scatter, src/dust/dust_pm.cpp:225-274 ------------------------------
+// CEN: also the centre mass of the consistent split (k_center_mass) into res, variable 3 of 4, for
+// a stage without a shear shift, whose weight position is the particle's own
+template <bool CEN>
 __global__ void __launch_bounds__(32 * kDepWarps, 5)
-k_scatter(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh, unsigned *err, int nb) {
-  deposit_particles<4, true>(P.npart, nb, d, qdep, 5, 0, [&](int p, Stencil &t, BlockScale &bs) {
+k_scatter(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh, unsigned *err, int nb,
+          double *res) {
+  deposit_particles<4, true, CEN>(P.npart, nb, d, qdep, 5, 0, [&](int p, Stencil &t, BlockScale &bs) {
     const double x = P.r(DUSTB_IPX, p);
     if (!place(P, M, d, p, x, P.r(DUSTB_IPY, p) + sh * x, P.r(DUSTB_IPZ, p), t, bs, err)) return false;
     const double cj = a_dt / (P.r(DUSTB_IPTS, p) + a_dt);
-    t.fac = P.r(DUSTB_IPM, p) * cj / bs.vol;
+    const double mass = P.r(DUSTB_IPM, p);
+    t.fac = mass * cj / bs.vol;
     t.q[0] = P.r(DUSTB_IPVX, p); t.q[1] = P.r(DUSTB_IPVY, p); t.q[2] = P.r(DUSTB_IPVZ, p);
-    t.q[3] = 0.0;
+    t.q[3] = (CEN && !(mass <= 0.0)) ? t.fac : 0.0;
     return true;
-  });
+  }, CEN ? res + 3 * d.cells() : nullptr, 4);
 }
 
 // ---- ghost exchanges (pull form, one thread per destination cell) -----------------------
@@ -3428,7 +3441,24 @@ int dustb_deposit_qp(const dustb_ctx *c, double a_dt, double sh, void *stream) {
   Ind d = make_ind(c->mesh);
   cudaMemsetAsync(c->f.qdep, 0, (size_t)n_all(d) * 5 * sizeof(double), S(stream));
   if (c->part.npart > 0)
-    k_scatter<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, c->err, NB(c));
+    k_scatter<false><<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, c->err, NB(c), nullptr);
+  return launch_status("deposit_qp");
+}
+
+// whether a cycle's deposit leaves the split's centre mass beside Q/P
+static bool centre_with_qp(const dustb_ctx *c, double sh) {
+  return c->phys.back_reaction && c->phys.consistent_gas && sh == 0.0;
+}
+
+// dustb_deposit_qp of a cycle, with the centre mass (resid, zeroed first) where centre_with_qp
+static int deposit_qp_stage(const dustb_ctx *c, double a_dt, double sh, void *stream) {
+  if (!centre_with_qp(c, sh)) return dustb_deposit_qp(c, a_dt, sh, stream);
+  const Ind d = make_ind(c->mesh);
+  cudaMemsetAsync(c->f.qdep, 0, (size_t)n_all(d) * 5 * sizeof(double), S(stream));
+  cudaMemsetAsync(c->f.resid, 0, (size_t)n_all(d) * 4 * sizeof(double), S(stream));
+  if (c->part.npart > 0)
+    k_scatter<true><<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, c->err, NB(c),
+                                         c->f.resid);
   return launch_status("deposit_qp");
 }
 
@@ -3518,7 +3548,8 @@ int dustb_gather_kick_pmbr(const dustb_ctx *c, double a_dt, double sh, void *str
   return launch_status("gather_kick_pmbr");
 }
 
-int dustb_apply_pmbr(const dustb_ctx *c, double a_dt, void *stream) {
+// centre: resid holds the centre mass already (deposit_qp_stage)
+static int apply_pmbr(const dustb_ctx *c, double a_dt, bool centre, void *stream) {
   CHECK_CTX(c);
   if (!c->phys.back_reaction) return DUSTB_OK;
   Ind d = make_ind(c->mesh);
@@ -3527,14 +3558,20 @@ int dustb_apply_pmbr(const dustb_ctx *c, double a_dt, void *stream) {
     k_pmbr<<<blocks_for(n_active(d)), kThreads, 0, S(stream)>>>(d, c->f.u0, c->f.nvar_gas, c->f.dmom, inv_adt);
     return launch_status("apply_pmbr");
   }
-  cudaMemsetAsync(c->f.resid, 0, (size_t)n_all(d) * 4 * sizeof(double), S(stream));
-  if (c->part.npart > 0)
-    k_center_mass<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt, c->err);
+  if (!centre) {
+    cudaMemsetAsync(c->f.resid, 0, (size_t)n_all(d) * 4 * sizeof(double), S(stream));
+    if (c->part.npart > 0)
+      k_center_mass<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt, c->err);
+  }
   k_consistent_gas<<<blocks_for(n_active(d)), kThreads, 0, S(stream)>>>(
       d, c->f.u0, c->f.nvar_gas, c->f.ustar, c->f.qdep, c->f.dmom, c->f.resid, inv_adt);
   if (c->part.npart > 0)
     k_consistent_dust<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt);
   return launch_status("apply_pmbr");
+}
+
+int dustb_apply_pmbr(const dustb_ctx *c, double a_dt, void *stream) {
+  return apply_pmbr(c, a_dt, false, stream);
 }
 
 int dustb_newdt(const dustb_ctx *c, double dt_cfl, double *dt_out, void *stream) {
@@ -3955,7 +3992,7 @@ int dustb_imex_cycle(const dustb_ctx *c, const dustb_imex_coeffs *co, double *x3
                   (stage == 2) ? atw22 * dt : 0.0, x3_removed, stream));
     const double sh = co->sh[stage - 1];
     if (br) {
-      RUN(dustb_deposit_qp(c, a_dt, sh, stream));
+      RUN(deposit_qp_stage(c, a_dt, sh, stream));
       RUN(dustb_ghost_add(c, c->f.qdep, 5, stream));
     }
     RUN(dustb_solve_ustar(c, stream));
@@ -3967,7 +4004,7 @@ int dustb_imex_cycle(const dustb_ctx *c, const dustb_imex_coeffs *co, double *x3
     RUN(dustb_gather_kick_pmbr(c, a_dt, sh, stream));
     if (br) {
       RUN(dustb_ghost_add(c, c->f.dmom, 3, stream));
-      RUN(dustb_apply_pmbr(c, a_dt, stream));
+      RUN(apply_pmbr(c, a_dt, centre_with_qp(c, sh), stream));
     }
     RUN(dustb_ghost_copy(c, c->f.u0, c->f.nvar_gas, 0, stream));
   }
@@ -4018,7 +4055,7 @@ int dustb_refined_imex_cycle(const dustb_ctx *c, const dustb_dep_plan *plan,
     RUN(imex_push(c, stage, gam0[stage - 1], gam1[stage - 1], beta[stage - 1] * dt,
                   (stage == 2) ? atw22 * dt : 0.0, x3_removed, stream));
     if (br) {
-      RUN(dustb_deposit_qp(c, a_dt, 0.0, stream));
+      RUN(deposit_qp_stage(c, a_dt, 0.0, stream));
       RUN(dustb_ghost_add_plan(c, plan, c->f.qdep, 5, stream));
     }
     RUN(dustb_solve_ustar(c, stream));
@@ -4031,7 +4068,7 @@ int dustb_refined_imex_cycle(const dustb_ctx *c, const dustb_dep_plan *plan,
     RUN(dustb_gather_kick_pmbr(c, a_dt, 0.0, stream));
     if (br) {
       RUN(dustb_ghost_add_plan(c, plan, c->f.dmom, 3, stream));
-      RUN(dustb_apply_pmbr(c, a_dt, stream));
+      RUN(apply_pmbr(c, a_dt, centre_with_qp(c, 0.0), stream));
     }
     RUN(dustb_ghost_copy_ml(c, c->f.u0, c->f.nvar_gas, coarse, coarse_bytes, stream));
   }
