@@ -1,0 +1,228 @@
+"""The grouped and fused forms of the FP64 kernels at the sizes where they can go wrong: deposits
+summed per cell inside a warp (any row order, weights, partial warps, non-finite values), the
+cycle's fused push and centre mass, the history row's chunk edges, long runs of the cell sort,
+the scan's two forms, the exchanges' variable groups and the clouds' slots on odd blocks --
+against the CPU oracle; the mixed stage's window and buffer rules against the FP64 form."""
+import numpy as np
+import pytest
+
+from athenak_b200.inputs import make_state
+from athenak_b200.mesh import uniform_mesh
+from oracle.oracle import Oracle
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12                    # FP64 sums in another order, of the field's scale
+
+
+def fields(a, b):
+    return max(np.abs(a[:, v] - b[:, v]).max() / max(np.abs(b[:, v]).max(), 1e-300)
+               for v in range(a.shape[1]))
+
+
+def state(cells, block, ppc, seed=5, **kw):
+    d = 0.01
+    ms = uniform_mesh(cells, block, 2, tuple(-0.5 * d * n for n in cells),
+                      tuple(0.5 * d * n for n in cells))
+    return ms, make_state(ms, [0.01, 0.3], [1.0, 0.5], ppc, seed=seed, vel_noise=0.05,
+                          gas_noise=1e-2, **kw)
+
+
+def permute(st, order):
+    st.pr[:, :st.npart] = st.pr[:, order]
+    st.pi[:, :st.npart] = st.pi[:, order]
+
+
+def clump(st, n, seed=3):
+    """the first n particles into one cell of block 0"""
+    rng = np.random.default_rng(seed)
+    mb = st.mesh.mb_size[0]
+    c = [st.mesh.nx[0] - 1, 0, st.mesh.nx[2] // 2]
+    for a, (r, r1) in enumerate(((0, 6), (2, 8), (4, 10))):
+        if a == 2 and not st.mesh.three_d:
+            continue
+        x = mb[a] + (c[a] + rng.random(n)) * mb[6 + a]
+        st.pr[r, :n] = st.pr[r1, :n] = x
+    st.pi[0, :n] = 0
+
+
+def pair(st, phys):
+    from athenak_b200.drag import DeviceDust
+    return Oracle(st, phys), DeviceDust(st, phys)
+
+
+@pytest.mark.parametrize("order", ["cell", "drawn", "reversed", "clumped"])
+@pytest.mark.parametrize("scheme,cells,block", [(2, (10, 14, 6), (5, 7, 6)), (1, (12, 18, 1), (12, 9, 1)),
+                                                (0, (8, 6, 6), (4, 6, 3))])
+def test_deposits_of_every_row_order(order, scheme, cells, block):
+    ms, st = state(cells, block, 3)
+    if order == "clumped":
+        clump(st, min(300, st.npart))
+    phys = dict(scheme=scheme, drag_solver=2)
+    if order != "drawn":
+        o = Oracle(st, phys)
+        by_cell, _ = o.sort_order()
+        permute(st, by_cell if order != "reversed" else by_cell[::-1].copy())
+    o, g = pair(st, phys)
+    a_dt = 2e-3
+    o.register_copy(); g.register_copy()
+    assert o.pc2_predictor(a_dt) == 0
+    g.pc2_predictor(a_dt)
+    assert fields(g.host("qdep")[:, 1:], o.qdep[:, 1:]) < TOL
+    assert o.deposit_qp(a_dt) == 0
+    g.deposit_qp(a_dt)
+    assert fields(g.host("qdep")[:, :4], o.qdep[:, :4]) < TOL
+    for s in (o, g):
+        s.ghost_add("qdep", 5); s.solve_ustar(); s.dc1_sweep(a_dt); s.ghost_copy("ustar", 3)
+    assert fields(g.host("ustar"), o.ustar) < TOL
+    o.gather_kick_pmbr(a_dt); g.gather_kick_pmbr(a_dt)
+    assert fields(g.host("dmom"), o.dmom) < TOL
+    assert g.error_word() == 0
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 129])
+def test_partial_warps_and_fused_cycle(n):
+    ms, st = state((8, 8, 8), (4, 8, 8), 1, seed=8)
+    st.npart = n
+    phys = dict(scheme=2, drag_solver=2)
+    o, g = pair(st, phys)
+    for _ in range(2):
+        assert o.imex_cycle(2e-3) == 0
+        g.imex_cycle(2e-3)
+    gp, gi = g.host("pr"), g.host("pi")
+    np.testing.assert_array_equal(gi, o.st.pi[:, :n])
+    for r in range(17):
+        sc = max(np.abs(o.st.pr[r, :n]).max(), 1e-300)
+        assert np.abs(gp[r] - o.st.pr[r, :n]).max() <= TOL * sc, r
+    assert fields(g.host("u0"), o.u0) < 1e-11
+    assert g.error_word() == 0
+
+
+def test_zero_weights_keep_non_finite_values_out():
+    """NGP: a particle with an infinite velocity reaches its own cell alone."""
+    ms, st = state((8, 8, 8), (8, 8, 8), 2, seed=4)
+    st.pr[1, 7] = np.inf
+    phys = dict(scheme=0)
+    o, g = pair(st, phys)
+    assert o.deposit_qp(1e-3) == 0
+    g.deposit_qp(1e-3)
+    np.testing.assert_array_equal(np.isfinite(g.host("qdep")[:, :4]), np.isfinite(o.qdep[:, :4]))
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 4095, 4096, 4097, 8300])
+def test_history_row_at_chunk_edges(n):
+    ms, st = state((16, 16, 16), (16, 16, 16), 2, seed=9)
+    st.npart = n
+    st.pr[16, n // 2] = 0.0 if n > 1 else st.pr[16, 0]
+    o, g = pair(st, dict(scheme=2))
+    rg = g.phst().cpu().numpy()
+    ro, err = o.phst()
+    assert err == 0 and g.error_word() == 0
+    np.testing.assert_array_equal(rg[:7], ro[:7])
+    np.testing.assert_array_equal(rg[8:12], ro[8:12])
+
+
+@pytest.mark.parametrize("run", [47, 48, 49, 128, 129, 256, 257, 1024, 1025])
+def test_sort_of_long_runs(run):
+    ms, st = state((8, 8, 8), (8, 8, 8), 2, seed=6)
+    clump(st, min(run, st.npart))
+    rng = np.random.default_rng(run)
+    permute(st, rng.permutation(st.npart))
+    o, g = pair(st, {})
+    np.testing.assert_array_equal(g.cell_index()[0].cpu().numpy(), o.sort_order()[0])
+
+
+@pytest.mark.parametrize("cells", [(256, 256, 192), (256, 256, 256)])
+def test_scan_on_both_sides_of_the_two_launch_limit(cells):
+    """3073 and 4097 tiles of 4096 bins: the bins' starts against a count on the host."""
+    from athenak_b200.drag import DeviceDust
+    ms = uniform_mesh(cells, (64, 64, 64), 2, tuple(-0.5 * n for n in cells),
+                      tuple(0.5 * n for n in cells))
+    g = DeviceDust.empty(ms, 5000, {}, nspecies=1)
+    rng = np.random.default_rng(2)
+    c = np.stack([rng.integers(0, n, 5000) for n in cells])
+    b = c // 64
+    blk = (b[2] * ms.nblocks[1] + b[1]) * ms.nblocks[0] + b[0]
+    l = c % 64
+    key = ((blk * 64 + l[2]) * 64 + l[1]) * 64 + l[0]
+    for a in range(3):
+        g.t["pr"][2 * a].copy_(torch.from_numpy(c[a] + 0.5 - 0.5 * cells[a]))
+    g.t["pi"][0].copy_(torch.from_numpy(blk.astype(np.int32)))
+    order, cstart = g.cell_index()
+    np.testing.assert_array_equal(order.cpu().numpy(), np.argsort(key, kind="stable"))
+    cs = cstart.cpu().numpy()
+    assert cs[-1] == 5000
+    np.testing.assert_array_equal(np.diff(cs)[np.unique(key)], np.unique(key, return_counts=True)[1])
+
+
+@pytest.mark.parametrize("x3bc,shear", [(0, False), (1, False), (2, True)])
+def test_additive_exchange_in_any_number_of_variables(x3bc, shear):
+    """The variables are taken five, three or one at a time: 7 together as each alone."""
+    from athenak_b200.drag import DeviceDust
+    ms = uniform_mesh((8, 12, 8), (4, 4, 4), 2, (-0.5,) * 3, (0.5,) * 3, x3bc=x3bc, shear_x1=shear)
+    st = make_state(ms, [0.1], [1.0], 1, seed=2)
+    g = DeviceDust(st, dict(scheme=2, shearing_box=shear))
+    g.set_time(0.37)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1)
+    for nv in (1, 2, 3, 4, 5, 7):
+        f = torch.randn(ms.field_shape(nv), dtype=torch.float64, device="cuda", generator=gen)
+        g.t["many"] = f.clone()
+        g.ghost_add("many", nv)
+        one = torch.empty_like(f)
+        for v in range(nv):
+            g.t["single"] = f[:, v:v + 1].contiguous()
+            g.ghost_add("single", 1)
+            one[:, v:v + 1] = g.t["single"]
+        assert torch.equal(g.t["many"], one), nv
+
+
+@pytest.mark.parametrize("cells,block", [((10, 14, 6), (5, 7, 6)), ((12, 18, 1), (4, 9, 1)),
+                                         ((6, 4, 8), (2, 2, 4))])
+def test_cloud_slots_on_odd_blocks(cells, block):
+    """Levels 0 to 3 in the drawn order: the gathered velocities bit for bit, the deposits to
+    their order."""
+    ms, st = state(cells, block, 3, seed=13)
+    st.pi[3, :st.npart] = np.arange(st.npart) % 4
+    o, g = pair(st, dict(scheme=2))
+    assert o.cloud_deposit_qp(1.3e-3, 0.0) == 0
+    g.cloud_deposit_qp(1.3e-3, 0.0)
+    assert fields(g.host("qdep")[:, :4], o.qdep[:, :4]) < TOL
+    us = np.random.default_rng(6).standard_normal(o.ustar.shape) * 0.05
+    o.ustar[...] = us
+    g.t["ustar"].copy_(torch.from_numpy(us))
+    o.ghost_copy("ustar", 3, 0); g.ghost_copy("ustar", 3, 0)
+    assert o.cloud_gather_kick(2e-3, 0.0, o.gather_pack()) == 0
+    g.cloud_gather_kick(2e-3, 0.0)
+    for r in (1, 3, 5, 12, 13, 14):
+        np.testing.assert_array_equal(g.host("pr")[r], o.st.pr[r, :st.npart])
+    assert fields(g.host("dmom"), o.dmom) < TOL
+    assert g.error_word() == 0
+
+
+@pytest.mark.parametrize("cells,block,ppc", [
+    ((6, 10, 14), (6, 10, 14), 3),      # one block, its own neighbour on every side
+    ((4, 6, 4), (2, 6, 2), 5),          # blocks of two cells: every cell at a face
+    ((64, 36, 1), (64, 9, 1), 2),       # 2-D, few particles per tile: the small buffer
+    ((64, 8, 1), (64, 4, 1), 40),       # 2-D, dense: the large one, several passes
+])
+def test_mixed_stage_matches_fp64(cells, block, ppc):
+    """The window written by the solves and the buffer rule: every velocity and the gas within
+    the mixed form's 1e-5 of the largest (plain back-reaction, two cycles)."""
+    from athenak_b200.drag import DeviceDust
+    from athenak_b200.mixed import MixedDust
+    ms, st = state(cells, block, ppc, seed=17)
+    phys = dict(scheme=2, drag_solver=3, consistent_gas=False)
+    ref, mx = DeviceDust(st, phys), MixedDust(st, phys)
+    for _ in range(2):
+        ref.imex_cycle(2e-3)
+        mx.imex_cycle(2e-3)
+    mx.export()
+    assert ref.error_word() == 0 and mx.error_word() == 0
+    a, b = mx.dev.host("pr"), ref.host("pr")
+    for r in (1, 3, 5):
+        assert np.abs(a[r] - b[r]).max() < 1e-5 * np.abs(b[[1, 3, 5]]).max(), r
+    ua, ub = ms.active(mx.dev.host("u0")), ms.active(ref.host("u0"))
+    for v in range(1, 4):
+        assert np.abs(ua[:, v] - ub[:, v]).max() < 1e-5 * max(np.abs(ub[:, v]).max(), 1e-300), v
