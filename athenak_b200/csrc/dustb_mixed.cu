@@ -977,12 +977,9 @@ __device__ __forceinline__ void move_particle(const PBuf &S, const PBuf &D, cons
   D.f[F_TS][q] = ts; D.f[F_M][q] = mass; D.f[F_CC][q] = cc;
 }
 
-// (held to 64 registers, four CTAs per SM: the level carry of SP 2, which few particles take, had
-// it at 87, two CTAs and 24 % of the DRAM rate; 5.0 M particles 0.29 -> 0.21 ms)
 template <int KIND, int SP>
-__global__ void __launch_bounds__(kT, 4) k_move(PBuf S, PBuf D, const int *key_in, int *cursor,
-                                             const __grid_constant__ Geo G, int n,
-                                             const __grid_constant__ PushArgs P) {
+__device__ __forceinline__ void move_cta(const PBuf &S, const PBuf &D, const int *key_in,
+                                         int *cursor, const Geo &G, int n, const PushArgs &P) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = p < n;
   const unsigned act = __ballot_sync(0xffffffffu, live);
@@ -1012,6 +1009,23 @@ __global__ void __launch_bounds__(kT, 4) k_move(PBuf S, PBuf D, const int *key_i
       }
     }
   }
+}
+
+// (no minimum of CTAs: by itself the compiler takes 48 registers for the periodic form, five CTAs;
+// asked for four it takes 64 and the move of 33.5 M particles goes from 1.03 to 1.14 ms)
+template <int KIND, int SP>
+__global__ void __launch_bounds__(kT) k_move(PBuf S, PBuf D, const int *key_in, int *cursor,
+                                             const __grid_constant__ Geo G, int n,
+                                             const __grid_constant__ PushArgs P) {
+  move_cta<KIND, SP>(S, D, key_in, cursor, G, n, P);
+}
+// the refined form held to 64 registers, four CTAs per SM: the level carry, which few particles
+// take, had it at 87, two CTAs and 24 % of the DRAM rate (5.0 M particles 0.29 -> 0.21 ms)
+template <int KIND>
+__global__ void __launch_bounds__(kT, 4) k_move_ml(PBuf S, PBuf D, const int *key_in, int *cursor,
+                                                   const __grid_constant__ Geo G, int n,
+                                                   const __grid_constant__ PushArgs P) {
+  move_cta<KIND, 2>(S, D, key_in, cursor, G, n, P);
 }
 
 // ---- tile deposit kernels -------------------------------------------------------------------
@@ -1859,23 +1873,39 @@ __global__ void __maxnreg__(168) k_tile(PBuf S, Geo G, TileArgs T,
 // and finish on short ones.  One CTA; also clears the stage's queue counters.
 // (tile t is cells t nct .. (t + 1) nct - 1 of the sort.  The tiles of a uniform mesh all fall
 // into one bucket: lanes with the same bucket add once, or the counter's address serialises
-// them -- 16384 tiles 43 us)
+// them; and a thread reads four tiles' ranges at a time, or their latencies add up -- 16384
+// tiles 43 us without either)
 __global__ void __launch_bounds__(1024) k_tile_order(const int *cstart, int nct, int ntiles,
                                                      int *order, int *qhead) {
   __shared__ int hist[33], base[33];
-  auto bucket = [&](int t) {
-    if (t >= ntiles) return 33;                    // (no tile)
-    const int cost = cstart[(long long)(t + 1) * nct] - cstart[(long long)t * nct];
-    return cost > 0 ? __clz(cost) : 32;            // 32 - log2 size: heavy tiles first
+  constexpr int U = 4;
+  auto buckets = [&](int t0, int b[U]) {
+    int lo[U], hi[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = min(t0 + u * 1024, ntiles - 1);
+      lo[u] = cstart[(long long)t * nct];
+      hi[u] = cstart[(long long)(t + 1) * nct];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int cost = hi[u] - lo[u];
+      // (33: no tile; 32 - log2 size: heavy tiles first)
+      b[u] = (t0 + u * 1024 >= ntiles) ? 33 : (cost > 0 ? __clz(cost) : 32);
+    }
   };
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < 33) hist[threadIdx.x] = 0;
   if (threadIdx.x < kQueues) qhead[threadIdx.x] = 0;
   __syncthreads();
-  for (int t0 = 0; t0 < ntiles; t0 += 1024) {
-    const int b = bucket(t0 + (int)threadIdx.x);
-    const unsigned peers = __match_any_sync(0xffffffffu, b);
-    if (b < 33 && lane == __ffs(peers) - 1) atomicAdd(&hist[b], __popc(peers));
+  for (int c0 = 0; c0 < ntiles; c0 += U * 1024) {
+    int b[U];
+    buckets(c0 + (int)threadIdx.x, b);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned peers = __match_any_sync(0xffffffffu, b[u]);
+      if (b[u] < 33 && lane == __ffs(peers) - 1) atomicAdd(&hist[b[u]], __popc(peers));
+    }
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -1883,14 +1913,18 @@ __global__ void __launch_bounds__(1024) k_tile_order(const int *cstart, int nct,
     for (int b = 0; b < 33; ++b) { base[b] = run; run += hist[b]; }
   }
   __syncthreads();
-  for (int t0 = 0; t0 < ntiles; t0 += 1024) {
-    const int t = t0 + (int)threadIdx.x, b = bucket(t);
-    const unsigned peers = __match_any_sync(0xffffffffu, b);
-    const int lead = __ffs(peers) - 1;
-    int at = 0;
-    if (b < 33 && lane == lead) at = atomicAdd(&base[b], __popc(peers));
-    at = __shfl_sync(0xffffffffu, at, lead) + __popc(peers & ((1u << lane) - 1u));
-    if (b < 33) order[at] = t;
+  for (int c0 = 0; c0 < ntiles; c0 += U * 1024) {
+    int b[U];
+    buckets(c0 + (int)threadIdx.x, b);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned peers = __match_any_sync(0xffffffffu, b[u]);
+      const int lead = __ffs(peers) - 1;
+      int at = 0;
+      if (b[u] < 33 && lane == lead) at = atomicAdd(&base[b[u]], __popc(peers));
+      at = __shfl_sync(0xffffffffu, at, lead) + __popc(peers & ((1u << lane) - 1u));
+      if (b[u] < 33) order[at] = c0 + (int)threadIdx.x + u * 1024;
+    }
   }
 }
 
@@ -2378,9 +2412,11 @@ int push_sort(const MState &S, const PBuf &src, const PBuf &dst, const Geo &G, i
   if (n > 0) {
 #define DUSTB_MOVE(K, SPF) k_move<K, SPF><<<nblk(n), kT, 0, st>>>(src, dst, S.key, S.cursor, G, n, P)
     if (G.ml) {
-      if (P.kind == PK_HALF) DUSTB_MOVE(PK_HALF, 2);
-      else if (P.kind == PK_FULL) DUSTB_MOVE(PK_FULL, 2);
-      else DUSTB_MOVE(PK_IMEX, 2);
+#define DUSTB_MOVE_ML(K) k_move_ml<K><<<nblk(n), kT, 0, st>>>(src, dst, S.key, S.cursor, G, n, P)
+      if (P.kind == PK_HALF) DUSTB_MOVE_ML(PK_HALF);
+      else if (P.kind == PK_FULL) DUSTB_MOVE_ML(PK_FULL);
+      else DUSTB_MOVE_ML(PK_IMEX);
+#undef DUSTB_MOVE_ML
     } else if (G.ghost) {
       if (P.kind == PK_HALF) DUSTB_MOVE(PK_HALF, 1);
       else if (P.kind == PK_FULL) DUSTB_MOVE(PK_FULL, 1);
