@@ -214,7 +214,7 @@ __global__ void k_restrict(AmrArgs A) {
 // 2. the exchange, pulled by every receiving (block, slot): one CTA each, its threads over the
 // cells of the slot's box and the variables (most slots are empty or small: a thread per cell
 // of the largest box of every slot left nine in ten idle after its index divisions; 176 blocks
-// of 16^3 and 4 variables: 130 -> 13 us)
+// of 16^3, 3 and 4 variables: 128 -> 30 us)
 __global__ void __launch_bounds__(kThr) k_exchange(AmrArgs A) {
   const int m = blockIdx.x / 56, n = blockIdx.x - m * 56;
   const int gs = A.nb[(long long)m * 56 + n];

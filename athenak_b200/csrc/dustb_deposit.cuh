@@ -13,12 +13,13 @@
 // more than before and land on three consecutive cells per row.  The products are those of the
 // one-thread-per-particle form; only the order of the sums differs.
 //
-// 4.2 M particles at 16 per cell in cell order (64^3 cells, 5 CTAs per SM): Q/P 2.88 -> 0.30 ms,
-// operator 2.59 -> 0.40, gather-kick 2.63 -> 0.47.  What bounds it now is instruction issue and
-// its latencies (IPC 2.0, 38 warp instructions per particle in Q/P: about 9 to form and stage
-// a particle, 10 to sum it, the rest the changes of cell), no longer atomics (L2 at 25 %).
-// Measured and not kept: nine lanes per stream with three x columns and all values in registers
-// (0.40 ms Q/P: the streams' flushes diverge).
+// 4.2 M particles at 16 per cell (64^3 cells, 5 CTAs per SM), the mean of the eight stages after
+// a sort: Q/P 2.88 -> 0.35 ms (with the centre mass), operator 2.59 -> 0.41, gather-kick 2.63 ->
+// 0.49.  What bounds it now is instruction issue and its latencies (IPC 2.0, 38 warp
+// instructions per particle in Q/P: about 9 to form and stage a particle, 10 to sum it, the
+// rest the changes of cell), no longer atomics (L2 at 25 %).  Measured and not kept: nine lanes
+// per stream with three x columns and all values in registers (0.40 ms Q/P: the streams'
+// flushes diverge); six CTAs per SM (80 registers, spilled: 4 % slower).
 #pragma once
 
 #include "dustb_common.cuh"

@@ -726,8 +726,38 @@ __device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &
     }
     const int n = __popc(__ballot_sync(0xffffffffu, live));
     const bool check = __any_sync(0xffffffffu, !isfinite(sum));
+    // lanes on consecutive cells (a lattice: one particle per cell, cell after cell) add by
+    // themselves: their atomics fall on consecutive words, and a window per particle would
+    // move on for every one of them (128 damping boxes, FP64 cycles: 0.66 G particle-steps/s all
+    // through the windows, 0.72 by one atomic per particle and cell alone, 0.86 so)
+    const unsigned next = __shfl_down_sync(0xffffffffu, key, 1);
+    const bool row = __popc(__ballot_sync(0xffffffffu, lane < 31 && live && next == key + 1)) >= 24;
     __syncwarp();
-    dep.walk(st, n, check, vs, at);
+    if (row) {
+      if (live) {
+        double *f = field + st.kb[at_] - ((long long)d.n2 + 1) * d.n1 - 1;
+        for (int x = 0; x < 9; ++x) {
+          const int c = x / 3, b = x - 3 * c;
+          const double wyz = st.w[3 + x][at_];
+          if ((!d.three_d && c != 1) || wyz == 0.0) continue;
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            const double w = wyz * st.w[a][at_];
+            double *g = f + ((long long)c * d.n2 + b) * d.n1 + a;
+            if (ONE) atomicAdd(g, w);
+#pragma unroll
+            for (int v = 0; v < NV - (ONE ? 1 : 0); ++v)
+              atomicAdd(g + (v + (ONE ? 1 : 0)) * vs, w * st.q[at_][v]);
+          }
+        }
+        if (CEN) {
+          const unsigned cells = (unsigned)vs, m = key / cells;
+          if (st.q[at_][3] != 0.0) atomicAdd(cen + (long long)m * nvc * vs + (key - m * cells), st.q[at_][3]);
+        }
+      }
+    } else {
+      dep.walk(st, n, check, vs, at);
+    }
     __syncwarp();
   }
   dep.flush(vs, at);
@@ -891,8 +921,8 @@ constexpr unsigned kYhi = dir_mask(1, 1), kZlo = dir_mask(2, -1), kZhi = dir_mas
 // Grid: x over the shell cells of a block, y over the blocks; a thread takes NV variables of
 // its cell at a time.  The directions whose ghost cells reach the cell are the bits of a mask
 // (one for most cells), taken in NeighborIndex order; each one's neighbour is looked up once
-// for all variables.  (A thread per cell and variable that tested all 26 directions took 600
-// instructions: 88 us for 5 variables of eight blocks of 64^3.)
+// for all variables.  (A thread per cell and variable that tested all 26 directions: 68 us on
+// average over the exchanges of 5 and 3 variables of eight blocks of 64^3, now 17.)
 template <int NV>
 __device__ __forceinline__ void ghost_add_cell(const Ind &d, const int *nb, int gids, double *a,
                                                int nvar, int v0, int m, int k, int j, int i,
@@ -1013,7 +1043,7 @@ __global__ void k_dep_plan_apply(int nseg, const int *__restrict__ tgt, const in
 // copy exchange: every ghost cell <- the neighbour's active cell at index - o*nx.  One warp per
 // row of a block: the whole row in a ghost row, the 2 ng ghost columns (of all variables at
 // once) in the others, so that no thread is started for an active cell (a thread per padded
-// cell with 64-bit index divisions: 42 us against 10 for 4 variables of eight blocks of 64^3)
+// cell with 64-bit index divisions: 42 us against 22 for 4 variables of eight blocks of 64^3)
 __global__ void __launch_bounds__(kThreads)
 k_ghost_copy(Ind d, const int *nghbr, int gids, double *a, int nvar) {
   const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -1172,7 +1202,7 @@ __global__ void k_consistent_gas(Ind d, double *u0, int nv, const double *us, co
 
 // (all of a particle's rows are loaded before its cell is known: with the velocities and rates
 // loaded behind the cell's residual the kernel waited out two memory latencies in turn, 170 us
-// for 4.2 M particles)
+// for 4.2 M particles against 136)
 __global__ void __launch_bounds__(kThreads) k_consistent_dust(PCtx P, MCtx M, Ind d,
                                                               const double *res, double a_dt) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1405,7 +1435,7 @@ constexpr int kPhstChunk = 4096, kPhstSums = 7;
 // One CTA per chunk: four warps load 128 particles at a time, coalesced, and leave their seven
 // terms in shared memory; seven lanes of a fifth warp add the tile before in particle order, so
 // that the loads run beside the serial chain of additions, which bounds it.  (A term of a
-// massless particle is zero.)  3.5 M particles: 3.52 -> 0.06 ms against one thread per chunk.
+// massless particle is zero.)  3.5 M particles: 3.52 -> 0.046 ms against one thread per chunk.
 constexpr int kPhstTile = 128;
 __global__ void __launch_bounds__(kPhstTile + 32)
 k_phst_chunks(PCtx P, int zc, double *part) {

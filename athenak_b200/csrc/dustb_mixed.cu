@@ -2156,7 +2156,8 @@ bool pick_cfg(const dustb_mesh &ms, int npart, const dustb_mixed_params *mp, Cfg
     // 2-D: the Q/P and operator tiles use 106 registers and stage a third of the sums, so four
     // CTAs of 128 threads fit an SM with the smaller buffer; taken where a tile of the mean
     // particle count (five standard deviations allowed) still fits one pass of it -- a second
-    // pass costs more than the fourth CTA gives (1.0 M particles at 4 per cell: Q/P 44 -> 38 us)
+    // pass costs more than the fourth CTA gives (1.0 M particles at 4 per cell: Q/P 43 -> 37 us,
+    // operator 57 -> 49)
     const double mean = (double)npart / (double)ncell_of(ms) * tj * nx1;
     const int ch = default_chunk(tj, nx1, 0, 112);
     if (mean + 5.0 * sqrt(mean) + 16.0 <= ch && ch < cf.chunk) cf.chunk = ch;

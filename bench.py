@@ -403,11 +403,12 @@ def run_ours(args, rep):
         del d2
         torch.cuda.empty_cache()
     fp64_best = min(ms_fp64, fp64_seeded["ms_per_step"]) if fp64_seeded else ms_fp64
-    # kernels of ours per mixed cycle (dc1, consistent split): per stage gas update, count,
-    # scan (3), move, Q/P tile, solve, operator tile, correction, kick tile, consistent gas
-    # = 12, stage 2 adds the history term, and one ghost exchange of u0 closes the cycle:
-    # 12 + 13 + 1 (the consistent dust kicks are folded into the next stage's push)
-    launches_mixed = 26 * args.steps
+    # kernels of ours per mixed cycle (dc1, consistent split): per stage the stage start (gas
+    # register, update, history term), count, scan (2, or 3 beyond 4096 tiles of 4096 bins),
+    # move, Q/P tile, solve, operator tile, correction, kick tile, consistent gas, and one ghost
+    # exchange of u0 closes the cycle (the consistent dust kicks are folded into the next
+    # stage's push; the tile queue's kernel, where the tuner picks it, is not counted)
+    launches_mixed = (2 * (12 if ncell + 2 > 4096 * 4096 else 11) + 1) * args.steps
     # ---- the stratified pc2 workload (mixed pc2 vs FP64 pc2) ----
     strat = None
     if not args.no_pc2:

@@ -81,6 +81,22 @@ def test_deposits_of_every_row_order(order, scheme, cells, block):
     assert g.error_word() == 0
 
 
+@pytest.mark.parametrize("cells,block", [((40, 6, 4), (40, 6, 4)), ((26, 10, 1), (26, 5, 1)), ((8, 8, 8), (4, 8, 8))])
+def test_deposits_of_a_lattice(cells, block):
+    """One particle per cell, cell after cell: rows of consecutive anchors add by themselves, the
+    batches that cross several rows through the windows."""
+    ms, st = state(cells, block, 1, placement="lattice")
+    o, g = pair(st, dict(scheme=2, drag_solver=2))
+    assert o.deposit_qp(2e-3) == 0
+    g.deposit_qp(2e-3)
+    assert fields(g.host("qdep")[:, :4], o.qdep[:, :4]) < TOL
+    for _ in range(2):
+        assert o.imex_cycle(2e-3) == 0
+        g.imex_cycle(2e-3)
+    assert fields(g.host("u0"), o.u0) < 1e-11
+    assert g.error_word() == 0
+
+
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 129])
 def test_partial_warps_and_fused_cycle(n):
     ms, st = state((8, 8, 8), (4, 8, 8), 1, seed=8)
