@@ -148,11 +148,10 @@ struct CellDeposit {
     cur = k;
     base = kb;
   }
-  // the n staged particles of the batch.  check: some staged value is not finite, so that zero
-  // weights (skipped, as the reference skips them) have to be told apart
+  // the n staged particles of the batch, whose values are all finite (the zero weights of a
+  // stencil then add nothing)
   template <typename At>
-  __device__ __forceinline__ void walk(const WarpStage &s, int n, bool check, long long vs,
-                                       At &&at) {
+  __device__ __forceinline__ void walk(const WarpStage &s, int n, long long vs, At &&at) {
     const int lane = threadIdx.x & 31;
     const unsigned key = lane < n ? s.key[lane] : kNoCell;
     const double *wx = s.w[a + 1], *wyz = s.w[3 + 3 * (c + 1) + b + 1];
@@ -161,25 +160,13 @@ struct CellDeposit {
       const unsigned k = __shfl_sync(0xffffffffu, key, lo);
       const int hi = lo + __popc(__ballot_sync(0xffffffffu, key == k));
       move_to(k, s.kb[lo], vs, at);
-      if (!check) {
 #pragma unroll 4
-        for (int p = lo; p < hi; ++p) {
-          const double w = wyz[p] * wx[p];
-          if (ONE) acc[0] += centre ? s.q[p][3] : w;
+      for (int p = lo; p < hi; ++p) {
+        const double w = wyz[p] * wx[p];
+        if (ONE) acc[0] += centre ? s.q[p][3] : w;
 #pragma unroll
-          for (int v = 0; v < NQ; ++v)
-            acc[v + (ONE ? 1 : 0)] = __fma_rn(w, s.q[p][v], acc[v + (ONE ? 1 : 0)]);
-        }
-      } else {
-        for (int p = lo; p < hi; ++p) {
-          if (CEN && centre) acc[0] += s.q[p][3];
-          if (wyz[p] == 0.0 || (CEN && centre)) continue;
-          const double w = wyz[p] * wx[p];
-          if (ONE) acc[0] += w;
-#pragma unroll
-          for (int v = 0; v < NQ; ++v)
-            acc[v + (ONE ? 1 : 0)] = __fma_rn(w, s.q[p][v], acc[v + (ONE ? 1 : 0)]);
-        }
+        for (int v = 0; v < NQ; ++v)
+          acc[v + (ONE ? 1 : 0)] = __fma_rn(w, s.q[p][v], acc[v + (ONE ? 1 : 0)]);
       }
       lo = hi;
     }

@@ -690,7 +690,11 @@ struct BlockScale {
 // every particle of the launch through particle(p, stencil, scale), which returns whether it
 // deposits, and its deposit into variable v0 on of an nvar-variable field
 // (cen, CEN: a field that takes q[3] of every particle at its anchor cell, one variable of nvc)
-template <int NV, bool ONE, bool CEN = false, typename F>
+// A batch with a value that is not finite adds by itself, lane by lane, so that zero weights are
+// told apart as the reference tells them: the drag deposits skip a zero product of the y and z
+// weights and the factor (src/dust/dust_pm.cpp:225-274), the point fields (ALL) a zero weight
+// of the cell (src/dust/dust_gravity_points.cpp:215-245, :257-304)
+template <int NV, bool ONE, bool CEN = false, bool ALL = false, typename F>
 __device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &d, double *field,
                                                   int nvar, int v0, F &&particle,
                                                   double *cen = nullptr, int nvc = 0) {
@@ -733,7 +737,7 @@ __device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &
     const unsigned next = __shfl_down_sync(0xffffffffu, key, 1);
     const bool row = __popc(__ballot_sync(0xffffffffu, lane < 31 && live && next == key + 1)) >= 24;
     __syncwarp();
-    if (row) {
+    if (row || check) {
       if (live) {
         double *f = field + st.kb[at_] - ((long long)d.n2 + 1) * d.n1 - 1;
         for (int x = 0; x < 9; ++x) {
@@ -743,6 +747,7 @@ __device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &
 #pragma unroll
           for (int a = 0; a < 3; ++a) {
             const double w = wyz * st.w[a][at_];
+            if (ALL && w == 0.0) continue;
             double *g = f + ((long long)c * d.n2 + b) * d.n1 + a;
             if (ONE) atomicAdd(g, w);
 #pragma unroll
@@ -756,7 +761,7 @@ __device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &
         }
       }
     } else {
-      dep.walk(st, n, check, vs, at);
+      dep.walk(st, n, vs, at);
     }
     __syncwarp();
   }
@@ -1505,7 +1510,7 @@ k_phst_sums(const double *part, int nchunk, const double *chi, int br, double *r
 // m/V with the deposit weights into the block's cells, ghost cells included
 __global__ void __launch_bounds__(32 * kDepWarps, 5)
 k_mass_deposit(PCtx P, MCtx M, Ind d, double *f, unsigned *err, int nb) {
-  deposit_particles<1, true>(P.npart, nb, d, f, 1, 0, [&](int p, Stencil &t, BlockScale &bs) {
+  deposit_particles<1, true, false, true>(P.npart, nb, d, f, 1, 0, [&](int p, Stencil &t, BlockScale &bs) {
     const double mass = P.r(DUSTB_IPM, p);
     if (mass == 0.0) return false;
     if (!place(P, M, d, p, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p), P.r(DUSTB_IPZ, p), t, bs, err))
@@ -1595,7 +1600,7 @@ __device__ __forceinline__ bool point_stencil(const PCtx &P, const MCtx &M, cons
 template <int NCOMP>
 __global__ void __launch_bounds__(32 * kDepWarps, 5)
 k_point_deposit(PCtx P, MCtx M, Ind d, double *f, int species, int gravity, unsigned *err, int nb) {
-  deposit_particles<NCOMP, true>(P.npart, nb, d, f, NCOMP, 0, [&](int p, Stencil &t, BlockScale &bs) {
+  deposit_particles<NCOMP, true, false, true>(P.npart, nb, d, f, NCOMP, 0, [&](int p, Stencil &t, BlockScale &bs) {
     const double mass = P.r(DUSTB_IPM, p);
     if (gravity) {
       if (!(mass >= 0.0) || !isfinite(mass)) { report(err, DUSTB_ERR_POINT); return false; }
@@ -2785,8 +2790,9 @@ __device__ __forceinline__ void slot_weights(const MCtx &M, const Ind &d, const 
   }
 }
 
-// every cloud of the launch through cloud(p, position, stencil) and its deposit into variable v0
-// on of an nvar-variable field, cells beyond a block in the owning neighbour's active cells
+// every cloud of the launch through cloud(p, position, stencil) -- fac its mass, that is the
+// weights' factor without the cell measure -- and its deposit into variable v0 on of an
+// nvar-variable field, cells beyond a block in the owning neighbour's active cells
 // (report: a cell no block owns sets the error bit)
 template <int NV, bool ONE, typename F>
 __device__ __forceinline__ void deposit_clouds(const MCtx &M, int npart, int nb, const Ind &d,
@@ -2830,6 +2836,27 @@ __device__ __forceinline__ void deposit_clouds(const MCtx &M, int npart, int nb,
     CloudPos c;
     c.L[0] = M.x1max - M.x1min; c.L[1] = M.x2max - M.x2min; c.L[2] = M.x3max - M.x3min;
     const bool live = p0 + lane < npart && cloud((int)(p0 + lane), c, t);
+    double sum = 0.0;                            // (not finite: some value is not, or their sum)
+    if (live) {
+      sum = t.fac;
+#pragma unroll
+      for (int v = 0; v < NV - (ONE ? 1 : 0); ++v) sum += t.q[v];
+    }
+    // a batch with a value that is not finite: a cloud reaches the leaves of nonzero weight
+    // alone (src/dust/dust_leaf3d.hpp:368-513), which the slots' sums would not tell from the rest
+    if (__any_sync(0xffffffffu, !isfinite(sum))) {
+      if (live) {
+        cloud_leaves<false, 0>(M, d, c.m, c.x, c.lev, c.L, 0, [&](const CloudLeaf &lf) {
+          const double w = t.fac * lf.w / cloud_measure(M, d, lf.b);
+          double *g = field + d.at(lf.b, nvar, v0, lf.k, lf.j, lf.i);
+          if (ONE) atomicAdd(g, w);
+#pragma unroll
+          for (int v = 0; v < NV - (ONE ? 1 : 0); ++v)
+            atomicAdd(g + (v + (ONE ? 1 : 0)) * vs, w * t.q[v]);
+        }, err);
+      }
+      continue;
+    }
     unsigned key = kNoCell;
     long long kb = 0;
     if (live) {
@@ -2838,16 +2865,11 @@ __device__ __forceinline__ void deposit_clouds(const MCtx &M, int npart, int nb,
       kb = 2 * d.at(c.m, nvar, v0, k, j, i) + (c.inside ? 1 : 0);
     }
     const int slot = warp_rank(key, live);
-    double sum = 0.0;
-    if (live) {
-      st.put(slot, t.wx, t.wy, t.wz, t.fac, t.q, key, kb);
-#pragma unroll
-      for (int v = 0; v < NV - (ONE ? 1 : 0); ++v) sum += t.q[v];
-    }
+    if (live)
+      st.put(slot, t.wx, t.wy, t.wz, t.fac / cloud_measure(M, d, c.m), t.q, key, kb);
     const int n = __popc(__ballot_sync(0xffffffffu, live));
-    const bool check = __any_sync(0xffffffffu, !isfinite(sum));
     __syncwarp();
-    dep.walk(st, n, check, vs, at);
+    dep.walk(st, n, vs, at);
     __syncwarp();
   }
   dep.flush(vs, at);
@@ -2994,7 +3016,7 @@ k_cloud_deposit_s(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh, u
     slot_weights(M, d, c, t.wx, t.wy, t.wz);
     const double mass_c = d.three_d ? P.r(DUSTB_IPM, p) * a_dt / (P.r(DUSTB_IPTS, p) + a_dt)
                                     : P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt));
-    t.fac = mass_c / cloud_measure(M, d, c.m);
+    t.fac = mass_c;
     t.q[0] = P.r(DUSTB_IPVX, p); t.q[1] = P.r(DUSTB_IPVY, p); t.q[2] = P.r(DUSTB_IPVZ, p);
     t.q[3] = 0.0;
     return true;
@@ -3014,7 +3036,7 @@ k_cloud_gather_kick_s(PCtx P, MCtx M, Ind d, const double *gp, double *dmom, dou
     P.r(DUSTB_IPVX, p) = vx + dvx; P.r(DUSTB_IPVY, p) = vy + dvy; P.r(DUSTB_IPVZ, p) = vz + dvz;
     P.r(DUSTB_IPRX, p) = dvx / a_dt; P.r(DUSTB_IPRY, p) = dvy / a_dt; P.r(DUSTB_IPRZ, p) = dvz / a_dt;
     if (!br) return false;
-    t.fac = -P.r(DUSTB_IPM, p) / cloud_measure(M, d, c.m);
+    t.fac = -P.r(DUSTB_IPM, p);
     t.q[0] = dvx; t.q[1] = dvy; t.q[2] = dvz; t.q[3] = 0.0;
     return true;
   });
@@ -3026,7 +3048,7 @@ k_cloud_operator_s(PCtx P, MCtx M, Ind d, const double *gp, double *result, doub
   deposit_clouds<3, false>(M, P.npart, nb, d, result, 3, 0, nullptr, [&](int p, CloudPos &c, Stencil &t) {
     if (!cloud_here(P, M, d, p, sh, c, err)) return false;
     slot_gather<true>(M, d, c, gp, 0, t.q, t.wx, t.wy, t.wz, err);
-    t.fac = P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt)) / cloud_measure(M, d, c.m);
+    t.fac = P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt));
     t.q[3] = 0.0;
     return true;
   });
@@ -3157,7 +3179,7 @@ k_cloud_pc2_predictor_s(PCtx P, MCtx M, Ind d, const double *gp, double *qdep, d
     double ug[3];
     slot_gather<true>(M, d, c, gp, 0, ug, t.wx, t.wy, t.wz, err);
     const double mass_rate = P.r(DUSTB_IPM, p) / P.r(DUSTB_IPTS, p);
-    t.fac = 1.0 / cloud_measure(M, d, c.m);
+    t.fac = 1.0;
     t.q[0] = -dt * mass_rate * (ug[0] - P.r(DUSTB_IPVX, p));
     t.q[1] = -dt * mass_rate * (ug[1] - P.r(DUSTB_IPVY, p));
     t.q[2] = -dt * mass_rate * (ug[2] - P.r(DUSTB_IPVZ, p));
@@ -3279,7 +3301,7 @@ k_cloud_pc2_advance_s(PCtx P, MCtx M, Ind d, const double *gp, double *dmom, dou
     slot_gather<true>(M, d, c, gp, 0, ug, t.wx, t.wy, t.wz, err);
     cloud_advance(P, d, p, dt, sbox, strat, q, om, aphi, H, ug, t.q);
     if (!br) return false;
-    t.fac = -P.r(DUSTB_IPM, p) / cloud_measure(M, d, c.m);
+    t.fac = -P.r(DUSTB_IPM, p);
     t.q[3] = 0.0;
     return true;
   });

@@ -125,6 +125,55 @@ def test_zero_weights_keep_non_finite_values_out():
     g.deposit_qp(1e-3)
     np.testing.assert_array_equal(np.isfinite(g.host("qdep")[:, :4]), np.isfinite(o.qdep[:, :4]))
 
+@pytest.mark.parametrize("placement", ["random", "lattice"])
+@pytest.mark.parametrize("scheme", [0, 1, 2])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_science_fields_skip_cells_of_zero_weight(scheme, placement, bad):
+    """A velocity that is not finite reaches the cells of nonzero weight alone, along x too, in
+    a batch of any order (the lattice: rows of consecutive cells)."""
+    ms, st = state((32, 6, 6), (32, 6, 6), 1, seed=4, placement=placement)
+    st.pr[1, 7] = bad
+    st.pr[5, 70] = -bad
+    o, g = pair(st, dict(scheme=scheme))
+    out, err = o.point_science_fields()
+    got = g.point_science_fields().cpu().numpy()
+    assert err == 0 and g.error_word() == 0
+    np.testing.assert_array_equal(np.isfinite(got), np.isfinite(out))
+    ok = np.isfinite(out)
+    assert np.abs(got[ok] - out[ok]).max() < TOL * np.abs(out[ok]).max()
+
+
+@pytest.mark.parametrize("row,bad", [(1, np.inf), (3, np.nan), (16, np.inf), (16, np.nan), ("massless", np.inf)])
+@pytest.mark.parametrize("cells,block", [((10, 14, 6), (5, 7, 6)), ((12, 18, 1), (4, 9, 1))])
+def test_clouds_skip_cells_of_zero_weight(cells, block, row, bad):
+    """Clouds of levels 0 to 3 with a velocity or a mass that is not finite: the leaves of nonzero
+    weight alone take them, in Q/P and the kick's back-reaction."""
+    ms, st = state(cells, block, 3, seed=13)
+    st.pi[3, :st.npart] = np.arange(st.npart) % 4
+    for p in (5, 34, 63):                      # (levels 1, 2 and 3)
+        if row == "massless":
+            st.pr[16, p], st.pr[1, p] = 0.0, bad
+        else:
+            st.pr[row, p] = bad
+    o, g = pair(st, dict(scheme=2))
+
+    def same(a, b):
+        ok = np.isfinite(b)
+        np.testing.assert_array_equal(np.isfinite(a), ok)
+        assert np.abs(a[ok] - b[ok]).max() < TOL * np.abs(b[ok]).max()
+
+    assert o.cloud_deposit_qp(1.3e-3, 0.0) == 0
+    g.cloud_deposit_qp(1.3e-3, 0.0)
+    same(g.host("qdep")[:, :4], o.qdep[:, :4])
+    us = np.random.default_rng(6).standard_normal(o.ustar.shape) * 0.05
+    o.ustar[...] = us
+    g.t["ustar"].copy_(torch.from_numpy(us))
+    o.ghost_copy("ustar", 3, 0); g.ghost_copy("ustar", 3, 0)
+    assert o.cloud_gather_kick(2e-3, 0.0, o.gather_pack()) == 0
+    g.cloud_gather_kick(2e-3, 0.0)
+    same(g.host("dmom"), o.dmom)
+    assert g.error_word() == 0
+
 
 @pytest.mark.parametrize("n", [1, 127, 128, 129, 4095, 4096, 4097, 8300])
 def test_history_row_at_chunk_edges(n):
