@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from athenak_b200.inputs import make_state
-from athenak_b200.mesh import uniform_mesh
+from athenak_b200.mesh import dir_index, uniform_mesh
 from oracle.oracle import Oracle
 
 torch = pytest.importorskip("torch")
@@ -173,6 +173,29 @@ def test_clouds_skip_cells_of_zero_weight(cells, block, row, bad):
     g.cloud_gather_kick(2e-3, 0.0)
     same(g.host("dmom"), o.dmom)
     assert g.error_word() == 0
+
+
+@pytest.mark.parametrize("mass", [0.0, 1e-7])
+@pytest.mark.parametrize("offset,missing", [((0.9, 0.9, 0.0), (1, 1, 0)), ((0.0, 0.9, 0.9), (0, 1, 1)),
+                                            ((0.9, 0.9, 0.9), (1, 1, 1)), ((0.9, 0.9, 0.0), (1, 0, 0))])
+def test_clouds_that_reach_an_unowned_cell(offset, missing, mass):
+    """A block without one of its edge or corner neighbours: a cloud that reaches into it sets the
+    error bit, a massless one too (a missing face ends the cloud there instead)."""
+    ms, st = state((8, 8, 8), (4, 4, 4), 1, seed=3)
+    ms.nghbr[0, dir_index(*missing)] = -1
+    st.npart = 40
+    st.pi[0, :40] = 0
+    mb = ms.mb_size[0]
+    for a in range(3):                          # (all at the centre of the block but one)
+        st.pr[2 * a, :40] = mb[a] + 2.0 * mb[6 + a]
+        st.pr[2 * a, 17] += 1.9 * mb[6 + a] * (offset[a] > 0)
+    st.pr[16, 17] = mass
+    o, g = pair(st, dict(scheme=2))
+    err = o.cloud_deposit_qp(1.3e-3, 0.0)
+    assert bool(err) == (missing != (1, 0, 0))
+    g.cloud_deposit_qp(1.3e-3, 0.0)
+    assert g.error_word() == err
+    assert fields(g.host("qdep")[:, :4], o.qdep[:, :4]) < TOL
 
 
 @pytest.mark.parametrize("n", [1, 127, 128, 129, 4095, 4096, 4097, 8300])
