@@ -2592,7 +2592,11 @@ __device__ void cloud_gather(const MCtx &M, const Ind &d, int m, const double x[
 // and its reciprocal -- is formed once per slot instead of once per leaf, from the block across
 // the face along that direction (blocks that share a position along a direction have the same
 // faces along it), with the expressions of cloud_axis and cloud_gather: the gathered velocity
-// is the same bit for bit, the deposits to the order of their sums.
+// is the same bit for bit, unless an edge of the hat falls on a cell face, where rounding
+// decides which cells cloud_axis lists and a cell more or less (its weight below 1e-30, its
+// moment of rounding's size) can change the last bit.  The deposits differ by the order of their
+// sums and by a rounding of the factor: it is m / V of the cloud's block instead of m w / V of
+// the leaf's.
 
 // n / d, correctly rounded, from y = 1 / d correctly rounded: two steps of Markstein's
 // quotient iteration (P. Markstein, IBM J. Res. Dev. 34 (1990) 111): the first brings the
@@ -2636,6 +2640,7 @@ __device__ __forceinline__ AxisSlot axis_slot(const MCtx &M, const Ind &d, int m
     if (s.o > 0 && org <= mo) bx0 += L;
   }
   const double za = (bx0 + i * dx - x) * inv, zb = (bx0 + (i + 1) * dx - x) * inv;
+  if (kM && (zb <= -1.0 || za >= 1.0)) return s;  // (beside the hat: no weight, no moment)
   s.w = hat_cdf(zb) - hat_cdf(za);
   if (kM) {
     s.g = ell * (hat_moment(zb) - hat_moment(za));
@@ -2652,6 +2657,7 @@ __device__ __forceinline__ AxisSlot axis_slot(const MCtx &M, const Ind &d, int m
 // a cloud of block m, its cell and its place
 struct CloudPos {
   int m, lev, ic[3];
+  int lo[3];                    // the first slot's cell along each direction
   double x[3], L[3];
   bool inside;                  // the 27 cells lie in the block
 };
@@ -2660,12 +2666,17 @@ __device__ __forceinline__ void cloud_cell(const MCtx &M, const Ind &d, CloudPos
   const int nx[3] = {d.nx1, d.nx2, d.nx3};
   c.inside = true;
   c.ic[2] = 0;
+  c.lo[2] = -1;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     if (a == 2 && !d.three_d) break;
+    const double x = c.x[a] - M.s(c.m, X1MIN + a), idx = 1.0 / M.s(c.m, DX1 + a);
     // (a gather position may lie up to one cell beyond the block; the clamp takes the rounding)
-    c.ic[a] = (int)floor((c.x[a] - M.s(c.m, X1MIN + a)) * (1.0 / M.s(c.m, DX1 + a)));
-    c.ic[a] = min(max(c.ic[a], -1), nx[a]);
+    c.ic[a] = min(max((int)floor(x * idx), -1), nx[a]);
+    // a cloud of level 1 or more is a cell wide at most: its two cells are its first two slots,
+    // so that the lanes of a warp visit them together
+    c.lo[a] = c.ic[a] - 1;
+    if (c.lev > 0 && (x - ldexp(M.s(c.m, DX1 + a), -c.lev)) * idx >= (double)c.ic[a]) c.lo[a] = c.ic[a];
     c.inside = c.inside && c.ic[a] >= 1 && c.ic[a] + 1 < nx[a];
   }
 }
@@ -2685,7 +2696,7 @@ __device__ __forceinline__ AxisHat axis_hat(const MCtx &M, const CloudPos &c, in
 template <bool kM>
 __device__ __forceinline__ AxisSlot slot_of(const MCtx &M, const Ind &d, const CloudPos &c, int a,
                                             int t, const AxisHat &h) {
-  return axis_slot<kM>(M, d, c.m, a, c.ic[a] + t - 1, c.x[a], h.dx, h.idx, h.ell, h.inv, c.L[a]);
+  return axis_slot<kM>(M, d, c.m, a, c.lo[a] + t, c.x[a], h.dx, h.idx, h.ell, h.inv, c.L[a]);
 }
 
 // cloud_gather over the slots (kM), or the sum of weights times a field of nvar variables
@@ -2729,16 +2740,16 @@ __device__ __forceinline__ void slot_gather(const MCtx &M, const Ind &d, const C
       Z.w = 1.0; Z.g = 0.0; Z.e = 0.0; Z.dx = 1.0; Z.y = 1.0; Z.o = 0;
     }
     if (Z.w == 0.0 && (!kM || Z.g == 0.0)) continue;
-    const int kk = d.three_d ? d.ks + c.ic[2] + q - 1 - Z.o * d.nx3 : d.ks;
+    const int kk = d.three_d ? d.ks + c.lo[2] + q - Z.o * d.nx3 : d.ks;
 #pragma unroll 1
     for (int b = 0; b < 3; ++b) {
       const AxisSlot &S = Y[b];
       const double w2 = S.w, g2 = S.g;
       if (w2 == 0.0 && (!kM || g2 == 0.0)) continue;
       const double w23 = w2 * Z.w;
-      const int jj = d.js + c.ic[1] + b - 1 - S.o * d.nx2;
+      const int jj = d.js + c.lo[1] + b - S.o * d.nx2;
       const int rb = cloud_owner(M, d, c.m, 0, S.o, Z.o);
-      const double *row = cell(rb < 0 ? c.m : rb, kk, jj, d.is + c.ic[0] - 1);
+      const double *row = cell(rb < 0 ? c.m : rb, kk, jj, d.is + c.lo[0]);
       const double ey = S.e, dy = S.dx, yy = S.y;
       auto leaf = [&](const AxisSlot &x, const double *g) {
         const double w = w23 * x.w;
@@ -2767,7 +2778,7 @@ __device__ __forceinline__ void slot_gather(const MCtx &M, const Ind &d, const C
         int blk = rb;
         if (X[a].o != 0) {
           blk = cloud_owner(M, d, c.m, X[a].o, S.o, Z.o);
-          if (blk >= 0) g = cell(blk, kk, jj, d.is + c.ic[0] + a - 1 - X[a].o * d.nx1);
+          if (blk >= 0) g = cell(blk, kk, jj, d.is + c.lo[0] + a - X[a].o * d.nx1);
         }
         if (blk < 0) { if (err) report(err, DUSTB_ERR_CLOUD); continue; }
         leaf(X[a], g);
@@ -2806,7 +2817,7 @@ __device__ __forceinline__ bool slots_owned(const MCtx &M, const Ind &d, const C
     in[a] = false;
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
-      const int i = c.ic[a] + t - 1, o = (a == 2 && !d.three_d) ? 0 : (i < 0 ? -1 : (i >= nx[a] ? 1 : 0));
+      const int i = c.lo[a] + t, o = (a == 2 && !d.three_d) ? 0 : (i < 0 ? -1 : (i >= nx[a] ? 1 : 0));
       if (w[t] == 0.0) continue;
       if (o) side[a] = o; else in[a] = true;
     }
@@ -2822,10 +2833,53 @@ __device__ __forceinline__ bool slots_owned(const MCtx &M, const Ind &d, const C
   return true;
 }
 
+// the cloud's deposit leaf by leaf (weights of its slots, fac with the cell measure): the leaves
+// of nonzero weight; one no block owns sets the error bit (err)
+template <int NV, bool ONE>
+__device__ __forceinline__ void slot_add(const MCtx &M, const Ind &d, const CloudPos &c,
+                                         const Stencil &t, double fac, double *field, int nvar,
+                                         int v0, unsigned *err) {
+  const long long vs = d.cells();
+  auto beyond = [](int i, int nx) { return (i < 0) ? -1 : ((i >= nx) ? 1 : 0); };
+#pragma unroll 1
+  for (int q = 0; q < 3; ++q) {
+    const double wz = q == 0 ? t.wz[0] : (q == 1 ? t.wz[1] : t.wz[2]);
+    if (wz == 0.0) continue;
+    const int oz = d.three_d ? beyond(c.lo[2] + q, d.nx3) : 0;
+    const int kk = d.three_d ? d.ks + c.lo[2] + q - oz * d.nx3 : d.ks;
+#pragma unroll 1
+    for (int b = 0; b < 3; ++b) {
+      const double wyz = (b == 0 ? t.wy[0] : (b == 1 ? t.wy[1] : t.wy[2])) * wz;
+      if (wyz == 0.0) continue;
+      const int oy = beyond(c.lo[1] + b, d.nx2), jj = d.js + c.lo[1] + b - oy * d.nx2;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const double w = wyz * t.wx[a];
+        if (w == 0.0) continue;
+        const int ox = beyond(c.lo[0] + a, d.nx1);
+        const int blk = cloud_owner(M, d, c.m, ox, oy, oz);
+        if (blk < 0) { if (err) report(err, DUSTB_ERR_CLOUD); continue; }
+        double *g = field + d.at(blk, nvar, v0, kk, jj, d.is + c.lo[0] + a - ox * d.nx1);
+        const double f = fac * w;
+        if (ONE) atomicAdd(g, f);
+#pragma unroll
+        for (int v = 0; v < NV - (ONE ? 1 : 0); ++v)
+          atomicAdd(g + (v + (ONE ? 1 : 0)) * vs, f * t.q[v]);
+      }
+    }
+  }
+}
+
+// the slots' weights about the cloud's cell: a first slot in the cell itself moves them up by one
+__device__ __forceinline__ void window_weights(double w[3], int lo, int ic) {
+  if (lo != ic) return;
+  w[2] = w[1]; w[1] = w[0]; w[0] = 0.0;
+}
+
 // every cloud of the launch through cloud(p, position, stencil) -- fac its mass, that is the
 // weights' factor without the cell measure -- and its deposit into variable v0 on of an
 // nvar-variable field, cells beyond a block in the owning neighbour's active cells (err: a cell
-// no block owns, reached by a cloud of positive mass, sets the error bit)
+// no block owns, reached by a cloud, sets the error bit)
 template <int NV, bool ONE, typename F>
 __device__ __forceinline__ void deposit_clouds(const MCtx &M, int npart, int nb, const Ind &d,
                                                double *field, int nvar, int v0, unsigned *err,
@@ -2865,37 +2919,44 @@ __device__ __forceinline__ void deposit_clouds(const MCtx &M, int npart, int nb,
     CloudPos c;
     c.L[0] = M.x1max - M.x1min; c.L[1] = M.x2max - M.x2min; c.L[2] = M.x3max - M.x3min;
     const bool live = p0 + lane < npart && cloud((int)(p0 + lane), c, t);
-    double sum = 0.0;                            // (not finite: some value is not, or their sum)
-    if (live) {
-      sum = t.fac;
-#pragma unroll
-      for (int v = 0; v < NV - (ONE ? 1 : 0); ++v) sum += t.q[v];
-    }
-    // a batch with a value that is not finite: a cloud reaches the leaves of nonzero weight
-    // alone (src/dust/dust_leaf3d.hpp:368-513), which the slots' sums would not tell from the rest
-    if (__any_sync(0xffffffffu, !isfinite(sum))) {
-      if (live) {
-        cloud_leaves<false, 0>(M, d, c.m, c.x, c.lev, c.L, 0, [&](const CloudLeaf &lf) {
-          const double w = t.fac * lf.w / cloud_measure(M, d, lf.b);
-          double *g = field + d.at(lf.b, nvar, v0, lf.k, lf.j, lf.i);
-          if (ONE) atomicAdd(g, w);
-#pragma unroll
-          for (int v = 0; v < NV - (ONE ? 1 : 0); ++v)
-            atomicAdd(g + (v + (ONE ? 1 : 0)) * vs, w * t.q[v]);
-        }, err);
-      }
-      continue;
-    }
     unsigned key = kNoCell;
     long long kb = 0;
+    double sum = 0.0;                            // (not finite: some value is not, or their sum)
     if (live) {
       const int k = d.ks + c.ic[2], j = d.js + c.ic[1], i = d.is + c.ic[0];
       key = (unsigned)d.at(c.m, 1, 0, k, j, i);
       kb = 2 * d.at(c.m, nvar, v0, k, j, i) + (c.inside ? 1 : 0);
+      sum = t.fac;
+#pragma unroll
+      for (int v = 0; v < NV - (ONE ? 1 : 0); ++v) sum += t.q[v];
+      t.fac /= cloud_measure(M, d, c.m);
     }
+    // a batch adds leaf by leaf, lane by lane,
+    // - if one of its values is not finite: a cloud reaches the leaves of nonzero weight alone
+    //   (src/dust/dust_leaf3d.hpp:368-513), which the window's sums would not tell from the rest;
+    // - if its clouds are of level 1 or more, at most two cells wide along a direction: a window
+    //   of 27 is mostly empty then (0.9 M clouds of a lattice, Q/P: level 1 0.41 ms through the
+    //   windows, 0.10 so; level 2 0.41 and 0.09; 3.5 M of level 1 at 8 per cell 0.55 and 0.48);
+    // - if 24 or more of its clouds follow on the cell before along x (a lattice): the window
+    //   moves with every one of them (level 0: 0.40 ms, 0.22 so)
+    const unsigned up = __shfl_up_sync(0xffffffffu, key, 1);
+    const int row = __popc(__ballot_sync(0xffffffffu, live && lane > 0 && up + 1 == key));
+    const bool narrow = __all_sync(0xffffffffu, !live || c.lev > 0);
+    if (__any_sync(0xffffffffu, !isfinite(sum)) || row >= 24 || narrow) {
+      if (live) slot_add<NV, ONE>(M, d, c, t, t.fac, field, nvar, v0, err);
+      continue;
+    }
+    // (a cell no block owns is an error of a massless cloud too, which the cell's sum does not
+    // show; looking for it with every cloud costs 8 % of the deposit)
+    if (ONE && err && live && !(t.fac > 1e-200) && !c.inside && !slots_owned(M, d, c, t.wx, t.wy, t.wz))
+      report(err, DUSTB_ERR_CLOUD);
     const int slot = warp_rank(key, live);
-    if (live)
-      st.put(slot, t.wx, t.wy, t.wz, t.fac / cloud_measure(M, d, c.m), t.q, key, kb);
+    if (live) {
+      window_weights(t.wx, c.lo[0], c.ic[0]);
+      window_weights(t.wy, c.lo[1], c.ic[1]);
+      if (d.three_d) window_weights(t.wz, c.lo[2], c.ic[2]);
+      st.put(slot, t.wx, t.wy, t.wz, t.fac, t.q, key, kb);
+    }
     const int n = __popc(__ballot_sync(0xffffffffu, live));
     __syncwarp();
     dep.walk(st, n, vs, at);
@@ -3038,7 +3099,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_cloud_operator_l(PCtx P, MCtx M
   if (p < P.npart) k_cloud_operator_body<1>(p, P, M, d, gp, result, a_dt, sh, x3phys, err);
 }
 
-__global__ void __launch_bounds__(32 * kDepWarps, 4)
+// (six CTAs, 80 registers: 7.1 M clouds of levels 0 to 2 in cell order 1.12 ms, four 1.25)
+__global__ void __launch_bounds__(32 * kDepWarps, 6)
 k_cloud_deposit_s(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh, unsigned *err, int nb) {
   deposit_clouds<4, true>(M, P.npart, nb, d, qdep, 5, 0, err, [&](int p, CloudPos &c, Stencil &t) {
     if (!cloud_here(P, M, d, p, sh, c, err)) return false;
@@ -3046,10 +3108,6 @@ k_cloud_deposit_s(PCtx P, MCtx M, Ind d, double *qdep, double a_dt, double sh, u
     const double mass_c = d.three_d ? P.r(DUSTB_IPM, p) * a_dt / (P.r(DUSTB_IPTS, p) + a_dt)
                                     : P.r(DUSTB_IPM, p) * (a_dt / (P.r(DUSTB_IPTS, p) + a_dt));
     t.fac = mass_c;
-    // (a cell no block owns is an error of a massless cloud too, which the cell's sum does not
-    // show; looking for it with every cloud costs 8 % of this kernel)
-    if (!(mass_c > 1e-200) && !c.inside && !slots_owned(M, d, c, t.wx, t.wy, t.wz))
-      report(err, DUSTB_ERR_CLOUD);
     t.q[0] = P.r(DUSTB_IPVX, p); t.q[1] = P.r(DUSTB_IPVY, p); t.q[2] = P.r(DUSTB_IPVZ, p);
     t.q[3] = 0.0;
     return true;
@@ -3332,6 +3390,7 @@ k_cloud_pc2_advance_s(PCtx P, MCtx M, Ind d, const double *gp, double *dmom, dou
     cloud_cell(M, d, c);
     double ug[3];
     slot_gather<true>(M, d, c, gp, 0, ug, t.wx, t.wy, t.wz, err);
+    cloud_midpoint(P, d, p, dt, sbox, q, om, H);   // (again: held over the gather it spills)
     cloud_advance(P, d, p, dt, sbox, strat, q, om, aphi, H, ug, t.q);
     if (!br) return false;
     t.fac = -P.r(DUSTB_IPM, p);

@@ -289,6 +289,40 @@ def test_cloud_slots_on_odd_blocks(cells, block):
     assert g.error_word() == 0
 
 
+@pytest.mark.parametrize("placement", ["random", "lattice"])
+@pytest.mark.parametrize("levels", [[0], [1], [2], [1, 2, 3], [0, 1]])
+@pytest.mark.parametrize("cells,block", [((32, 6, 4), (32, 3, 4)), ((30, 8, 1), (10, 4, 1)), ((4, 6, 8), (2, 2, 2))])
+def test_clouds_of_one_kind_and_lattices(cells, block, levels, placement):
+    """Batches whose clouds are all narrow, and lattices in cell order, add leaf by leaf: the
+    deposits to their order, the gathered velocities (narrow clouds on two slots) bit for bit.
+    At the centre of a cell a cloud of level 1 or more has its edges on faces or near them: a
+    neighbour listed or not by rounding changes a coefficient by its moment's rounding, some 2 eps
+    of each of up to 19 leaves and 3 coefficients, here times velocities and differences up to 0.3."""
+    ms, st = state(cells, block, 1, seed=13, placement=placement)
+    st.pi[3, :st.npart] = np.resize(levels, st.npart)
+    if placement == "lattice":
+        o = Oracle(st, dict(scheme=2))
+        permute(st, o.sort_order()[0])
+    o, g = pair(st, dict(scheme=2))
+    assert o.cloud_deposit_qp(1.3e-3, 0.0) == 0
+    g.cloud_deposit_qp(1.3e-3, 0.0)
+    assert fields(g.host("qdep")[:, :4], o.qdep[:, :4]) < TOL
+    us = np.random.default_rng(6).standard_normal(o.ustar.shape) * 0.05
+    o.ustar[...] = us
+    g.t["ustar"].copy_(torch.from_numpy(us))
+    o.ghost_copy("ustar", 3, 0); g.ghost_copy("ustar", 3, 0)
+    assert o.cloud_gather_kick(2e-3, 0.0, o.gather_pack()) == 0
+    g.cloud_gather_kick(2e-3, 0.0)
+    for r in (1, 3, 5):
+        a, b = g.host("pr")[r], o.st.pr[r, :st.npart]
+        if placement == "random":
+            np.testing.assert_array_equal(a, b)
+        else:
+            assert np.abs(a - b).max() <= 2 * 19 * 3 * 0.3 * np.finfo(float).eps
+    assert fields(g.host("dmom"), o.dmom) < TOL
+    assert g.error_word() == 0
+
+
 @pytest.mark.parametrize("cells,block,ppc", [
     ((6, 10, 14), (6, 10, 14), 3),      # one block, its own neighbour on every side
     ((4, 6, 4), (2, 6, 2), 5),          # blocks of two cells: every cell at a face
