@@ -690,6 +690,9 @@ struct BlockScale {
 // every particle of the launch through particle(p, stencil, scale), which returns whether it
 // deposits, and its deposit into variable v0 on of an nvar-variable field
 // (cen, CEN: a field that takes q[3] of every particle at its anchor cell, one variable of nvc)
+// (Every kernel of it is held to five CTAs of four warps per SM, 96 registers.  4.2 M particles
+// at 16 per cell, with four, five and six: pc2 predictor 587, 562, 579 us, advance 515, 493, 482;
+// 2-D, 2.1 M at 8 per cell: 257, 230, 253 and 259, 237, 253.  The advance spills 144 B under it.)
 // A batch with a value that is not finite adds by itself, lane by lane, so that zero weights are
 // told apart as the reference tells them: the drag deposits skip a zero product of the y and z
 // weights and the factor (src/dust/dust_pm.cpp:225-274), the point fields (ALL) a zero weight
@@ -721,23 +724,30 @@ __device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &
     const bool live = p0 + lane < npart && particle((int)(p0 + lane), t, bs);
     // (the padded cell's index over all blocks: below 2^32 in one GPU's memory)
     const unsigned key = live ? (unsigned)d.at(t.m, 1, 0, t.kp, t.jp, t.ip) : kNoCell;
-    const int at_ = warp_rank(key, live);
     double sum = 0.0;                            // (not finite: some value is not, or their sum)
     if (live) {
-      st.put(at_, t.wx, t.wy, t.wz, t.fac, t.q, key, d.at(t.m, nvar, v0, t.kp, t.jp, t.ip));
 #pragma unroll
       for (int v = 0; v < NV - (ONE ? 1 : 0); ++v) sum += t.q[v];
     }
-    const int n = __popc(__ballot_sync(0xffffffffu, live));
     const bool check = __any_sync(0xffffffffu, !isfinite(sum));
-    // lanes on consecutive cells (a lattice: one particle per cell, cell after cell) add by
-    // themselves: their atomics fall on consecutive words, and a window per particle would
-    // move on for every one of them (128 damping boxes, FP64 cycles: 0.66 G particle-steps/s all
-    // through the windows, 0.72 by one atomic per particle and cell alone, 0.86 so)
+    // the lanes add by themselves, too,
+    // - on consecutive cells (a lattice: one particle per cell, cell after cell): their atomics
+    //   fall on consecutive words, and a window per particle would move on for every one of them
+    //   (128 damping boxes, FP64 cycles: 0.66 G particle-steps/s all through the windows, 0.72 by
+    //   one atomic per particle and cell alone, 0.86 so);
+    // - in 2-D, where 9 lanes hold a window, on 12 or more changes of cell from one particle to the
+    //   next (1.0 M particles in no order at 4 per cell, imex cycle: 2.10 ms through the windows,
+    //   1.66 so; in cell order at 1 and 2 per cell 0.59 and 0.80, 0.47 and 0.67 so)
     const unsigned next = __shfl_down_sync(0xffffffffu, key, 1);
     const bool row = __popc(__ballot_sync(0xffffffffu, lane < 31 && live && next == key + 1)) >= 24;
+    const bool spread = !d.three_d &&
+        __popc(__ballot_sync(0xffffffffu, lane < 31 && live && next != key)) >= 12;
+    const bool alone = row || check || spread;
+    const int at_ = alone ? lane : warp_rank(key, live);
+    if (live) st.put(at_, t.wx, t.wy, t.wz, t.fac, t.q, key, d.at(t.m, nvar, v0, t.kp, t.jp, t.ip));
+    const int n = __popc(__ballot_sync(0xffffffffu, live));
     __syncwarp();
-    if (row || check) {
+    if (alone) {
       if (live) {
         double *f = field + st.kb[at_] - ((long long)d.n2 + 1) * d.n1 - 1;
         for (int x = 0; x < 9; ++x) {

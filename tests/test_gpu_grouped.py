@@ -96,6 +96,69 @@ def test_deposits_of_a_lattice(cells, block):
     assert fields(g.host("u0"), o.u0) < 1e-11
     assert g.error_word() == 0
 
+@pytest.mark.parametrize("order", ["cell", "drawn", "reversed", "lattice"])
+@pytest.mark.parametrize("scheme,cells,block,ppc", [(2, (26, 28, 18), (13, 14, 9), 1), (1, (18, 20, 12), (9, 10, 6), 4),
+                                                    (2, (96, 64, 1), (48, 32, 1), 2), (0, (40, 72, 1), (20, 9, 1), 8)])
+def test_deposits_of_more_than_two_warps_per_sm(order, scheme, cells, block, ppc):
+    """Launches beyond the direct form's 9472 particles: the windows in cell order, the direct form
+    of 2-D batches that change cell often (drawn) and of lattices; the cycle's centre mass too."""
+    if order == "lattice":
+        ppc = 1
+        cells = tuple(2 * c if c > 1 else 1 for c in cells)
+        block = tuple(2 * b if b > 1 else 1 for b in block)
+    ms, st = state(cells, block, ppc, seed=15, placement="lattice" if order == "lattice" else "random")
+    assert st.npart > 9472
+    phys = dict(scheme=scheme, drag_solver=2)
+    if order in ("cell", "reversed"):
+        by_cell = Oracle(st, phys).sort_order()[0]
+        permute(st, by_cell if order == "cell" else by_cell[::-1].copy())
+    o, g = pair(st, phys)
+    a_dt = 2e-3
+    o.register_copy(); g.register_copy()
+    for rate_dep in (1, 0):
+        assert o.pc2_predictor(a_dt, rate_dep) == 0
+        g.pc2_predictor(a_dt, rate_dep)
+        assert fields(g.host("qdep")[:, 1:4], o.qdep[:, 1:4]) < TOL
+        assert np.abs(g.host("qdep")[:, 4] - o.qdep[:, 4]).max() <= TOL * np.abs(o.qdep[:, 4]).max()
+    assert o.deposit_qp(a_dt) == 0
+    g.deposit_qp(a_dt)
+    assert fields(g.host("qdep")[:, :4], o.qdep[:, :4]) < TOL
+    for s in (o, g):
+        s.ghost_add("qdep", 5); s.solve_ustar(); s.dc1_sweep(a_dt); s.ghost_copy("ustar", 3)
+    assert fields(g.host("ustar"), o.ustar) < TOL
+    o.gather_kick_pmbr(a_dt); g.gather_kick_pmbr(a_dt)
+    assert fields(g.host("dmom"), o.dmom) < TOL
+    assert o.imex_cycle(a_dt) == 0
+    g.imex_cycle(a_dt)
+    assert fields(g.host("u0"), o.u0) < 1e-11
+    assert g.error_word() == 0
+
+
+@pytest.mark.parametrize("order", ["cell", "drawn"])
+@pytest.mark.parametrize("scheme,bad", [(0, np.inf), (1, np.nan), (2, np.inf)])
+def test_values_that_are_not_finite_beside_the_windows(scheme, bad, order):
+    """The batches of such a value add lane by lane, the others through the windows."""
+    ms, st = state((16, 16, 16), (8, 16, 16), 3, seed=4)
+    assert st.npart > 9472
+    if order == "cell":
+        permute(st, Oracle(st, {}).sort_order()[0])
+    st.pr[1, 7] = bad
+    st.pr[5, 7000] = -bad
+    o, g = pair(st, dict(scheme=scheme))
+
+    def same(a, b):
+        ok = np.isfinite(b)
+        np.testing.assert_array_equal(np.isfinite(a), ok)
+        assert np.abs(a[ok] - b[ok]).max() < TOL * np.abs(b[ok]).max()
+
+    out, err = o.point_science_fields()
+    assert err == 0
+    same(g.point_science_fields().cpu().numpy(), out)
+    assert o.deposit_qp(1e-3) == 0
+    g.deposit_qp(1e-3)
+    same(g.host("qdep")[:, :4], o.qdep[:, :4])
+    assert g.error_word() == 0
+
 
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 129])
 def test_partial_warps_and_fused_cycle(n):
