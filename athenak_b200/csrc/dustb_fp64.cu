@@ -737,11 +737,13 @@ __device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &
     //   one atomic per particle and cell alone, 0.86 so);
     // - in 2-D, where 9 lanes hold a window, on 12 or more changes of cell from one particle to the
     //   next (1.0 M particles in no order at 4 per cell, imex cycle: 2.10 ms through the windows,
-    //   1.66 so; in cell order at 1 and 2 per cell 0.59 and 0.80, 0.47 and 0.67 so)
+    //   1.66 so; in cell order at 1 and 2 per cell 0.59 and 0.80, 0.47 and 0.67 so);
+    // - in a launch of two warps per SM or fewer, whose time is a warp's walk and not the atomics
+    //   (8000 particles in 32^3 cells, imex cycle: 0.31 ms, 0.27 so; 60,000: 0.30, 0.36 so)
     const unsigned next = __shfl_down_sync(0xffffffffu, key, 1);
     const bool row = __popc(__ballot_sync(0xffffffffu, lane < 31 && live && next == key + 1)) >= 24;
-    const bool spread = !d.three_d &&
-        __popc(__ballot_sync(0xffffffffu, lane < 31 && live && next != key)) >= 12;
+    const bool spread = npart <= 2 * 32 * 148 ||
+        (!d.three_d && __popc(__ballot_sync(0xffffffffu, lane < 31 && live && next != key)) >= 12);
     const bool alone = row || check || spread;
     const int at_ = alone ? lane : warp_rank(key, live);
     if (live) st.put(at_, t.wx, t.wy, t.wz, t.fac, t.q, key, d.at(t.m, nvar, v0, t.kp, t.jp, t.ip));
