@@ -1057,30 +1057,72 @@ __global__ void k_dep_plan_apply(int nseg, const int *__restrict__ tgt, const in
   a[((long long)tm * nvar + v) * ncell + (c - tm * ncell)] += sum;
 }
 
-// copy exchange: every ghost cell <- the neighbour's active cell at index - o*nx.  One warp per
-// row of a block: the whole row in a ghost row, the 2 ng ghost columns (of all variables at
-// once) in the others, so that no thread is started for an active cell (a thread per padded
-// cell with 64-bit index divisions: 42 us against 22 for 4 variables of eight blocks of 64^3)
+// the ghost cells of a block, enumerated: the ghost planes whole, then in each inner plane its
+// ghost rows whole and the 2 ng ghost columns of its inner rows
+__host__ __device__ inline int ghost_cells(const Ind &d) {
+  const int gz = d.n3 - d.nx3, gy = d.n2 - d.nx2;
+  return gz * d.n2 * d.n1 + d.nx3 * (gy * d.n1 + d.nx2 * 2 * d.ng);
+}
+__device__ __forceinline__ void ghost_cell(const Ind &d, int t, int &k, int &j, int &i) {
+  const int plane = d.n2 * d.n1, gz = d.n3 - d.nx3, gy = d.n2 - d.nx2;
+  if (t < gz * plane) {
+    const int z = t / plane, r = t - z * plane;
+    k = z < d.ks ? z : z + d.nx3;
+    j = r / d.n1;
+    i = r - j * d.n1;
+    return;
+  }
+  t -= gz * plane;
+  const int inner = gy * d.n1 + d.nx2 * 2 * d.ng;
+  const int z = t / inner;
+  int r = t - z * inner;
+  k = d.ks + z;
+  if (r < gy * d.n1) {
+    const int y = r / d.n1;
+    j = y < d.js ? y : y + d.nx2;
+    i = r - y * d.n1;
+    return;
+  }
+  r -= gy * d.n1;
+  const int y = r / (2 * d.ng), u = r - y * 2 * d.ng;
+  j = d.js + y;
+  i = u < d.ng ? u : u + d.nx1;
+}
+
+// copy exchange: every ghost cell <- the neighbour's active cell at index - o*nx.  Grid: x over
+// the ghost cells of a block, y over the blocks; a thread takes all variables of its cell, so
+// that the owner is looked up once and the loads of NV variables run together.  5 variables, us: 64^3
+// cells in blocks of 4^3 57, in blocks of 8^3 27; one block of 128^3 14, of 1024^2 8 (a thread per
+// padded cell 57, 33, 47, 16; a warp per row 121, 41, 29, 104: rows of few ghost cells leave its
+// lanes idle, the few long rows of a flat block are its only warps)
+template <int NV>
+__device__ __forceinline__ void copy_cell(double *to, const double *from, long long vs) {
+  double x[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) x[v] = from[v * vs];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) to[v * vs] = x[v];
+}
 __global__ void __launch_bounds__(kThreads)
-k_ghost_copy(Ind d, const int *nghbr, int gids, double *a, int nvar) {
-  const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (row >= d.n2 * d.n3) return;
-  const int k = row / d.n2, j = row - k * d.n2;
+k_ghost_copy(Ind d, const int *nghbr, int gids, double *a, int nvar, int per) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= per) return;
+  int k, j, i;
+  ghost_cell(d, t, k, j, i);
+  const int o1 = (i < d.is) ? -1 : ((i > d.ie) ? 1 : 0);
   const int o2 = (j < d.js) ? -1 : ((j > d.je) ? 1 : 0);
   const int o3 = (k < d.ks) ? -1 : ((k > d.ke) ? 1 : 0);
-  const bool inner = o2 == 0 && o3 == 0;
-  const int cols = inner ? 2 * d.ng : d.n1;
+  const int slot = dir_slot(o1, o2, o3);
+  const long long vs = d.cells();
   for (int m = blockIdx.y; m < d.nmb; m += gridDim.y) {
-    const int *nb = nghbr + (long long)m * 27;
-    for (int x = lane; x < cols * nvar; x += 32) {
-      const int v = x / cols, c = x - v * cols;
-      const int i = (inner && c >= d.ng) ? c + d.nx1 : c;
-      const int o1 = (i < d.is) ? -1 : ((i > d.ie) ? 1 : 0);
-      const int src = nb[dir_slot(o1, o2, o3)] - gids;
-      if (src < 0 || src >= d.nmb) continue;
-      a[d.at(m, nvar, v, k, j, i)] =
-          a[d.at(src, nvar, v, k - o3 * d.nx3, j - o2 * d.nx2, i - o1 * d.nx1)];
-    }
+    const int src = nghbr[(long long)m * 27 + slot] - gids;
+    if (src < 0 || src >= d.nmb) continue;
+    double *to = a + d.at(m, nvar, 0, k, j, i);
+    const double *from = a + d.at(src, nvar, 0, k - o3 * d.nx3, j - o2 * d.nx2, i - o1 * d.nx1);
+    int v = 0;
+    for (; v + 4 <= nvar; v += 4) copy_cell<4>(to + v * vs, from + v * vs, vs);
+    for (; v + 3 <= nvar; v += 3) copy_cell<3>(to + v * vs, from + v * vs, vs);
+    for (; v < nvar; ++v) to[v * vs] = from[v * vs];
   }
 }
 
@@ -3666,9 +3708,9 @@ int dustb_ghost_copy(const dustb_ctx *c, double *field, int nvar, int x3_bcs, vo
   if (!field || nvar <= 0) return DUSTB_EINVAL;
   if (c->mesh.nghbr_ml) return DUSTB_EUNSUP;        // (no prolongation across levels)
   Ind d = make_ind(c->mesh);
-  k_ghost_copy<<<dim3((unsigned)((d.n2 * d.n3 + kThreads / 32 - 1) / (kThreads / 32)),
-                      (unsigned)(d.nmb < 65535 ? d.nmb : 65535)), kThreads, 0, S(stream)>>>(
-      d, c->mesh.nghbr, c->mesh.gids, field, nvar);
+  const int per = ghost_cells(d);
+  k_ghost_copy<<<dim3(blocks_for(per), (unsigned)(d.nmb < 65535 ? d.nmb : 65535)), kThreads, 0, S(stream)>>>(
+      d, c->mesh.nghbr, c->mesh.gids, field, nvar, per);
   const SBox B = sbview(c);
   if (B.on) {
     // the shearing box remap of the x1 ghost strips, after the plain copy and before the

@@ -329,6 +329,26 @@ def test_additive_exchange_in_any_number_of_variables(x3bc, shear):
         assert torch.equal(g.t["many"], one), nv
 
 
+@pytest.mark.parametrize("cells,block,x3bc", [((4, 6, 8), (2, 2, 2), 0), ((300, 4, 1), (300, 2, 1), 0),
+                                              ((4, 300, 1), (2, 300, 1), 0), ((70, 3, 9), (35, 3, 3), 1)])
+def test_copy_exchange_of_flat_and_tiny_blocks(cells, block, x3bc):
+    """The ghost cells' enumeration at its smallest and flattest blocks, in 1 to 7 variables: bit for
+    bit the oracle's, variable by variable."""
+    ms = uniform_mesh(cells, block, 2, (-0.5,) * 3, (0.5,) * 3, x3bc=x3bc)
+    st = make_state(ms, [0.1], [1.0], 1, seed=2)
+    o, g = pair(st, dict(scheme=2))
+    f = np.random.default_rng(5).standard_normal(ms.field_shape(7))
+    want = np.empty_like(f)
+    for v in range(7):
+        o.ustar[...] = f[:, v:v + 1]
+        o.ghost_copy("ustar", 3, 0)
+        want[:, v] = o.ustar[:, 0]
+    for nv in (1, 3, 4, 5, 7):
+        g.t["many"] = torch.from_numpy(np.ascontiguousarray(f[:, :nv])).cuda()
+        g.ghost_copy("many", nv, 0)
+        np.testing.assert_array_equal(g.t["many"].cpu().numpy(), want[:, :nv])
+
+
 @pytest.mark.parametrize("cells,block", [((10, 14, 6), (5, 7, 6)), ((12, 18, 1), (4, 9, 1)),
                                          ((6, 4, 8), (2, 2, 4))])
 def test_cloud_slots_on_odd_blocks(cells, block):
