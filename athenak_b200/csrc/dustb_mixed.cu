@@ -2121,11 +2121,15 @@ struct Cfg {
 
 // the default particles per pass: the largest multiple of 4 that lets as many CTAs share an
 // SM as their registers allow (about 168 per thread), so that a typical tile's particles
-// fit one pass (a second pass costs a second window flush)
+// fit one pass (a second pass costs a second window flush).  In 2-D the Q/P and operator tiles
+// would fit four CTAs with a buffer of 1676 instead of 2284 (64 x 128 blocks, uniform particles: 5 %
+// off a cycle), but the tiles of clumped particles then take more passes: 2.1 M particles of a
+// lognormal density of sigma 2, 8 per cell, 1.38 ms per cycle against 1.08.  Which it is the host
+// does not know
 // (extra: shared memory a CTA needs beyond the head and the rows: the staged window)
-int default_chunk(int tj, int nx1, long long extra = 0, int regs = 168) {
+int default_chunk(int tj, int nx1, long long extra = 0) {
   const int nct = tj * nx1;
-  int ctas = 65536 / (regs * nct);
+  int ctas = 65536 / (168 * nct);
   ctas = ctas < 1 ? 1 : (ctas > 8 ? 8 : ctas);
   const long long per = 233472 / ctas - 2560 - 64;     // less a reserve and the statics
   long long ch = (per - (long long)tile_head_bytes(nct) - extra) / (kTileRows * 4);
@@ -2133,7 +2137,7 @@ int default_chunk(int tj, int nx1, long long extra = 0, int regs = 168) {
   return (int)(ch < 64 ? 64 : (ch > 8192 ? 8192 : ch));
 }
 
-bool pick_cfg(const dustb_mesh &ms, int npart, const dustb_mixed_params *mp, Cfg &cf) {
+bool pick_cfg(const dustb_mesh &ms, const dustb_mixed_params *mp, Cfg &cf) {
   const int nx1 = ms.nx1, nx2 = ms.multi_d ? ms.nx2 : 1;
   const int base = mp->variant & ~(DUSTB_MIXED_GRID_TILES | DUSTB_MIXED_NO_LEDGER |
                                    DUSTB_MIXED_WINDOW_TMA);
@@ -2152,16 +2156,6 @@ bool pick_cfg(const dustb_mesh &ms, int npart, const dustb_mixed_params *mp, Cfg
   cf.tj = tj;
   cf.chunk = mp->chunk > 0 ? mp->chunk
                            : default_chunk(tj, nx1, cf.wtma ? 128 + (long long)tile_window_bytes(tj, nx1) : 0);
-  if (mp->chunk <= 0 && !ms.three_d) {
-    // 2-D: the Q/P and operator tiles use 106 registers and stage a third of the sums, so four
-    // CTAs of 128 threads fit an SM with the smaller buffer; taken where a tile of the mean
-    // particle count (five standard deviations allowed) still fits one pass of it -- a second
-    // pass costs more than the fourth CTA gives (1.0 M particles at 4 per cell: Q/P 43 -> 37 us,
-    // operator 57 -> 49)
-    const double mean = (double)npart / (double)ncell_of(ms) * tj * nx1;
-    const int ch = default_chunk(tj, nx1, 0, 112);
-    if (mean + 5.0 * sqrt(mean) + 16.0 <= ch && ch < cf.chunk) cf.chunk = ch;
-  }
   if (cf.chunk < 64 || cf.chunk > 8192 || (cf.chunk & 3)) return false;
   cf.tpp = nx2 / tj;
   cf.probe_timeout = (base == DUSTB_MIXED_PROBE_COPY_TIMEOUT);
@@ -2528,7 +2522,7 @@ int dustb_mixed_tune(const dustb_ctx *c, dustb_mixed_params *mp, void *ws, long 
     t.chunk = cands[q].chunk;
     t.variant = keep | (cands[q].grid ? DUSTB_MIXED_GRID_TILES : 0);
     Cfg cf;
-    if (!pick_cfg(c->mesh, c->part.npart, &t, cf)) continue;     // (the shape does not fit shared memory)
+    if (!pick_cfg(c->mesh, &t, cf)) continue;     // (the shape does not fit shared memory)
     // the Q/P and operator tiles on the shadow as it stands: they write only the stage's
     // scratch fields (qdep, the centre mass, work), which every cycle rewrites before use
     auto trial = [&]() {
@@ -2594,7 +2588,7 @@ int dustb_mixed_imex_cycle(const dustb_ctx *c, const dustb_mixed_params *mp, voi
   MState S;
   if (!carve(c->mesh, c->part.npart, ws, bytes, S, nullptr)) return DUSTB_ESCRATCH;
   Cfg cf;
-  if (!pick_cfg(c->mesh, c->part.npart, mp, cf)) return DUSTB_EUNSUP;
+  if (!pick_cfg(c->mesh, mp, cf)) return DUSTB_EUNSUP;
   cudaStream_t st = (cudaStream_t)stream;
   const int n = c->part.npart;
   const long long ncell = ncell_of(c->mesh);
@@ -2760,7 +2754,7 @@ int dustb_mixed_pc2_cycle(const dustb_ctx *c, const dustb_mixed_params *mp, void
   MState S;
   if (!carve(c->mesh, c->part.npart, ws, bytes, S, nullptr)) return DUSTB_ESCRATCH;
   Cfg cf;
-  if (!pick_cfg(c->mesh, c->part.npart, mp, cf)) return DUSTB_EUNSUP;
+  if (!pick_cfg(c->mesh, mp, cf)) return DUSTB_EUNSUP;
   cudaStream_t st = (cudaStream_t)stream;
   const int n = c->part.npart;
   const long long ncell = ncell_of(c->mesh);

@@ -2,7 +2,7 @@
 summed per cell inside a warp (any row order, weights, partial warps, non-finite values), the
 cycle's fused push and centre mass, the history row's chunk edges, long runs of the cell sort,
 the scan's two forms, the exchanges' variable groups and the clouds' slots on odd blocks --
-against the CPU oracle; the mixed stage's window and buffer rules against the FP64 form."""
+against the CPU oracle; the mixed stage's window against the FP64 form."""
 import numpy as np
 import pytest
 
@@ -409,11 +409,11 @@ def test_clouds_of_one_kind_and_lattices(cells, block, levels, placement):
 @pytest.mark.parametrize("cells,block,ppc", [
     ((6, 10, 14), (6, 10, 14), 3),      # one block, its own neighbour on every side
     ((4, 6, 4), (2, 6, 2), 5),          # blocks of two cells: every cell at a face
-    ((64, 36, 1), (64, 9, 1), 2),       # 2-D, few particles per tile: the small buffer
-    ((64, 8, 1), (64, 4, 1), 40),       # 2-D, dense: the large one, several passes
+    ((64, 36, 1), (64, 9, 1), 2),       # 2-D, few particles per tile: one pass
+    ((64, 8, 1), (64, 4, 1), 40),       # 2-D, dense: several passes
 ])
 def test_mixed_stage_matches_fp64(cells, block, ppc):
-    """The window written by the solves and the buffer rule: every velocity and the gas within
+    """The window written by the solves: every velocity and the gas within
     the mixed form's 1e-5 of the largest (plain back-reaction, two cycles)."""
     from athenak_b200.drag import DeviceDust
     from athenak_b200.mixed import MixedDust
