@@ -1347,10 +1347,12 @@ __global__ void k_tstop(PCtx P, double *out, unsigned *err) {
 
 // ---- pc2 ---------------------------------------------------------------------------------
 // DepositDrag pc2 predictor, src/dust/dust_pm.cpp:141-193
+// (NV: 4 with the rate, 3 without: its zeros cost a batch that adds lane by lane a third more atomics)
+template <int NV>
 __global__ void __launch_bounds__(32 * kDepWarps, 5)
 k_pc2_predictor(PCtx P, MCtx M, Ind d, const double *uold, int nv, double *qdep, double dt,
-                int rate_dep, unsigned *err, int nb) {
-  deposit_particles<4, false>(P.npart, nb, d, qdep, 5, 1, [&](int p, Stencil &t, BlockScale &bs) {
+                unsigned *err, int nb) {
+  deposit_particles<NV, false>(P.npart, nb, d, qdep, 5, 1, [&](int p, Stencil &t, BlockScale &bs) {
     if (!place(P, M, d, p, P.r(DUSTB_IPX, p), P.r(DUSTB_IPY, p), P.r(DUSTB_IPZ, p), t, bs, err))
       return false;
     double ugx = 0.0, ugy = 0.0, ugz = 0.0;
@@ -1378,7 +1380,7 @@ k_pc2_predictor(PCtx P, MCtx M, Ind d, const double *uold, int nv, double *qdep,
     t.q[0] = -dt * rate * (ugx - P.r(DUSTB_IPVX, p));
     t.q[1] = -dt * rate * (ugy - P.r(DUSTB_IPVY, p));
     t.q[2] = -dt * rate * (ugz - P.r(DUSTB_IPVZ, p));
-    t.q[3] = rate_dep ? rate : 0.0;
+    t.q[3] = NV > 3 ? rate : 0.0;
     return true;
   });
 }
@@ -3316,10 +3318,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_cloud_pc2_predictor_l(PCtx P, M
   if (p < P.npart) k_cloud_pc2_predictor_body<1>(p, P, M, d, gp, qdep, dt, rate_dep, x3phys, err);
 }
 
+template <int NV>
 __global__ void __launch_bounds__(32 * kDepWarps, 3)
 k_cloud_pc2_predictor_s(PCtx P, MCtx M, Ind d, const double *gp, double *qdep, double dt,
-                        int rate_dep, unsigned *err, int nb) {
-  deposit_clouds<4, false>(M, P.npart, nb, d, qdep, 5, 1, nullptr, [&](int p, CloudPos &c, Stencil &t) {
+                        unsigned *err, int nb) {
+  deposit_clouds<NV, false>(M, P.npart, nb, d, qdep, 5, 1, nullptr, [&](int p, CloudPos &c, Stencil &t) {
     if (!cloud_here(P, M, d, p, 0.0, c, err)) return false;
     double ug[3];
     slot_gather<true>(M, d, c, gp, 0, ug, t.wx, t.wy, t.wz, err);
@@ -3328,7 +3331,7 @@ k_cloud_pc2_predictor_s(PCtx P, MCtx M, Ind d, const double *gp, double *qdep, d
     t.q[0] = -dt * mass_rate * (ug[0] - P.r(DUSTB_IPVX, p));
     t.q[1] = -dt * mass_rate * (ug[1] - P.r(DUSTB_IPVY, p));
     t.q[2] = -dt * mass_rate * (ug[2] - P.r(DUSTB_IPVZ, p));
-    t.q[3] = rate_dep ? mass_rate : 0.0;
+    t.q[3] = NV > 3 ? mass_rate : 0.0;
     return true;
   });
 }
@@ -3808,9 +3811,14 @@ int dustb_pc2_predictor(const dustb_ctx *c, double dt, int rate_dep, void *strea
   CHECK_CTX(c);
   Ind d = make_ind(c->mesh);
   cudaMemsetAsync(c->f.qdep, 0, (size_t)n_all(d) * 5 * sizeof(double), S(stream));
-  if (c->part.npart > 0)
-    k_pc2_predictor<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.u1, c->f.nvar_gas, c->f.qdep, dt,
-                                  rate_dep, c->err, NB(c));
+  if (c->part.npart > 0) {
+    if (rate_dep)
+      k_pc2_predictor<4><<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.u1, c->f.nvar_gas, c->f.qdep, dt,
+                                              c->err, NB(c));
+    else
+      k_pc2_predictor<3><<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.u1, c->f.nvar_gas, c->f.qdep, dt,
+                                              c->err, NB(c));
+  }
   return launch_status("pc2_predictor");
 }
 
@@ -4013,7 +4021,8 @@ int dustb_cloud_pc2_predictor(const dustb_ctx *c, double dt, int rate_dep, doubl
                                         cloud_x3phys(c), c->err);
     else if (cloud_x3phys(c)) k_cloud_pc2_predictor_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, rate_dep,
                                         cloud_x3phys(c), c->err);
-    else k_cloud_pc2_predictor_s<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, rate_dep, c->err, NB(c));
+    else if (rate_dep) k_cloud_pc2_predictor_s<4><<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, c->err, NB(c));
+    else k_cloud_pc2_predictor_s<3><<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, c->err, NB(c));
   }
   return launch_status("cloud_pc2_predictor");
 }
