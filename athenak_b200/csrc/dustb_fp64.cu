@@ -663,6 +663,11 @@ __global__ void __launch_bounds__(kThreads, 3) k_push_route(PCtx P, PushCoef C, 
 }
 
 // ---- deposits: a warp's particles combined per cell (dustb_deposit.cuh) -------------------
+// whether the padded cells of the pack outnumber the 32-bit cell keys of a batch (a density field
+// of 4.3 G cells, 34 GB, fits one GPU)
+__host__ __device__ inline bool keys_wide(const Ind &d) {
+  return d.cells() * d.nmb >= (long long)kNoCell;
+}
 // a depositing particle: its block, anchor cell, weights, the factor of the weights and the
 // values
 struct Stencil {
@@ -722,7 +727,8 @@ __device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &
     if (p0 >= npart) break;
     Stencil t;
     const bool live = p0 + lane < npart && particle((int)(p0 + lane), t, bs);
-    // (the padded cell's index over all blocks: below 2^32 in one GPU's memory)
+    // the padded cell's index over all blocks (cut to 32 bits on a mesh too large for them, where
+    // every batch adds lane by lane and the key serves nothing)
     const unsigned key = live ? (unsigned)d.at(t.m, 1, 0, t.kp, t.jp, t.ip) : kNoCell;
     double sum = 0.0;                            // (not finite: some value is not, or their sum)
     if (live) {
@@ -742,7 +748,7 @@ __device__ __forceinline__ void deposit_particles(int npart, int nb, const Ind &
     //   (8000 particles in 32^3 cells, imex cycle: 0.31 ms, 0.27 so; 60,000: 0.30, 0.36 so)
     const unsigned next = __shfl_down_sync(0xffffffffu, key, 1);
     const bool row = __popc(__ballot_sync(0xffffffffu, lane < 31 && live && next == key + 1)) >= 24;
-    const bool spread = npart <= 2 * 32 * 148 ||
+    const bool spread = npart <= 2 * 32 * 148 || keys_wide(d) ||
         (!d.three_d && __popc(__ballot_sync(0xffffffffu, lane < 31 && live && next != key)) >= 12);
     const bool alone = row || check || spread;
     const int at_ = alone ? lane : warp_rank(key, live);
@@ -2632,7 +2638,8 @@ __device__ void cloud_gather(const MCtx &M, const Ind &d, int m, const double x[
 
 // Every cloud kernel below has a body, templated on the traversal form, for one cloud in the
 // general traversal, and three kernels: _u, a thread per cloud through the uniform-mesh
-// traversal (meshes with physical x3 faces, whose clouds have a mirrored part); _l, over the
+// traversal (meshes with physical x3 faces, whose clouds have a mirrored part, and meshes of 2^32
+// cells and more); _l, over the
 // leaf tables of refined meshes (held to 128 registers, 2 CTAs of 256 threads per SM: about 15 %
 // faster than its unbounded 230 registers, which allow one CTA); and _s, the slots of the next
 // section.  (The slots for the clouds inside their block on refined meshes, the others listed
@@ -3660,7 +3667,7 @@ int dustb_deposit_qp(const dustb_ctx *c, double a_dt, double sh, void *stream) {
 
 // whether a cycle's deposit leaves the split's centre mass beside Q/P
 static bool centre_with_qp(const dustb_ctx *c, double sh) {
-  return c->phys.back_reaction && c->phys.consistent_gas && sh == 0.0;
+  return c->phys.back_reaction && c->phys.consistent_gas && sh == 0.0 && !keys_wide(make_ind(c->mesh));
 }
 
 // dustb_deposit_qp of a cycle, with the centre mass (resid, zeroed first) where centre_with_qp
@@ -3924,6 +3931,11 @@ static int cloud_ustar_exchange(const dustb_ctx *c, void *stream) {
 static int cloud_x3phys(const dustb_ctx *c) {
   return c->mesh.three_d && c->mesh.x3bc != DUSTB_X3_PERIODIC;
 }
+// the uniform clouds' general traversal instead of the slots: a mirrored part at physical x3
+// faces, or more cells than the slots' batches have keys
+static bool cloud_general(const dustb_ctx *c) {
+  return cloud_x3phys(c) || keys_wide(make_ind(c->mesh));
+}
 
 long long dustb_cloud_gpack_bytes(const dustb_mesh *mesh) {
   if (!mesh) return -1;
@@ -3938,7 +3950,7 @@ int dustb_cloud_deposit_qp(const dustb_ctx *c, double a_dt, double sh, void *str
   cudaMemsetAsync(c->f.qdep, 0, (size_t)(n_all(d) * 5) * sizeof(double), S(stream));
   if (c->part.npart > 0) {
     if (c->mesh.leaf) k_cloud_deposit_l<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, cloud_x3phys(c), c->err);
-    else if (cloud_x3phys(c)) k_cloud_deposit_u<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, cloud_x3phys(c), c->err);
+    else if (cloud_general(c)) k_cloud_deposit_u<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, cloud_x3phys(c), c->err);
     else k_cloud_deposit_s<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, c->f.qdep, a_dt, sh, c->err, NB(c));
   }
   return launch_status("cloud_deposit_qp");
@@ -3955,7 +3967,7 @@ int dustb_cloud_gather_kick(const dustb_ctx *c, double a_dt, double sh, double *
   if (c->part.npart > 0) {
     if (c->mesh.leaf) k_cloud_gather_kick_l<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, a_dt, sh,
                                       c->phys.back_reaction, cloud_x3phys(c), c->err);
-    else if (cloud_x3phys(c)) k_cloud_gather_kick_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, a_dt, sh,
+    else if (cloud_general(c)) k_cloud_gather_kick_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, a_dt, sh,
                                       c->phys.back_reaction, cloud_x3phys(c), c->err);
     else k_cloud_gather_kick_s<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.dmom, a_dt, sh,
                                       c->phys.back_reaction, c->err, NB(c));
@@ -3976,7 +3988,7 @@ int dustb_cloud_dc1_sweep(const dustb_ctx *c, double a_dt, double sh, double *gp
   if (c->part.npart > 0) {
     if (c->mesh.leaf) k_cloud_operator_l<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.work, a_dt, sh,
                                    cloud_x3phys(c), c->err);
-    else if (cloud_x3phys(c)) k_cloud_operator_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.work, a_dt, sh,
+    else if (cloud_general(c)) k_cloud_operator_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.work, a_dt, sh,
                                    cloud_x3phys(c), c->err);
     else k_cloud_operator_s<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.work, a_dt, sh, c->err, NB(c));
   }
@@ -3998,7 +4010,7 @@ int dustb_cloud_apply_pmbr(const dustb_ctx *c, double a_dt, double sh, void *str
   if (c->part.npart > 0) {
     if (c->mesh.leaf) k_cloud_consistent_dust_l<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt, sh,
                                           cloud_x3phys(c));
-    else if (cloud_x3phys(c)) k_cloud_consistent_dust_u<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt, sh,
+    else if (cloud_general(c)) k_cloud_consistent_dust_u<<<PGRID(c)>>>(pview(c), mview(c), d, c->f.resid, a_dt, sh,
                                           cloud_x3phys(c));
     else k_cloud_consistent_dust_s<<<(unsigned)((c->part.npart + 127) / 128), 128, 0, S(stream)>>>(pview(c), mview(c), d, c->f.resid, a_dt, sh);
   }
@@ -4019,7 +4031,7 @@ int dustb_cloud_pc2_predictor(const dustb_ctx *c, double dt, int rate_dep, doubl
   if (c->part.npart > 0) {
     if (c->mesh.leaf) k_cloud_pc2_predictor_l<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, rate_dep,
                                         cloud_x3phys(c), c->err);
-    else if (cloud_x3phys(c)) k_cloud_pc2_predictor_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, rate_dep,
+    else if (cloud_general(c)) k_cloud_pc2_predictor_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, rate_dep,
                                         cloud_x3phys(c), c->err);
     else if (rate_dep) k_cloud_pc2_predictor_s<4><<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, c->err, NB(c));
     else k_cloud_pc2_predictor_s<3><<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.qdep, dt, c->err, NB(c));
@@ -4039,7 +4051,7 @@ int dustb_cloud_pc2_advance(const dustb_ctx *c, double dt, double *gpack, void *
     if (c->mesh.leaf) k_cloud_pc2_advance_l<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, dt,
                                       ph.back_reaction, ph.shearing_box, ph.stratified,
                                       ph.qshear, ph.omega0, ph.const_accel_phi, cloud_x3phys(c), c->err);
-    else if (cloud_x3phys(c)) k_cloud_pc2_advance_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, dt,
+    else if (cloud_general(c)) k_cloud_pc2_advance_u<<<PGRID(c)>>>(pview(c), mview(c), d, gpack, c->f.dmom, dt,
                                       ph.back_reaction, ph.shearing_box, ph.stratified,
                                       ph.qshear, ph.omega0, ph.const_accel_phi, cloud_x3phys(c), c->err);
     else k_cloud_pc2_advance_s<<<DGRID(c, NB(c))>>>(pview(c), mview(c), d, gpack, c->f.dmom, dt,

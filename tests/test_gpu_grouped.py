@@ -160,6 +160,51 @@ def test_values_that_are_not_finite_beside_the_windows(scheme, bad, order):
     assert g.error_word() == 0
 
 
+def test_deposit_on_more_cells_than_32_bit_keys():
+    """Two cells 2^32 apart in the pack's padded cells: their particles stay apart.  Needs 69 GB for
+    the density and its halo."""
+    from athenak_b200.drag import DeviceDust
+    if torch.cuda.mem_get_info()[0] < 80 << 30:
+        pytest.skip("needs 80 GB of free device memory")
+    torch.cuda.empty_cache()
+    ms = uniform_mesh((1792, 1792, 1280), (256, 256, 256), 2, (0.0,) * 3, (1792.0, 1792.0, 1280.0))
+    per = 260 ** 3
+    assert ms.nmb * per > 2 ** 32
+    a = np.array([0, 20, 10, 10])                # block, padded k, j, i
+    at = (a[1] * 260 + a[2]) * 260 + a[3] + 2 ** 32
+    b = np.array([at // per, at % per // 260 ** 2, at % 260 ** 2 // 260, at % 260])
+    assert b[0] == ms.nmb - 1 and (b[1:] >= 4).all() and (b[1:] < 256).all()
+    n = 12000                                    # (beyond the launches that add lane by lane)
+    g = DeviceDust.__new__(DeviceDust)
+    from athenak_b200 import capi
+    g.lib, g.mesh, g.device, g.npart, g.nspecies, g.stride = capi.load(), ms, torch.device("cuda"), n, 1, n
+    f64 = dict(dtype=torch.float64, device="cuda")
+    g.t = {k: torch.zeros(1, **f64) for k in ("u0", "u1", "qdep", "ustar", "dmom", "resid", "work", "sb_gid", "scalar")}
+    g.t.update(pr=torch.zeros((17, n), **f64), pi=torch.zeros((5, n), dtype=torch.int32, device="cuda"),
+               mb_size=torch.from_numpy(ms.mb_size).cuda(), nghbr=torch.from_numpy(ms.nghbr).cuda(),
+               err=torch.zeros(1, dtype=torch.int32, device="cuda"), x3_removed=torch.zeros(2, **f64))
+    g.phys = dict(scheme=2)
+    g._rebuild_ctx()
+    for q, c in enumerate((a, b)):               # a particle of each in turn, at the cells' centres
+        g.t["pi"][0, q::2] = int(c[0])
+        for x in range(3):
+            g.t["pr"][2 * x, q::2] = float(ms.mb_size[c[0], x]) + float(c[3 - x]) - 2.0 + 0.5
+    g.t["pr"][16] = 1.0
+    g.t["pr"][16, 1::2] = 2.0
+    rho = g.point_gravity_density()
+    assert g.error_word() == 0
+    w = np.array([0.125, 0.75, 0.125])
+    w = w[:, None, None] * w[None, :, None] * w[None, None, :] * (n // 2)
+    total = 0.0
+    for c, m in ((a, 1.0), (b, 2.0)):
+        got = rho[c[0], 0, c[1] - 1:c[1] + 2, c[2] - 1:c[2] + 2, c[3] - 1:c[3] + 2].cpu().numpy()
+        np.testing.assert_allclose(got, m * w, rtol=TOL)
+        total += m * n / 2
+    assert abs(float(sum(rho[m].sum() for m in range(ms.nmb))) - total) < TOL * total
+    del rho, g
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 129])
 def test_partial_warps_and_fused_cycle(n):
     ms, st = state((8, 8, 8), (4, 8, 8), 1, seed=8)
