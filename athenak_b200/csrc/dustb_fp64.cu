@@ -8,6 +8,7 @@
 
 #include "dustb_common.cuh"
 #include "dustb_deposit.cuh"
+#include "dustb_div.cuh"
 #include "dustb_sort.cuh"
 
 using namespace dustb;
@@ -2660,16 +2661,6 @@ __device__ void cloud_gather(const MCtx &M, const Ind &d, int m, const double x[
 // moment of rounding's size) can change the last bit.  The deposits differ by the order of their
 // sums and by a rounding of the factor: it is m / V of the cloud's block instead of m w / V of
 // the leaf's.
-
-// n / d, correctly rounded, from y = 1 / d correctly rounded: two steps of Markstein's
-// quotient iteration (P. Markstein, IBM J. Res. Dev. 34 (1990) 111): the first brings the
-// quotient within an ulp, the second rounds it correctly.  The operands are cell widths and
-// weights times distances, far from overflow and underflow
-__device__ __forceinline__ double div_by(double n, double d, double y) {
-  double q = n * y;
-  q = __fma_rn(__fma_rn(-q, d, n), y, q);
-  return __fma_rn(__fma_rn(-q, d, n), y, q);
-}
 
 struct AxisSlot {
   double w, g;                  // weight and first moment of the slot's cell
