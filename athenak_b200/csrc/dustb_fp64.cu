@@ -1,7 +1,7 @@
 // dustb_fp64.cu -- the FP64 form of the dust drag step: one kernel per reference kernel,
 // one thread per particle or per cell, the deposits combined per cell inside a warp
 // (dustb_deposit.cuh).  Compiled with --fmad=false so that the per-particle arithmetic rounds
-// exactly as the CPU oracle's does.
+// exactly as the CPU oracle's does (the deposits' weights and sums to a few eps, see there).
 #include <cfloat>
 #include <cstdio>
 #include <cstring>
