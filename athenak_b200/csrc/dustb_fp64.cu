@@ -2857,7 +2857,7 @@ __device__ __forceinline__ void slot_weights(const MCtx &M, const Ind &d, const 
 
 // whether every cell the cloud reaches with a weight other than zero has an owner (a direction
 // whose face has no neighbour has no slot beyond it).  nx >= 2, so the cells beyond the block lie
-// on one side along each direction
+// on one side along each direction.  (3-D: the windows' batches)
 __device__ __forceinline__ bool slots_owned(const MCtx &M, const Ind &d, const CloudPos &c,
                                             const double wx[3], const double wy[3],
                                             const double wz[3]) {
@@ -2871,7 +2871,7 @@ __device__ __forceinline__ bool slots_owned(const MCtx &M, const Ind &d, const C
     in[a] = false;
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
-      const int i = c.lo[a] + t, o = (a == 2 && !d.three_d) ? 0 : (i < 0 ? -1 : (i >= nx[a] ? 1 : 0));
+      const int i = c.lo[a] + t, o = i < 0 ? -1 : (i >= nx[a] ? 1 : 0);
       if (w[t] == 0.0) continue;
       if (o) side[a] = o; else in[a] = true;
     }
@@ -2942,7 +2942,7 @@ __device__ __forceinline__ void deposit_clouds(const MCtx &M, int npart, int nb,
   WarpStage &st = s_stage[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   CellDeposit<NV, ONE> dep;
-  dep.init(d.three_d);
+  dep.init(true);                                // (the windows are for 3-D batches)
   const long long vs = d.cells();
   double *mine = field + ((long long)(dep.c * d.n2 + dep.b) * d.n1 + dep.a);
   // the anchor's index is doubled: its low bit says that the window lies inside the block
@@ -2957,7 +2957,7 @@ __device__ __forceinline__ void deposit_clouds(const MCtx &M, int npart, int nb,
     int j = (int)(r / (unsigned)d.n1), i = (int)(r - (unsigned)(j * d.n1));
     i += dep.a - d.is; j += dep.b - d.js; k += dep.c - d.ks;
     const int ox = (i < 0) ? -1 : ((i >= d.nx1) ? 1 : 0), oy = (j < 0) ? -1 : ((j >= d.nx2) ? 1 : 0);
-    const int oz = d.three_d ? ((k < 0) ? -1 : ((k >= d.nx3) ? 1 : 0)) : 0;
+    const int oz = (k < 0) ? -1 : ((k >= d.nx3) ? 1 : 0);
     const int b = cloud_owner(M, d, m, ox, oy, oz);
     if (b < 0) {
       if (ONE && err && dep.acc[0] != 0.0) report(err, DUSTB_ERR_CLOUD);
@@ -2992,11 +2992,13 @@ __device__ __forceinline__ void deposit_clouds(const MCtx &M, int npart, int nb,
     //   of 27 is mostly empty then (0.9 M clouds of a lattice, Q/P: level 1 0.41 ms through the
     //   windows, 0.10 so; level 2 0.41 and 0.09; 3.5 M of level 1 at 8 per cell 0.55 and 0.48);
     // - if 24 or more of its clouds follow on the cell before along x (a lattice): the window
-    //   moves with every one of them (level 0: 0.40 ms, 0.22 so)
+    //   moves with every one of them (level 0: 0.40 ms, 0.22 so);
+    // - in 2-D, where 9 lanes hold a window and a cloud has 9 leaves (512^2 cells, imex cycle, 1 and
+    //   8 per cell in cell order 1.05 and 4.01 ms, 0.79 and 3.74 so; 8 in no order 8.41, 5.85 so)
     const unsigned up = __shfl_up_sync(0xffffffffu, key, 1);
     const int row = __popc(__ballot_sync(0xffffffffu, live && lane > 0 && up + 1 == key));
     const bool narrow = __all_sync(0xffffffffu, !live || c.lev > 0);
-    if (__any_sync(0xffffffffu, !isfinite(sum)) || row >= 24 || narrow) {
+    if (__any_sync(0xffffffffu, !isfinite(sum)) || row >= 24 || narrow || !d.three_d) {
       if (live) slot_add<NV, ONE>(M, d, c, t, t.fac, field, nvar, v0, err);
       continue;
     }
@@ -3008,7 +3010,7 @@ __device__ __forceinline__ void deposit_clouds(const MCtx &M, int npart, int nb,
     if (live) {
       window_weights(t.wx, c.lo[0], c.ic[0]);
       window_weights(t.wy, c.lo[1], c.ic[1]);
-      if (d.three_d) window_weights(t.wz, c.lo[2], c.ic[2]);
+      window_weights(t.wz, c.lo[2], c.ic[2]);
       st.put(slot, t.wx, t.wy, t.wz, t.fac, t.q, key, kb);
     }
     const int n = __popc(__ballot_sync(0xffffffffu, live));
