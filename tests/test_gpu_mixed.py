@@ -67,7 +67,10 @@ def run_pair(name, cycles=3):
     return st, ref, mx, p0, c
 
 
-def check(st, ref, mx, c):
+def check(st, ref, mx, c, stages=0):
+    """stages: of a run whose dust is faster than its gas, for the bound on the gas.  Per stage a
+    cell takes the sum of m W dv, dv the difference of two FP32 velocities and a gathered FP32
+    one: 2 roundings of 2^-24 of the largest velocity, times a dust-to-gas ratio of about 1."""
     assert ref.error_word() == 0 and mx.error_word() == 0
     a, b = mx.dev.host("pr"), ref.host("pr")
     vscale = np.abs(b[[1, 3, 5]]).max()
@@ -84,7 +87,7 @@ def check(st, ref, mx, c):
     for v in range(1, 4):
         sc = np.abs(ub[:, v]).max()
         if sc > 0:
-            assert np.abs(ua[:, v] - ub[:, v]).max() < VTOL * sc, v
+            assert np.abs(ua[:, v] - ub[:, v]).max() < max(VTOL * sc, stages * 2 * 2.0 ** -24 * vscale), v
 
 
 @pytest.mark.parametrize("name", list(CASES))
@@ -394,7 +397,9 @@ def test_mixed_imex_shear_shift_matches_fp64(mesh):
         t += dt
     mx.export()
     torch.cuda.synchronize()
-    check(st, ref, mx, None)
+    # (velocities up to 0.107, gas momentum along x3 up to 0.0031: VTOL of the latter is 5 roundings of
+    # the former, and the largest difference of a cell is 0.94 of it, 1.1 in a run out of 25)
+    check(st, ref, mx, None, stages=6)
 
 
 def test_copy_wait_timeout_is_reported_and_recoverable():
